@@ -200,9 +200,9 @@ typedef struct {
     /* launch tuning (0 = library default; chosen by rumi_b200.autotune) */
     int32_t trace_mode;    /* traversal scheme.  Binary tree -- 1: a warp traces 32 rays to
                               completion; 2: per-lane ray refill; 3: per-lane refill with
-                              leaves intersected warp-wide; 4: speculative while-while walk
-                              with per-lane refill.  5: the same walk over the compressed
-                              eight-wide tree, collapsed from the binary tree by the scene's
+                              leaves intersected warp-wide.  4: speculative while-while walk
+                              with per-lane refill over the four-wide tree.  5: that scheme
+                              over the compressed eight-wide tree, collapsed from the binary tree by the scene's
                               first call that asks for it (rumi_render_noalloc cannot: it
                               rejects 5 until then).  0: the library default (4).  Every
                               scheme gives the same hits and films */
@@ -227,7 +227,8 @@ typedef struct {
     int64_t rays_extend;         /* closest-hit rays traced */
     int64_t rays_shadow;         /* shadow rays traced */
     int64_t extend_node_fetches; /* node bytes fetched by closest-hit rays / 32 (STATS): a binary
-                                    node counts 1, a compressed eight-wide node 2.5 */
+                                    node counts 1, a four-wide node 3, a compressed eight-wide
+                                    node 2.5 */
     int64_t extend_prim_tests;   /* primitives tested by closest-hit rays (STATS) */
 } rumi_render_stats;
 

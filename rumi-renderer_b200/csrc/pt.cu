@@ -22,6 +22,9 @@
 #include "traverse.cuh"
 #include "shading.cuh"
 #include "camera.cuh"
+#include <map>
+#include <mutex>
+#include <utility>
 #include <vector>
 #include <type_traits>
 
@@ -42,9 +45,9 @@ static constexpr int TRACE_THREADS = 128;
 #ifndef RUMI_SHADOW_MIN_BLOCKS
 #define RUMI_SHADOW_MIN_BLOCKS RUMI_TRACE_MIN_BLOCKS
 #endif
-// The default walk (scheme 3, the speculative while-while walk over the binary tree) at 9
-// blocks: 56 registers with a 38-byte spill (closest-hit) and 55 without one (any-hit);
-// per 1024x1024x64 frame 83.3 / 44.5 ms of closest-hit / any-hit against 83.8 / 45.7 at 8.
+// The default walk (scheme 3, the speculative while-while walk over the four-wide tree) at 9
+// blocks: 56 registers (a 42-byte spill in closest-hit, none in any-hit); per 1024x1024x64 frame
+// 65.7 / 35.2 ms of closest-hit / any-hit against 66.7 / 36.4 at 8 and 69.9 / 35.2 at 10.
 #ifndef RUMI_WW_MIN_BLOCKS
 #define RUMI_WW_MIN_BLOCKS 9
 #endif
@@ -57,6 +60,9 @@ static constexpr int trace_min_blocks(int mode, bool extend) {
 #define RUMI_PT_OVERLAP 1
 #endif
 static constexpr int STACK_SMEM = 32;
+static constexpr int WALK_SMEM = 16;  // of the default walk (stack_entries)
+static_assert(TRACE_THREADS == WW_THREADS, "the walk's shared-memory columns are one per thread");
+static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? 4 : 3;
 // Threads per block of the shading kernels; a block groups its next rays by direction, so
 // the block size is also the grouping's width (128: shading 0.5 ms faster per frame,
 // closest-hit 0.5 ms slower).
@@ -267,8 +273,8 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, true)) p
         const int code = h.t > 0.0f ? (h.id | (h.back ? (int)0x80000000 : 0)) : -1;
         P.hit[i] = make_float4(h.t, __int_as_float(code), h.u, h.v);
     };
-    traverse_queue<MODE, false, SMEM, STATS>(P.s, P.cnt[cur], &P.cnt[C_FETCH_EXT], P.refill_min,
-                                             stack + threadIdx.x, TRACE_THREADS, fetch, finish, st);
+    traverse_queue<MODE, false, SMEM, STATS>(P.s, P.cnt[cur], &P.cnt[C_FETCH_EXT], P.refill_min, stack, fetch, finish,
+                                             st);
     if (STATS) {
         atomicAdd(&P.stats[S_NODES], (unsigned long long)st.nodes);
         atomicAdd(&P.stats[S_PRIMS], (unsigned long long)st.prims);
@@ -307,7 +313,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, false)) 
         }
     };
     traverse_queue<MODE, true, SMEM, false>(P.s, P.cnt[C_SHADOW], &P.cnt[C_FETCH_SH], P.refill_min,
-                                            stack + threadIdx.x, TRACE_THREADS, fetch, finish, st);
+                                            stack, fetch, finish, st);
     if (ADJ) {
         __syncwarp();
         acc_sigma = warp_sum(acc_sigma);
@@ -323,8 +329,9 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, false)) 
 // rumi_render uses) with each ray's own scene, so a batched scene resolves exact-distance
 // ties exactly as its single-scene render does.
 template <bool ANYHIT>
-__global__ void __launch_bounds__(TRACE_THREADS, RUMI_TRACE_MIN_BLOCKS) pt_trace_multi(PtLaunch P, int bounce) {
-    __shared__ int stack[STACK_SMEM * TRACE_THREADS];
+__global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(DEFAULT_WALK_MODE, !ANYHIT))
+    pt_trace_multi(PtLaunch P, int bounce) {
+    __shared__ int stack[WALK_SMEM * TRACE_THREADS];
     const int cur = bounce & 1;
     const int n = ANYHIT ? P.cnt[C_SHADOW] : P.cnt[cur];
     int *counter = ANYHIT ? &P.cnt[C_FETCH_SH] : &P.cnt[C_FETCH_EXT];
@@ -356,8 +363,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, RUMI_TRACE_MIN_BLOCKS) pt_trace
             P.hit[i] = make_float4(h.t, __int_as_float(code), h.u, h.v);
         }
     };
-    traverse_queue_walk<ANYHIT, STACK_SMEM, false>(scene_of, n, counter, P.refill_min, stack + threadIdx.x,
-                                                   TRACE_THREADS, fetch, finish, st);
+    traverse_queue_walk<ANYHIT, WALK_SMEM, false>(scene_of, n, counter, P.refill_min, stack, fetch, finish, st);
 }
 
 // Next-event estimation toward one light sample from p.  Returns false when the light
@@ -943,10 +949,8 @@ static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b)
 static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Traversal scheme index (traverse_queue MODE) from rumi_render_params.trace_mode:
-// 1..4 select modes 0..3, 0 selects the default, the speculative while-while walk (mode 3),
-// which measured fastest on the BVH-bound workload (238 vs 302 ms per 1024x1024x64 frame
-// for mode 0).
-static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? 4 : 3;
+// 1..5 select modes 0..4, 0 selects the default, the speculative while-while walk over the
+// four-wide tree (mode 3), the fastest on the BVH-bound workload.
 static inline int trace_scheme(int trace_mode) {
     return trace_mode >= 1 && trace_mode <= 5 ? trace_mode - 1 : DEFAULT_WALK_MODE;
 }
@@ -957,9 +961,8 @@ using ShadowKernel = void (*)(PtLaunch);
 
 // Shared-memory stack depth from rumi_render_params.stack_depth: 8, 16 or 32 entries per
 // thread (0 = 16).  Only the while-while walks (schemes 3 and 4) come in all three depths.
-// Measured on the 1024x1024x64 BVH-bound frame (binary walk, closest-hit ms): 8: 100.5,
-// 16: 100.3, 32 with the L1 carveout sized to it: 107.0 -- the 32-entry stack takes L1 that
-// node fetches use, and deeper entries are rare.
+// Measured on the 1024x1024x64 BVH-bound frame (four-wide walk, closest-hit / any-hit ms):
+// 8: 65.8 / 35.9, 16: 65.7 / 35.2, 32 with the L1 carveout sized to it: 65.5 / 35.2.
 static inline int stack_entries(int stack_depth) { return stack_depth == 8 || stack_depth == 32 ? stack_depth : 16; }
 
 // Kernel selection and launches.  A host build of this file (RUMI_HOST_BUILD: the kernels
@@ -1010,34 +1013,46 @@ static void launch_shadow(int mode, int smem, int grid, cudaStream_t st, const P
     shadow_kernel<ADJ>(mode, smem)<<<grid, TRACE_THREADS, 0, st>>>(L);
 }
 
-// Asks for just the shared memory the resident blocks' stacks need (`blocks` blocks of smem
-// entries per thread), so the rest of the unified L1 / shared storage stays L1.
-template <typename K>
-static void prefer_l1(K k, int smem, int blocks) {
-    const int need = blocks * smem * TRACE_THREADS * (int)sizeof(int);
-    int pct = (need * 100 + 228 * 1024 - 1) / (228 * 1024);
-    if (pct > 100) pct = 100;
-    cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+// Resident blocks per SM of a persistent traversal kernel, asked of the runtime once per kernel
+// and device (about 2 us a question, as long as a small frame's launch).  The first question
+// also sets the kernel's shared-memory preference to just what `blocks` resident blocks need, so
+// that the rest of the unified L1 / shared storage stays L1.
+static int resident_blocks(const void *k, int blocks) {
+    static std::mutex mutex;
+    static std::map<std::pair<const void *, int>, int> known;
+    int device = 0;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto it = known.find({k, device});
+    if (it != known.end()) return it->second;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k) == cudaSuccess) {
+        const int need = blocks * ((int)fa.sharedSizeBytes + 1024);  // 1 KB per block is the runtime's
+        const int pct = (need * 100 + 228 * 1024 - 1) / (228 * 1024);
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct > 100 ? 100 : pct);
+    }
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, TRACE_THREADS, 0) != cudaSuccess || occ < 1) return 1;
+    known[{k, device}] = occ;
+    return occ;
 }
 
-// Persistent grids: blocks per SM at the kernels' occupancy (capped by blocks_per_sm > 0).
-static void trace_grids(int mode, int smem, int num_sms, int blocks_per_sm, bool adj, int &grid, int &grid_sh) {
-    int occ = 0, occ_sh = 0;
-    const ExtendKernel ke = extend_kernel<false>(mode, smem);
-    const ShadowKernel ks = adj ? shadow_kernel<true>(mode, smem) : shadow_kernel<false>(mode, smem);
-    prefer_l1(ke, smem, trace_min_blocks(mode, true));
-    prefer_l1(extend_kernel<true>(mode, smem), smem, trace_min_blocks(mode, true));
-    prefer_l1(ks, smem, trace_min_blocks(mode, false));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ke, TRACE_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_sh, ks, TRACE_THREADS, 0);
-    if (occ < 1) occ = 1;
-    if (occ_sh < 1) occ_sh = 1;
-    if (blocks_per_sm > 0) {
-        occ = blocks_per_sm < occ ? blocks_per_sm : occ;
-        occ_sh = blocks_per_sm < occ_sh ? blocks_per_sm : occ_sh;
-    }
-    grid = num_sms * occ;
-    grid_sh = num_sms * occ_sh;
+// Persistent grid of a traversal kernel for at most n rays: blocks per SM at the kernel's
+// occupancy (capped by blocks_per_sm > 0), and no block that could not get a ray.
+template <typename K>
+static int trace_grid(K k, int min_blocks, int num_sms, int blocks_per_sm, long long n) {
+    int occ = resident_blocks((const void *)k, min_blocks);
+    if (blocks_per_sm > 0 && blocks_per_sm < occ) occ = blocks_per_sm;
+    const long long useful = (n + TRACE_THREADS - 1) / TRACE_THREADS, all = (long long)num_sms * occ;
+    return (int)(useful < 1 ? 1 : (useful < all ? useful : all));
+}
+
+static void trace_grids(int mode, int smem, int num_sms, int blocks_per_sm, bool adj, bool stats, long long n, int &grid,
+                        int &grid_sh) {
+    grid = trace_grid(stats ? extend_kernel<true>(mode, smem) : extend_kernel<false>(mode, smem),
+                      trace_min_blocks(mode, true), num_sms, blocks_per_sm, n);
+    grid_sh = trace_grid(adj ? shadow_kernel<true>(mode, smem) : shadow_kernel<false>(mode, smem),
+                         trace_min_blocks(mode, false), num_sms, blocks_per_sm, n);
 }
 
 #endif  // RUMI_HOST_BUILD
@@ -1133,11 +1148,10 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
     const int mode = trace_scheme(p->trace_mode);
     const int smem = stack_entries(p->stack_depth);
     L.refill_min = p->refill_min > 0 ? p->refill_min : 8;
-    int trace_grid = 0, shadow_grid = 0;
-    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, false, trace_grid, shadow_grid);
-
     const bool timing = (p->flags & RUMI_FLAG_TIMING) != 0;
     const bool count_stats = (p->flags & RUMI_FLAG_STATS) != 0;
+    int grid = 0, shadow_grid = 0;
+    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, false, count_stats, (long long)Wp, grid, shadow_grid);
     const bool lean = shade_lean(sc);
     std::vector<cudaEvent_t> evs;
     auto mark_on = [&](cudaStream_t st_) {
@@ -1170,9 +1184,9 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
                 int e0 = 0;
                 if (timing) { e0 = (int)evs.size(); mark(); }
                 if (count_stats)
-                    launch_extend<true>(mode, smem, trace_grid, stream, L, b);
+                    launch_extend<true>(mode, smem, grid, stream, L, b);
                 else
-                    launch_extend<false>(mode, smem, trace_grid, stream, L, b);
+                    launch_extend<false>(mode, smem, grid, stream, L, b);
                 if (timing) { mark(); ext_ev.push_back({e0, e0 + 1}); }
                 if (b > 0) cudaStreamWaitEvent(stream, sc->ev_join, 0);
                 pt_reset_shade<<<1, 1, 0, stream>>>(L, b);
@@ -1206,9 +1220,9 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
             int e0 = 0;
             if (timing) { e0 = (int)evs.size(); mark(); }
             if (count_stats)
-                launch_extend<true>(mode, smem, trace_grid, stream, L, b);
+                launch_extend<true>(mode, smem, grid, stream, L, b);
             else
-                launch_extend<false>(mode, smem, trace_grid, stream, L, b);
+                launch_extend<false>(mode, smem, grid, stream, L, b);
             if (timing) { mark(); ext_ev.push_back({e0, e0 + 1}); }
             if (timing) { e0 = (int)evs.size(); mark(); }
             if (whitted)
@@ -1333,8 +1347,8 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
     const int smem = stack_entries(p->stack_depth);
     A.refill_min = B.refill_min = p->refill_min > 0 ? p->refill_min : 8;
     int grid = 0, grid_sh = 0, grid_dummy = 0, grid_sh_adj = 0;
-    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, false, grid, grid_sh);
-    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, true, grid_dummy, grid_sh_adj);
+    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, false, false, (long long)Wp, grid, grid_sh);
+    trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, true, false, (long long)Wp, grid_dummy, grid_sh_adj);
 
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (p->flags & RUMI_FLAG_TIMING) {
@@ -1447,26 +1461,20 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
     L.refill_min = 8;
     cudaMemsetAsync(L.cnt, 0, C_NUM * sizeof(int), stream);
     cudaMemsetAsync(L.stats, 0, S_NUM * sizeof(unsigned long long), stream);
-    int occ = 0, occ_sh = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pt_trace_multi<false>, TRACE_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_sh, pt_trace_multi<true>, TRACE_THREADS, 0);
-    if (occ < 1) occ = 1;
-    if (occ_sh < 1) occ_sh = 1;
-    if (F.blocks_per_sm > 0) {
-        occ = F.blocks_per_sm < occ ? F.blocks_per_sm : occ;
-        occ_sh = F.blocks_per_sm < occ_sh ? F.blocks_per_sm : occ_sh;
-    }
+    const int mb = trace_min_blocks(DEFAULT_WALK_MODE, true), mb_sh = trace_min_blocks(DEFAULT_WALK_MODE, false);
     for (const BatchWave &wv : F.waves) {
         L.pix0 = (int)wv.pix0;
         L.n_pix = (int)(wv.pix1 - wv.pix0);
         L.path0 = wv.path0;
         L.n_paths = (int)(wv.path1 - wv.path0);
+        const int grid = trace_grid(pt_trace_multi<false>, mb, num_sms, F.blocks_per_sm, L.n_paths);
+        const int grid_sh = trace_grid(pt_trace_multi<true>, mb_sh, num_sms, F.blocks_per_sm, L.n_paths);
         pt_generate<<<cdiv(L.n_paths, 256), 256, 0, stream>>>(L);
         // the two-stream schedule of pt_render_in (a graph capture takes the auxiliary
         // stream in through the fork event and every fork is joined before shading)
         for (int b = 0; b < F.max_depth; ++b) {
             pt_reset_extend<<<1, 1, 0, stream>>>(L, b);
-            pt_trace_multi<false><<<num_sms * occ, TRACE_THREADS, 0, stream>>>(L, b);
+            pt_trace_multi<false><<<grid, TRACE_THREADS, 0, stream>>>(L, b);
             if (b > 0 && aux) cudaStreamWaitEvent(stream, ev_join, 0);
             pt_reset_shade<<<1, 1, 0, stream>>>(L, b);
             launch_shade(F.lean, stream, L, b);
@@ -1475,7 +1483,7 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
                 cudaEventRecord(ev_fork, stream);
                 cudaStreamWaitEvent(aux, ev_fork, 0);
             }
-            pt_trace_multi<true><<<num_sms * occ_sh, TRACE_THREADS, 0, aside ? aux : stream>>>(L, b);
+            pt_trace_multi<true><<<grid_sh, TRACE_THREADS, 0, aside ? aux : stream>>>(L, b);
             if (aside) cudaEventRecord(ev_join, aux);
         }
         pt_finish<<<1, 1, 0, stream>>>(L);
@@ -1507,9 +1515,10 @@ struct TraceLaunch {
 // Ray queries: the renderer's default traversal scheme (speculative while-while with
 // per-lane refill) over a caller's ray array, in chunks of at most 2^30 rays.
 template <int MODE, bool ANYHIT, bool STATS>
-__global__ void __launch_bounds__(TRACE_THREADS, RUMI_TRACE_MIN_BLOCKS) trace_batch_kernel(TraceLaunch T, long long first,
-                                                                                         int n, int *fetch_counter) {
-    __shared__ int stack[STACK_SMEM * TRACE_THREADS];
+__global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, !ANYHIT))
+    trace_batch_kernel(TraceLaunch T, long long first, int n, int *fetch_counter) {
+    constexpr int SMEM = MODE == 3 ? WALK_SMEM : STACK_SMEM;
+    __shared__ int stack[SMEM * TRACE_THREADS];
     TraceStats st{0, 0};
     auto fetch = [&](int i, float3 &o, float3 &d, float &tmax, bool &in_obj) {
         const long long k = first + i;
@@ -1524,8 +1533,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, RUMI_TRACE_MIN_BLOCKS) trace_ba
         T.t[k] = h.t;
         T.prim[k] = ANYHIT ? (h.t > 0.0f ? 1 : 0) : (h.t > 0.0f ? h.id : -1);
     };
-    traverse_queue<MODE, ANYHIT, STACK_SMEM, STATS>(T.s, n, fetch_counter, 8, stack + threadIdx.x, TRACE_THREADS,
-                                                    fetch, finish, st);
+    traverse_queue<MODE, ANYHIT, SMEM, STATS>(T.s, n, fetch_counter, 8, stack, fetch, finish, st);
     if (STATS) {
         atomicAdd(&T.counters[1], (unsigned long long)st.nodes);
         atomicAdd(&T.counters[2], (unsigned long long)st.prims);
@@ -1534,16 +1542,14 @@ __global__ void __launch_bounds__(TRACE_THREADS, RUMI_TRACE_MIN_BLOCKS) trace_ba
 
 template <bool ANYHIT, bool STATS, int MODE = DEFAULT_WALK_MODE>
 static void launch_trace_batch(const TraceLaunch &T, int num_sms, cudaStream_t stream) {
-    int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_batch_kernel<MODE, ANYHIT, STATS>, TRACE_THREADS, 0);
-    if (occ < 1) occ = 1;
     const long long chunk = 1LL << 30;
     int k = 0;
     for (long long first = 0; first < T.n; first += chunk, ++k) {
         const int n = (int)(T.n - first < chunk ? T.n - first : chunk);
         // one fetch counter per chunk (counters[3 + k]; chunk count is bounded by the caller's n)
         int *ctr = reinterpret_cast<int *>(T.counters + 3) + k;
-        trace_batch_kernel<MODE, ANYHIT, STATS><<<num_sms * occ, TRACE_THREADS, 0, stream>>>(T, first, n, ctr);
+        const int grid = trace_grid(trace_batch_kernel<MODE, ANYHIT, STATS>, trace_min_blocks(MODE, !ANYHIT), num_sms, 0, n);
+        trace_batch_kernel<MODE, ANYHIT, STATS><<<grid, TRACE_THREADS, 0, stream>>>(T, first, n, ctr);
     }
 }
 

@@ -2,12 +2,13 @@
 //
 // HBM layout (all arrays cudaMalloc'd by rumi_scene_create, 256-byte aligned):
 //   nodes      : BvhNode[n_nodes]        32 B each; siblings adjacent, pairs 64-B aligned
-//   nodes4     : Bvh4Node[n_nodes4]      128 B each, collapsed from `nodes`; siblings adjacent
 //   nodes8     : Bvh8Node[n_nodes8]      80 B each, compressed eight-wide tree collapsed from
 //                                        `nodes`; a node's interior children are adjacent
 //   prims8     : float4[3 * n_prims]     the leaf primitives re-laid out for nodes8: the leaf
 //                                        children of one node are adjacent, in slot order
 //   leaf_prims : float4[3 * n_prims]     48 B per primitive, in BVH leaf order
+//   wide       : WideNode[n_wide]       96 B each, `nodes` collapsed for the default walk
+//   recs       : LeafRec[n_recs]         96 B each, its leaves: two triangles per record
 //   tri_shade  : float4[3 * n_tris]      shading normals n0,n1,n2 (canonical order);
 //                                        .w of the first holds the material index
 //   tri_albedo : float4[n_tris]          optional per-triangle Matte colour (rgb)
@@ -43,29 +44,6 @@ struct __align__(16) BvhNode {
     int count;
 };
 
-// 128-byte four-wide node, collapsed from the binary tree (bvh4.cu): child boxes in SoA
-// order so a node is eight float4 loads (one 128-byte line).  count[i] > 0: leaf over
-// leaf_prims[child[i] .. child[i]+count[i]); count[i] == 0: interior child node
-// nodes4[child[i]]; count[i] < 0: empty slot (its box is empty).
-struct __align__(128) Bvh4Node {
-    float lo_x[4], hi_x[4];
-    float lo_y[4], hi_y[4];
-    float lo_z[4], hi_z[4];
-    int child[4];
-    int count[4];
-};
-
-// The four-wide tree halves the node steps per ray (34.6 vs 47.7 node units of 32 bytes per
-// camera ray on the 1M-triangle mesh, fewer primitive tests), but each step costs more issue
-// slots (four slabs, a sorting network, classification).  Measured per 1024x1024x64 frame on
-// B200: warp-batch walk, binary 143 / four-wide 178 ms of closest-hit; speculative while-while
-// walk (the default scheme), binary 100 / four-wide 130 ms (any-hit 83.5 / 87.8 ms).  So the
-// binary tree is the default and the four-wide tree is built and walked only when this is 1
-// (both walks pass the same hit and image parity tests).
-#ifndef RUMI_BVH_WIDE
-#define RUMI_BVH_WIDE 0  // 1: walk the four-wide tree (nodes4), 0: the binary tree
-#endif
-
 // 80-byte compressed eight-wide node (five float4 loads), collapsed from the binary tree by
 // bvh8.cu.  Child boxes are stored as 8-bit multiples of a per-axis power-of-two quantum
 // 2^e relative to the origin (ox, oy, oz), rounded strictly outward by at least one
@@ -95,6 +73,8 @@ struct __align__(16) Bvh8Node {
     unsigned int qhi_x[2], qhi_y[2], qhi_z[2];  // byte k: high bound
 };
 static_assert(sizeof(Bvh8Node) == 80, "Bvh8Node is five float4");
+
+#include "wide.cuh"
 
 struct DevMaterial {
     int type;
@@ -163,8 +143,6 @@ struct DevScene {
     int n_tris, n_rects, n_spheres, n_prims;
     int n_materials, n_lights;
     int n_nodes;
-    const Bvh4Node *nodes4;     // the four-wide tree the traversal kernels walk
-    int n_nodes4;
     const Bvh8Node *nodes8;     // the compressed eight-wide tree (0 nodes: empty scene)
     const float4 *prims8;       // leaf primitives in nodes8 order
     int n_nodes8;
@@ -176,6 +154,9 @@ struct DevScene {
     const int *prim_tex;
     const float4 *sphere_frame;
     int n_textures;
+    // the four-wide tree of the default walk (wide.cuh): six float4 per WideNode and per LeafRec
+    const float4 *wide;
+    const float4 *recs;
 };
 
 // Canonical primitive id -> material index.

@@ -9,18 +9,19 @@
 // The running closest distance plays the role of Ray::_tmin (0 = nothing hit yet), with
 // the same tie rule: an equal t replaces the previous hit.
 //
-// Traversal: both children of an interior node are adjacent (one 64-byte pair, four
-// float4 loads); leaf children are intersected at once, interior children are visited
-// near-first with the far one pushed.  The stack keeps its top STACK_SMEM entries in
+// The default walk reads the four-wide tree (wide.cuh).  In the binary walks both children of an
+// interior node are adjacent (one 64-byte pair, four float4 loads); leaf children are
+// intersected at once, interior children are visited near-first with the far one pushed.  The stack keeps its top STACK_SMEM entries in
 // shared memory (one column per thread) and spills deeper entries to a local array.
 #pragma once
 #include <cfloat>
+#include <type_traits>
 #include "scene.cuh"
 
 #define RUMI_MAX_BVH_DEPTH 64
 
 // 1: the default walk (trace_mode 0, ray queries, batches, per-thread rays) is the
-// compressed eight-wide tree; 0: the binary (or, with RUMI_BVH_WIDE, four-wide) tree.
+// compressed eight-wide tree; 0: the four-wide tree (per-thread rays: the binary one).
 #ifndef RUMI_WALK8
 #define RUMI_WALK8 0
 #endif
@@ -160,7 +161,7 @@ RUMI_D float cull_limit(float best_t, float tmax) {
 }
 
 struct TraceStats {
-    int nodes;   // node bytes fetched, in 16-byte units (a binary node is 2, an eight-wide node 5)
+    int nodes;   // node bytes fetched, in 16-byte units (a binary node is 2, a four-wide 6, an eight-wide 5)
     int prims;   // primitives tested
 };
 
@@ -292,134 +293,6 @@ RUMI_D HitRec trace_ray_bin(const DevScene &s, float3 o, float3 d, float tmax, b
     return h;
 }
 
-// ------------------------------------------------------------ four-wide traversal
-// Stack entries: at most three pushes per four-wide level.
-#define RUMI_STACK4 (3 * RUMI_MAX_BVH_DEPTH)
-
-RUMI_D bool slab_s(float lx, float ly, float lz, float hx, float hy, float hz, float3 inv, float3 oinv, float tlimit,
-                   float &tnear) {
-    const float tx0 = fmaf(lx, inv.x, -oinv.x), tx1 = fmaf(hx, inv.x, -oinv.x);
-    const float ty0 = fmaf(ly, inv.y, -oinv.y), ty1 = fmaf(hy, inv.y, -oinv.y);
-    const float tz0 = fmaf(lz, inv.z, -oinv.z), tz1 = fmaf(hz, inv.z, -oinv.z);
-    const float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fminf(tz0, tz1));
-    const float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
-    tnear = tn;
-    return tn <= tf && tf >= 0.0f && tn <= tlimit;
-}
-
-RUMI_D int sel4(int4 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
-
-#define RUMI_CSWAP(ka, sa, kb, sb)                  \
-    if (kb < ka) {                                  \
-        const float tk_ = ka; ka = kb; kb = tk_;    \
-        const int ts_ = sa; sa = sb; sb = ts_;      \
-    }
-
-// The same query over the four-wide tree: a node's four child boxes are tested together
-// and visited nearest first (leaves intersected at once, interior children: the nearest
-// next, the others pushed farthest first).
-template <bool ANYHIT, int STACK_SMEM, bool STATS>
-RUMI_D HitRec trace_ray_wide(const DevScene &s, float3 o, float3 d, float tmax, bool in_object, int *smem_stack,
-                             int stride, TraceStats &st) {
-    HitRec h;
-    h.t = 0.0f;
-    h.id = -1;
-    h.u = h.v = 0.0f;
-    h.back = 0;
-    if (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f) return h;  // bvh.cpp:161-162
-    if (s.n_nodes4 <= 0) return h;
-    const float3 inv = safe_inv(d);
-    const float3 oinv = mk3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-    int spill[RUMI_STACK4 - STACK_SMEM > 0 ? RUMI_STACK4 - STACK_SMEM : 1];
-    int sp = 0;
-    int cur = 0;
-    // every node is visited at most once per ray, so the bound is never reached by a
-    // well-formed tree; it keeps a malformed one from looping
-    for (int guard = 0; guard < s.n_nodes4; ++guard) {
-        const float4 *np = reinterpret_cast<const float4 *>(s.nodes4 + cur);
-        const float4 lx = __ldg(np + 0), hx = __ldg(np + 1), ly = __ldg(np + 2), hy = __ldg(np + 3);
-        const float4 lz = __ldg(np + 4), hz = __ldg(np + 5);
-        const int4 ch = __ldg(reinterpret_cast<const int4 *>(np + 6));
-        const int4 cn = __ldg(reinterpret_cast<const int4 *>(np + 7));
-        if (STATS) st.nodes += 8;  // counted in 16-byte units
-        const float lim = cull_limit(h.t, tmax);
-        float k0, k1, k2, k3;
-        if (!(cn.x >= 0 && slab_s(lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, inv, oinv, lim, k0))) k0 = FLT_MAX;
-        if (!(cn.y >= 0 && slab_s(lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, inv, oinv, lim, k1))) k1 = FLT_MAX;
-        if (!(cn.z >= 0 && slab_s(lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, inv, oinv, lim, k2))) k2 = FLT_MAX;
-        if (!(cn.w >= 0 && slab_s(lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, inv, oinv, lim, k3))) k3 = FLT_MAX;
-        int s0 = 0, s1 = 1, s2 = 2, s3 = 3;
-        if (!ANYHIT) {  // near-first order; occlusion queries take any order
-            RUMI_CSWAP(k0, s0, k1, s1);
-            RUMI_CSWAP(k2, s2, k3, s3);
-            RUMI_CSWAP(k0, s0, k2, s2);
-            RUMI_CSWAP(k1, s1, k3, s3);
-            RUMI_CSWAP(k1, s1, k2, s2);
-        }
-        // split the hit children (in that order) into leaves and interior nodes
-        int lf0 = 0, lf1 = 0, lf2 = 0, lf3 = 0, lc0 = 0, lc1 = 0, lc2 = 0, lc3 = 0, nl = 0;
-        float lk0 = 0.0f, lk1 = 0.0f, lk2 = 0.0f, lk3 = 0.0f;
-        int c0 = -1, c1 = -1, c2 = -1, c3 = -1, ni = 0;
-        float ck0 = 0.0f, ck1 = 0.0f, ck2 = 0.0f, ck3 = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float kj = j == 0 ? k0 : (j == 1 ? k1 : (j == 2 ? k2 : k3));
-            const int sj = j == 0 ? s0 : (j == 1 ? s1 : (j == 2 ? s2 : s3));
-            if (kj == FLT_MAX) continue;
-            const int child = sel4(ch, sj), count = sel4(cn, sj);
-            if (count > 0) {
-                if (nl == 0) { lf0 = child; lc0 = count; lk0 = kj; }
-                else if (nl == 1) { lf1 = child; lc1 = count; lk1 = kj; }
-                else if (nl == 2) { lf2 = child; lc2 = count; lk2 = kj; }
-                else { lf3 = child; lc3 = count; lk3 = kj; }
-                ++nl;
-            } else {
-                if (ni == 0) { c0 = child; ck0 = kj; }
-                else if (ni == 1) { c1 = child; ck1 = kj; }
-                else if (ni == 2) { c2 = child; ck2 = kj; }
-                else { c3 = child; ck3 = kj; }
-                ++ni;
-            }
-        }
-        // leaves now, nearest first (one copy of the primitive loop)
-#pragma unroll 1
-        for (int q = 0; q < nl; ++q) {
-            const float lk = q == 0 ? lk0 : (q == 1 ? lk1 : (q == 2 ? lk2 : lk3));
-            if (!ANYHIT && h.t > 0.0f && lk > h.t) break;
-            const int lf = q == 0 ? lf0 : (q == 1 ? lf1 : (q == 2 ? lf2 : lf3));
-            const int lc = q == 0 ? lc0 : (q == 1 ? lc1 : (q == 2 ? lc2 : lc3));
-            if (leaf_isect<ANYHIT, STATS>(s, lf, lc, o, d, tmax, in_object, h, st)) return h;
-        }
-        // interior children beyond the closest hit so far are culled
-        if (!ANYHIT && h.t > 0.0f) {
-            if (ni > 3 && ck3 > h.t) ni = 3;
-            if (ni > 2 && ck2 > h.t) ni = 2;
-            if (ni > 1 && ck1 > h.t) ni = 1;
-            if (ni > 0 && ck0 > h.t) ni = 0;
-        }
-        int next;
-        if (ni == 0) {
-            if (sp == 0) break;
-            --sp;
-            next = sp < STACK_SMEM ? smem_stack[sp * stride] : spill[sp - STACK_SMEM];
-        } else {
-            next = c0;
-            // push the others farthest first, so the nearest of them is popped first
-            for (int k = ni - 1; k >= 1; --k) {
-                const int c = k == 3 ? c3 : (k == 2 ? c2 : c1);
-                if (sp < STACK_SMEM)
-                    smem_stack[sp * stride] = c;
-                else if (sp < RUMI_STACK4)
-                    spill[sp - STACK_SMEM] = c;
-                if (sp < RUMI_STACK4) ++sp;  // three per level of a depth-limited tree: always holds
-            }
-        }
-        if ((unsigned)next >= (unsigned)s.n_nodes4) break;  // malformed tree guard
-        cur = next;
-    }
-    return h;
-}
-
 template <bool ANYHIT, int STACK_SMEM, bool STATS>
 RUMI_D HitRec trace_ray_w8(const DevScene &s, float3 o, float3 d, float tmax, bool in_object, int *smem_stack,
                            int stride, TraceStats &st);
@@ -429,8 +302,6 @@ RUMI_D HitRec trace_ray(const DevScene &s, float3 o, float3 d, float tmax, bool 
                         int stride, TraceStats &st) {
 #if RUMI_WALK8
     return trace_ray_w8<ANYHIT, STACK_SMEM, STATS>(s, o, d, tmax, in_object, smem_stack, stride, st);
-#elif RUMI_BVH_WIDE
-    return trace_ray_wide<ANYHIT, STACK_SMEM, STATS>(s, o, d, tmax, in_object, smem_stack, stride, st);
 #else
     return trace_ray_bin<ANYHIT, STACK_SMEM, STATS>(s, o, d, tmax, in_object, smem_stack, stride, st);
 #endif
@@ -620,60 +491,220 @@ RUMI_D bool run_pending(const DevScene &s, TravState &T, PendingLeaves &pl, Trac
     return found;
 }
 
-// Speculative while-while traversal with per-lane refill (Aila & Laine, "Understanding
-// the efficiency of ray traversal on GPUs", HPG 2009; Aila, Laine & Karras 2012): each
-// lane walks interior node pairs until it holds a postponed leaf, and keeps walking
-// (speculatively) until every lane of the warp holds one; then the warp intersects the
-// postponed leaves together.  Rounds repeat until a lane's ray is finished, and finished
-// lanes are refilled from the queue in warp-aggregated batches.
-//   cur >= 0: a node pair to test; cur < 0, != WW_DONE: the leaf node -(cur + 1);
-//   WW_DONE: the stack is empty.
-#define WW_DONE (-0x7fffffff - 1)
+// ------------------------------------------------------------------ four-wide walk
+// Two floats in one 64-bit register; the packed operations round each half as the scalar
+// ones do.
+#ifdef RUMI_HOST_BUILD
+struct f2 {
+    float a, b;
+};
+RUMI_D f2 pk(float a, float b) { return {a, b}; }
+RUMI_D void unpk(f2 v, float &a, float &b) { a = v.a; b = v.b; }
+RUMI_D f2 fma2(f2 a, f2 b, f2 c) { return {fmaf(a.a, b.a, c.a), fmaf(a.b, b.b, c.b)}; }
+RUMI_D f2 mul2(f2 a, f2 b) { return {a.a * b.a, a.b * b.b}; }
+RUMI_D f2 add2(f2 a, f2 b) { return {a.a + b.a, a.b + b.b}; }
+RUMI_D f2 sub2(f2 a, f2 b) { return {a.a - b.a, a.b - b.b}; }
+RUMI_D float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+RUMI_D float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
+RUMI_D void ldg32(const float4 *p, float4 &a, float4 &b) { a = p[0]; b = p[1]; }
+#else
+typedef unsigned long long f2;
+RUMI_D f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+RUMI_D void unpk(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+RUMI_D f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+RUMI_D f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Sums as fma by 1 and -1 read from constant memory: the assembler contracts a packed
+// product and a packed add or subtract into one fma (its .rn notwithstanding; a million random
+// pairs showed it), which these values, unknown to it, keep it from doing.
+__constant__ float2 c_ones[2] = {{1.0f, 1.0f}, {-1.0f, -1.0f}};
+RUMI_D f2 add2(f2 a, f2 b) { return fma2(a, pk(c_ones[0].x, c_ones[0].y), b); }
+RUMI_D f2 sub2(f2 a, f2 b) { return fma2(b, pk(c_ones[1].x, c_ones[1].y), a); }
+RUMI_D float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+RUMI_D float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// 32 bytes (32-byte aligned, read-only) in one load.
+RUMI_D void ldg32(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+#endif
 
-// scene_of(i): the scene ray i is traced in (one scene, or per ray in a multi-scene batch).
-template <bool ANYHIT, int STACK_SMEM, bool STATS, typename SceneOf, typename Fetch, typename Finish>
-RUMI_D void traverse_queue_ww(SceneOf scene_of, int n, int *counter, int refill_min, int *smem_stack, int stride,
-                              Fetch fetch, Finish finish, TraceStats &st) {
+// isect_triangle's acceptance on its u, v, t and determinant (the same rounded values).
+RUMI_D bool accept_triangle(float det, float un, float vn, float tn, float tmax, int id, HitRec &h) {
+    if (fabsf(det) < 1e-8f) return false;
+    const float inv_det = __frcp_rn(det);
+    const float u = __fmul_rn(un, inv_det);
+    if (u < 0.0f || u > 1.0f) return false;
+    const float v = __fmul_rn(vn, inv_det);
+    if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
+    const float t = __fmul_rn(tn, inv_det);
+    if (t < RUMI_EPS) return false;
+    if (h.t > RUMI_EPS && t > h.t) return false;
+    if (__fsub_rn(tmax, t) < RUMI_EPS) return false;
+    if (t == h.t && id < h.id) return false;  // a tie: the larger id stays
+    h.t = t;
+    h.id = id;
+    h.u = u;
+    h.v = v;
+    h.back = det < 0.0f;
+    return true;
+}
+
+// What the record test reads of a ray, from shared memory: direction and origin with every
+// component twice, so that a load gives the operand pairs of the packed operations.
+struct RayPairs {
+    float4 a, b, c;  // (dx dx dy dy) (dz dz ox ox) (oy oy oz oz)
+};
+
+// One leaf record: both triangles of a pair in packed operations (isect_triangle's
+// operations in its order, two at a time), or its one rect or sphere.
+template <bool ANYHIT, bool STATS>
+RUMI_D bool rec_isect(const float4 *__restrict__ recs, int i, const RayPairs &rp, float tmax, bool in_object, HitRec &h,
+                      bool &last, TraceStats &st) {
+    const float4 *r = recs + 6 * (size_t)i;
+    float4 A, B, C, D, E, F;
+    ldg32(r, A, B);
+    ldg32(r + 2, C, D);
+    ldg32(r + 4, E, F);
+    const unsigned w = __float_as_uint(E.z);
+    last = (w & REC_LAST) != 0;
+    const int id0 = (int)(w & REC_ID);
+    if (w & REC_SINGLE) {
+        const float3 d = mk3(rp.a.x, rp.a.z, rp.b.x), o = mk3(rp.b.z, rp.c.x, rp.c.z);
+        if (STATS) st.prims++;
+        const int tag = __float_as_int(B.w);
+        float t;
+        const bool ok = (tag & 0xff) == PRIM_RECT
+                            ? isect_rect(o, d, tmax, h.t, A, B, C, (tag & PRIM_FLAG_EMISSIVE) != 0, t)
+                            : isect_sphere(o, d, tmax, h.t, A, B, in_object && !ANYHIT, (tag & PRIM_FLAG_IBL) != 0, t);
+        if (!ok || (t == h.t && id0 < h.id)) return false;
+        h.t = t;
+        h.id = id0;
+        h.u = h.v = 0.0f;
+        h.back = 0;
+        return true;
+    }
+    const int id1 = __float_as_int(E.w);
+    if (STATS) st.prims += id0 == id1 ? 1 : 2;
+    const f2 dx = pk(rp.a.x, rp.a.y), dy = pk(rp.a.z, rp.a.w), dz = pk(rp.b.x, rp.b.y);
+    const f2 e1x = pk(B.z, B.w), e1y = pk(C.x, C.y), e1z = pk(C.z, C.w);
+    const f2 e2x = pk(D.x, D.y), e2y = pk(D.z, D.w), e2z = pk(E.x, E.y);
+    const f2 Px = sub2(mul2(dy, e2z), mul2(e2y, dz));
+    const f2 Py = sub2(mul2(dz, e2x), mul2(e2z, dx));
+    const f2 Pz = sub2(mul2(dx, e2y), mul2(e2x, dy));
+    const f2 det = add2(add2(mul2(Px, e1x), mul2(Py, e1y)), mul2(Pz, e1z));
+    const f2 Tx = add2(pk(rp.b.z, rp.b.w), pk(A.x, A.y)), Ty = add2(pk(rp.c.x, rp.c.y), pk(A.z, A.w)),
+             Tz = add2(pk(rp.c.z, rp.c.w), pk(B.x, B.y));
+    const f2 un = add2(add2(mul2(Px, Tx), mul2(Py, Ty)), mul2(Pz, Tz));
+    const f2 Qx = sub2(mul2(Ty, e1z), mul2(e1y, Tz));
+    const f2 Qy = sub2(mul2(Tz, e1x), mul2(e1z, Tx));
+    const f2 Qz = sub2(mul2(Tx, e1y), mul2(e1x, Ty));
+    const f2 vn = add2(add2(mul2(Qx, dx), mul2(Qy, dy)), mul2(Qz, dz));
+    const f2 tn = add2(add2(mul2(Qx, e2x), mul2(Qy, e2y)), mul2(Qz, e2z));
+    float det0, det1, u0, u1, v0, v1, t0, t1;
+    unpk(det, det0, det1);
+    unpk(un, u0, u1);
+    unpk(vn, v0, v1);
+    unpk(tn, t0, t1);
+    bool hit = accept_triangle(det0, u0, v0, t0, tmax, id0, h);
+    hit |= accept_triangle(det1, u1, v1, t1, tmax, id1, h);
+    return hit;
+}
+
+// Speculative while-while traversal with per-lane refill (Aila & Laine, "Understanding
+// the efficiency of ray traversal on GPUs", HPG 2009; Aila, Laine & Karras 2012) over the
+// four-wide tree (wide.cuh): each lane walks interior nodes until it holds a postponed leaf, and
+// keeps walking (speculatively) until every lane of the warp holds one; then the warp intersects
+// the postponed leaves together, a record per lane and turn.  Rounds repeat until a lane's ray is
+// finished, and finished lanes are refilled from the queue in warp-aggregated batches.
+//   cur >= 0: a node to test; cur < 0, != WW_DONE: the leaf at record ~cur; WW_DONE: the stack is
+//   empty.
+// A child's index is larger than its parent's and a leaf's last record is marked (bvh_wide.cu
+// builds no other tree), so every ray ends and every index is in range.
+//
+// Of a node's hit children the nearest is next and the others wait unsorted: a full order
+// costs more half-rate operations than it saves visits, and an occlusion query that takes
+// the first hit child instead is 4% slower.  Entry distances are not kept on the stack: dropping
+// children beyond the best hit when they are popped saves 5% of the visits, but with the entry
+// twice as large the frame's closest-hit time is 76 ms instead of 72.
+#define WW_DONE (-0x7fffffff - 1)
+#define WW_THREADS 128               // threads per block of the kernels that run this walk
+#define WW_DEEP (3 * RUMI_MAX_BVH_DEPTH)  // a node leaves at most three children behind
+
+// scene_of(i): the scene ray i is traced in (MULTI: per ray, of a multi-scene batch).
+template <bool ANYHIT, int STACK_SMEM, bool STATS, bool MULTI, typename SceneOf, typename Fetch, typename Finish>
+RUMI_D void traverse_queue_ww(SceneOf scene_of, int n, int *counter, int refill_min, int *smem_stack, Fetch fetch,
+                              Finish finish, TraceStats &st) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    int spill[RUMI_MAX_BVH_DEPTH - STACK_SMEM > 0 ? RUMI_MAX_BVH_DEPTH - STACK_SMEM : 1];
-    const DevScene *sp_scene = scene_of(-1);
-    const float4 *nodes = reinterpret_cast<const float4 *>(sp_scene->nodes);
-    float3 o = mk3(0, 0, 0), d = mk3(0, 0, 0), inv = mk3(0, 0, 0), oinv = mk3(0, 0, 0);
-    float tmax = 0.0f;
+    // The stack's top entries are in shared memory, a column per thread (smem_stack: the block's
+    // STACK_SMEM * WW_THREADS ints); what does not fit moves to local memory half a column at a
+    // time, so that a push is a store and an add.
+    const int bottom = threadIdx.x, full = bottom + (STACK_SMEM - 3) * WW_THREADS;
+    constexpr int HALF = STACK_SMEM / 2;
+    int deep[WW_DEEP];
+    int top = bottom, n_deep = 0;
+    // only the record tests need the ray itself
+    __shared__ float2 s_ray[3 * WW_THREADS];  // (dx dy) (dz ox) (oy oz) of each thread
+    float2 *const my_ray = s_ray + threadIdx.x;
+    const DevScene *sc = scene_of(-1);
+    const float4 *wide = sc->wide, *recs = sc->recs;
+    float3 inv = mk3(0, 0, 0), noi = mk3(0, 0, 0);  // 1 / d and -o / d
+    float tmax = 0.0f, lim = 0.0f;
     bool in_obj = false;
     HitRec h;
     h.t = 0.0f;
     h.id = -1;
     h.u = h.v = 0.0f;
     h.back = 0;
-    int ray = -1, cur = WW_DONE, sp = 0, lf_first = 0, lf_count = 0, steps = 0;
+    int ray = -1, cur = WW_DONE, leaf = 0;
     bool exhausted = false;
-    auto pop = [&]() -> int {
-        if (sp == 0) return WW_DONE;
-        --sp;
-        return sp < STACK_SMEM ? smem_stack[sp * stride] : spill[sp - STACK_SMEM];
+    // the next node or second leaf from the stack; a leaf met first is postponed
+    auto pop = [&]() {
+        cur = WW_DONE;
+        for (;;) {
+            if (top == bottom) {
+                if (n_deep == 0) return;
+                for (int k = 0; k < HALF; ++k) smem_stack[bottom + k * WW_THREADS] = deep[n_deep - HALF + k];
+                n_deep -= HALF;
+                top = bottom + HALF * WW_THREADS;
+            }
+            top -= WW_THREADS;
+            const int v = smem_stack[top];
+            if (v >= 0 || leaf < 0) {
+                cur = v;
+                return;
+            }
+            leaf = v;
+        }
     };
     auto push = [&](int v) {
-        if (sp < STACK_SMEM)
-            smem_stack[sp * stride] = v;
-        else if (sp < RUMI_MAX_BVH_DEPTH)
-            spill[sp - STACK_SMEM] = v;
-        if (sp < RUMI_MAX_BVH_DEPTH) ++sp;  // the build caps depth at 63: always holds
-    };
-    // leaf node -> pending leaf range (a range check keeps a malformed tree harmless)
-    auto take_leaf = [&](int node) {
-        if ((unsigned)node >= (unsigned)sp_scene->n_nodes) {
-            lf_count = 0;
-            return;
-        }
-        const float4 b = __ldg(nodes + 2 * node + 1);
-        lf_first = __float_as_int(b.z);
-        lf_count = __float_as_int(b.w);
+        smem_stack[top] = v;
+        top += WW_THREADS;
     };
     for (;;) {
         // finished rays -> results; idle lanes -> new rays
-        if (ray >= 0 && cur == WW_DONE && lf_count == 0) {
+        if (ray >= 0 && cur == WW_DONE && leaf == 0) {
             finish(ray, h);
             ray = -1;
         }
@@ -688,232 +719,115 @@ RUMI_D void traverse_queue_ww(SceneOf scene_of, int n, int *counter, int refill_
                 const int r = base + __popc(idle & lt);
                 if (r < n) {
                     ray = r;
+                    float3 o, d;
                     fetch(r, o, d, tmax, in_obj);
-                    sp_scene = scene_of(r);
-                    nodes = reinterpret_cast<const float4 *>(sp_scene->nodes);
+                    my_ray[0] = make_float2(d.x, d.y);
+                    my_ray[WW_THREADS] = make_float2(d.z, o.x);
+                    my_ray[2 * WW_THREADS] = make_float2(o.y, o.z);
+                    if (MULTI) {
+                        sc = scene_of(r);
+                        wide = sc->wide;
+                        recs = sc->recs;
+                    }
                     h.t = 0.0f;
                     h.id = -1;
                     h.u = h.v = 0.0f;
                     h.back = 0;
-                    sp = 0;
-                    steps = 0;
-                    cur = WW_DONE;
-                    lf_count = 0;
-                    if (!(d.x == 0.0f && d.y == 0.0f && d.z == 0.0f)) {  // bvh.cpp:161-162
-                        inv = safe_inv(d);
-                        oinv = mk3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-                        const float4 a = __ldg(nodes), b = __ldg(nodes + 1);
-                        if (STATS) st.nodes += 2;
-                        float tn;
-                        if (slab(a, b, inv, oinv, tmax, tn)) {
-                            const int first = __float_as_int(b.z), count = __float_as_int(b.w);
-                            if (count > 0) {
-                                lf_first = first;
-                                lf_count = count;
-                            } else if ((unsigned)first < (unsigned)(sp_scene->n_nodes - 1)) {
-                                cur = first;
-                            }
-                        }
-                    }
+                    lim = tmax;
+                    top = bottom;
+                    n_deep = 0;
+                    leaf = 0;
+                    inv = safe_inv(d);
+                    noi = mk3(-(o.x * inv.x), -(o.y * inv.y), -(o.z * inv.z));
+                    // no direction, no hit (bvh.cpp:161-162)
+                    cur = d.x == 0.0f && d.y == 0.0f && d.z == 0.0f ? WW_DONE : 0;
                 }
             }
         }
         if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        // interior node pairs, speculatively past the first leaf
+        // interior nodes, speculatively past the first leaf
         while (cur >= 0) {
-            if ((unsigned)cur >= (unsigned)(sp_scene->n_nodes - 1) || ++steps > sp_scene->n_nodes) {  // malformed tree guard
-                cur = WW_DONE;
-                lf_count = 0;
-                break;
-            }
-            const float4 a0 = __ldg(nodes + 2 * cur), b0 = __ldg(nodes + 2 * cur + 1);
-            const float4 a1 = __ldg(nodes + 2 * cur + 2), b1 = __ldg(nodes + 2 * cur + 3);
-            if (STATS) st.nodes += 4;
-            const float lim = cull_limit(h.t, tmax);
-            float tn0, tn1;
-            const bool h0 = slab(a0, b0, inv, oinv, lim, tn0);
-            const bool h1 = slab(a1, b1, inv, oinv, lim, tn1);
-            const int c0 = __float_as_int(b0.w), c1 = __float_as_int(b1.w);
-            const bool v0 = h0 && c0 >= 0, v1 = h1 && c1 >= 0;
-            const int e0 = c0 > 0 ? -(cur + 1) : __float_as_int(b0.z);
-            const int e1 = c1 > 0 ? -(cur + 2) : __float_as_int(b1.z);
-            if (v0 && v1) {
-                const bool sw = tn1 < tn0;
-                cur = sw ? e1 : e0;
-                push(sw ? e0 : e1);
-            } else if (v0) {
-                cur = e0;
-            } else if (v1) {
-                cur = e1;
-            } else {
-                cur = pop();
-            }
-            if (cur < 0 && cur != WW_DONE && lf_count == 0) {  // postpone the leaf, keep walking
-                take_leaf(-cur - 1);
-                cur = pop();
-            }
-            if (!__any_sync(__activemask(), lf_count == 0 && cur >= 0)) break;
-        }
-        // the postponed leaves, then any leaf the walk stopped at
-        while (lf_count > 0) {
-            if (leaf_isect<ANYHIT, STATS>(*sp_scene, lf_first, lf_count, o, d, tmax, in_obj, h, st)) {
-                cur = WW_DONE;
-                lf_count = 0;
-                break;
-            }
-            lf_count = 0;
-            if (cur < 0 && cur != WW_DONE) {
-                take_leaf(-cur - 1);
-                cur = pop();
-            }
-        }
-    }
-}
-
-// The same speculative while-while walk over the four-wide tree (nodes4): an interior
-// step tests a node's four child boxes, continues with the nearest hit child and pushes
-// the others farthest first; leaf children are stack entries -(1 + 4 * node + slot).
-template <bool ANYHIT, int STACK_SMEM, bool STATS, typename SceneOf, typename Fetch, typename Finish>
-RUMI_D void traverse_queue_ww4(SceneOf scene_of, int n, int *counter, int refill_min, int *smem_stack, int stride,
-                               Fetch fetch, Finish finish, TraceStats &st) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    int spill[RUMI_STACK4 - STACK_SMEM > 0 ? RUMI_STACK4 - STACK_SMEM : 1];
-    const DevScene *sp_scene = scene_of(-1);
-    const float4 *nodes = reinterpret_cast<const float4 *>(sp_scene->nodes4);
-    float3 o = mk3(0, 0, 0), d = mk3(0, 0, 0), inv = mk3(0, 0, 0), oinv = mk3(0, 0, 0);
-    float tmax = 0.0f;
-    bool in_obj = false;
-    HitRec h;
-    h.t = 0.0f;
-    h.id = -1;
-    h.u = h.v = 0.0f;
-    h.back = 0;
-    int ray = -1, cur = WW_DONE, sp = 0, lf_first = 0, lf_count = 0, steps = 0;
-    bool exhausted = false;
-    auto pop = [&]() -> int {
-        if (sp == 0) return WW_DONE;
-        --sp;
-        return sp < STACK_SMEM ? smem_stack[sp * stride] : spill[sp - STACK_SMEM];
-    };
-    auto push = [&](int v) {
-        if (sp < STACK_SMEM)
-            smem_stack[sp * stride] = v;
-        else if (sp < RUMI_STACK4)
-            spill[sp - STACK_SMEM] = v;
-        if (sp < RUMI_STACK4) ++sp;  // three per level of a depth-limited tree: always holds
-    };
-    auto take_leaf = [&](int ref) {
-        const int k = -ref - 1, node = k >> 2, slot = k & 3;
-        if ((unsigned)node >= (unsigned)sp_scene->n_nodes4) {
-            lf_count = 0;
-            return;
-        }
-        const int4 ch = __ldg(reinterpret_cast<const int4 *>(nodes + 8 * node + 6));
-        const int4 cn = __ldg(reinterpret_cast<const int4 *>(nodes + 8 * node + 7));
-        lf_first = sel4(ch, slot);
-        lf_count = sel4(cn, slot);
-    };
-    for (;;) {
-        if (ray >= 0 && cur == WW_DONE && lf_count == 0) {
-            finish(ray, h);
-            ray = -1;
-        }
-        const unsigned idle = __ballot_sync(0xffffffffu, ray < 0);
-        if (!exhausted && idle && (__popc(idle) >= refill_min || idle == 0xffffffffu)) {
-            int base = 0;
-            const int leader = __ffs(idle) - 1;
-            if (lane == leader) base = atomicAdd(counter, __popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + __popc(idle) >= n) exhausted = true;
-            if (ray < 0) {
-                const int r = base + __popc(idle & lt);
-                if (r < n) {
-                    ray = r;
-                    fetch(r, o, d, tmax, in_obj);
-                    sp_scene = scene_of(r);
-                    nodes = reinterpret_cast<const float4 *>(sp_scene->nodes4);
-                    h.t = 0.0f;
-                    h.id = -1;
-                    h.u = h.v = 0.0f;
-                    h.back = 0;
-                    sp = 0;
-                    steps = 0;
-                    lf_count = 0;
-                    cur = WW_DONE;
-                    if (!(d.x == 0.0f && d.y == 0.0f && d.z == 0.0f) && sp_scene->n_nodes4 > 0) {  // bvh.cpp:161-162
-                        inv = safe_inv(d);
-                        oinv = mk3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-                        cur = 0;
-                    }
-                }
-            }
-        }
-        if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        while (cur >= 0) {
-            if ((unsigned)cur >= (unsigned)sp_scene->n_nodes4 || ++steps > sp_scene->n_nodes4) {  // malformed tree guard
-                cur = WW_DONE;
-                lf_count = 0;
-                break;
-            }
-            const float4 *np = nodes + 8 * cur;
-            const float4 lx = __ldg(np + 0), hx = __ldg(np + 1), ly = __ldg(np + 2), hy = __ldg(np + 3);
-            const float4 lz = __ldg(np + 4), hz = __ldg(np + 5);
-            const int4 ch = __ldg(reinterpret_cast<const int4 *>(np + 6));
-            const int4 cn = __ldg(reinterpret_cast<const int4 *>(np + 7));
-            if (STATS) st.nodes += 8;  // counted in 16-byte units
-            const float lim = cull_limit(h.t, tmax);
-            float k0, k1, k2, k3;
-            if (!(cn.x >= 0 && slab_s(lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, inv, oinv, lim, k0))) k0 = FLT_MAX;
-            if (!(cn.y >= 0 && slab_s(lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, inv, oinv, lim, k1))) k1 = FLT_MAX;
-            if (!(cn.z >= 0 && slab_s(lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, inv, oinv, lim, k2))) k2 = FLT_MAX;
-            if (!(cn.w >= 0 && slab_s(lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, inv, oinv, lim, k3))) k3 = FLT_MAX;
-            int s0 = 0, s1 = 1, s2 = 2, s3 = 3;
-            if (!ANYHIT) {
-                RUMI_CSWAP(k0, s0, k1, s1);
-                RUMI_CSWAP(k2, s2, k3, s3);
-                RUMI_CSWAP(k0, s0, k2, s2);
-                RUMI_CSWAP(k1, s1, k3, s3);
-                RUMI_CSWAP(k1, s1, k2, s2);
-            }
-            // entries of the hit children in order: node index or leaf reference
-            auto entry = [&](int slot) {
-                return sel4(cn, slot) > 0 ? -(1 + 4 * cur + slot) : sel4(ch, slot);
+            const float4 *np = wide + 6 * (size_t)cur;
+            float4 N0, N1, N2, N3, N4, N5;
+            ldg32(np, N0, N1);
+            ldg32(np + 2, N2, N3);
+            ldg32(np + 4, N4, N5);
+            if (STATS) st.nodes += 6;
+            const f2 ixy = pk(inv.x, inv.y), nxy = pk(noi.x, noi.y), axy = pk(fabsf(inv.x), fabsf(inv.y)),
+                     mxy = pk(-fabsf(inv.x), -fabsf(inv.y));
+            const float az = fabsf(inv.z);
+            // entry distance of a child, FLT_MAX when the ray misses it
+            auto child = [&](float cx, float cy, float cz, float hxy, float hz, bool &hit) -> float {
+                const f2 c = fma2(pk(cx, cy), ixy, nxy);
+                const f2 e = pk(__uint_as_float(__float_as_uint(hxy) << 16), hxy);
+                const float zc = fmaf(cz, inv.z, noi.z);
+                float nx, ny, fx, fy;
+                unpk(fma2(e, mxy, c), nx, ny);
+                unpk(fma2(e, axy, c), fx, fy);
+                const float tn = max3(nx, ny, fmaf(hz, -az, zc)), tf = min3(fx, fy, fmaf(hz, az, zc));
+                hit = tn <= tf && tf >= 0.0f && tn <= lim;
+                return hit ? tn : FLT_MAX;
             };
-            const int e0 = entry(s0), e1 = entry(s1), e2 = entry(s2), e3 = entry(s3);
-            const int nh = (k0 != FLT_MAX) + (k1 != FLT_MAX) + (k2 != FLT_MAX) + (k3 != FLT_MAX);
-            if (!ANYHIT) {
-                // sorted: the hit children are the first nh
-                if (nh > 3) push(e3);
-                if (nh > 2) push(e2);
-                if (nh > 1) push(e1);
-                cur = nh > 0 ? e0 : pop();
-            } else {
-                int next = WW_DONE;
-                if (k3 != FLT_MAX) next = e3;
-                if (k2 != FLT_MAX) { if (next != WW_DONE) push(next); next = e2; }
-                if (k1 != FLT_MAX) { if (next != WW_DONE) push(next); next = e1; }
-                if (k0 != FLT_MAX) { if (next != WW_DONE) push(next); next = e0; }
-                cur = next != WW_DONE ? next : pop();
+            bool h0, h1, h2, h3;
+            const float t0 = child(N0.x, N0.y, N2.x, N3.x, N4.x, h0), t1 = child(N0.z, N0.w, N2.y, N3.y, N4.y, h1),
+                        t2 = child(N1.x, N1.y, N2.z, N3.z, N4.z, h2), t3 = child(N1.z, N1.w, N2.w, N3.w, N4.w, h3);
+            const int r0 = __float_as_int(N5.x), r1 = __float_as_int(N5.y), r2 = __float_as_int(N5.z),
+                      r3 = __float_as_int(N5.w);
+            const float best = fminf(min3(t0, t1, t2), t3);
+            const bool s0 = t0 == best, s1 = !s0 && t1 == best, s2 = !s0 && !s1 && t2 == best,
+                       s3 = !s0 && !s1 && !s2;
+            cur = s0 ? r0 : s1 ? r1 : s2 ? r2 : r3;
+            if (!s0 && h0) push(r0);
+            if (!s1 && h1) push(r1);
+            if (!s2 && h2) push(r2);
+            if (!s3 && h3) push(r3);
+            const bool none = !(h0 || h1 || h2 || h3);
+            if (none || (cur < 0 && leaf == 0)) {
+                if (!none) leaf = cur;  // postpone the leaf, keep walking
+                pop();
             }
-            if (cur < 0 && cur != WW_DONE && lf_count == 0) {  // postpone the leaf, keep walking
-                take_leaf(cur);
-                cur = pop();
+            if (top > full) {  // room for the three entries the next node can add
+                if (n_deep + HALF > WW_DEEP) {  // cannot happen: three per level, at most 63 levels
+                    cur = WW_DONE;
+                    top = bottom;
+                } else {
+                    for (int k = 0; k < HALF; ++k) deep[n_deep + k] = smem_stack[bottom + k * WW_THREADS];
+                    n_deep += HALF;
+                    for (int k = bottom + HALF * WW_THREADS; k < top; k += WW_THREADS)
+                        smem_stack[k - HALF * WW_THREADS] = smem_stack[k];
+                    top -= HALF * WW_THREADS;
+                }
             }
-            if (!__any_sync(__activemask(), lf_count == 0 && cur >= 0)) break;
+            if (!__any_sync(__activemask(), leaf == 0 && cur >= 0)) break;
         }
-        while (lf_count > 0) {
-            if (leaf_isect<ANYHIT, STATS>(*sp_scene, lf_first, lf_count, o, d, tmax, in_obj, h, st)) {
-                cur = WW_DONE;
-                lf_count = 0;
-                break;
-            }
-            lf_count = 0;
-            if (cur < 0 && cur != WW_DONE) {
-                take_leaf(cur);
-                cur = pop();
+        // the postponed leaf, then the leaf the walk stopped at
+        const float2 ra = my_ray[0], rb = my_ray[WW_THREADS], rc = my_ray[2 * WW_THREADS];
+        const RayPairs rp = {make_float4(ra.x, ra.x, ra.y, ra.y), make_float4(rb.x, rb.x, rb.y, rb.y),
+                             make_float4(rc.x, rc.x, rc.y, rc.y)};
+        int i = leaf < 0 ? ~leaf : -1;
+        bool second = false;
+        while (__any_sync(0xffffffffu, i >= 0)) {
+            if (i >= 0) {
+                bool last = false;
+                const bool any = rec_isect<ANYHIT, STATS>(recs, i, rp, tmax, in_obj, h, last, st);
+                ++i;
+                if (last) {
+                    i = -1;
+                    if (!second && cur < 0 && cur != WW_DONE) {
+                        i = ~cur;
+                        second = true;
+                    }
+                }
+                if (ANYHIT && any) {
+                    i = -1;
+                    second = false;
+                    cur = WW_DONE;
+                }
             }
         }
+        leaf = 0;
+        if (!ANYHIT && h.t > 0.0f) lim = cull_limit(h.t, tmax);
+        if (second) pop();
     }
 }
 
@@ -1228,20 +1142,15 @@ RUMI_D HitRec trace_ray_w8(const DevScene &s, float3 o, float3 d, float tmax, bo
     return h;
 }
 
-// The default walk: the compressed eight-wide tree (RUMI_WALK8), else the binary or the
-// four-wide tree by RUMI_BVH_WIDE.
+// The default walk with a scene per ray.
 template <bool ANYHIT, int STACK_SMEM, bool STATS, typename SceneOf, typename Fetch, typename Finish>
-RUMI_D void traverse_queue_walk(SceneOf scene_of, int n, int *counter, int refill_min, int *smem_stack, int stride,
-                                Fetch fetch, Finish finish, TraceStats &st) {
+RUMI_D void traverse_queue_walk(SceneOf scene_of, int n, int *counter, int refill_min, int *smem_stack, Fetch fetch,
+                                Finish finish, TraceStats &st) {
 #if RUMI_WALK8
-    traverse_queue_ww8<ANYHIT, STACK_SMEM, STATS>(scene_of, n, counter, refill_min, smem_stack, stride, fetch, finish,
-                                                  st);
-#elif RUMI_BVH_WIDE
-    traverse_queue_ww4<ANYHIT, STACK_SMEM, STATS>(scene_of, n, counter, refill_min, smem_stack, stride, fetch, finish,
-                                                  st);
+    traverse_queue_ww8<ANYHIT, STACK_SMEM, STATS>(scene_of, n, counter, refill_min, smem_stack + threadIdx.x,
+                                                  WW_THREADS, fetch, finish, st);
 #else
-    traverse_queue_ww<ANYHIT, STACK_SMEM, STATS>(scene_of, n, counter, refill_min, smem_stack, stride, fetch, finish,
-                                                 st);
+    traverse_queue_ww<ANYHIT, STACK_SMEM, STATS, true>(scene_of, n, counter, refill_min, smem_stack, fetch, finish, st);
 #endif
 }
 
@@ -1250,12 +1159,14 @@ RUMI_D void traverse_queue_walk(SceneOf scene_of, int n, int *counter, int refil
 //   MODE 1: per-lane refill; every iteration advances each ray by one node pair.
 //   MODE 2: per-lane refill; interior node pairs until every busy lane holds postponed
 //           leaves, then the warp intersects those leaves together.
-//   MODE 3: speculative while-while with per-lane refill (traverse_queue_ww).
-//   MODE 4: the same walk over the compressed eight-wide tree (traverse_queue_ww8).
-// fetch(i, o, d, tmax, in_obj) loads ray i; finish(i, hit) consumes its result.
+//   MODE 3: speculative while-while over the four-wide tree (traverse_queue_ww).
+//   MODE 4: the same scheme over the compressed eight-wide tree (traverse_queue_ww8).
+// smem_block: the block's STACK_SMEM * WW_THREADS ints.  fetch(i, o, d, tmax, in_obj) loads ray i; finish(i, hit) consumes its result.
 template <int MODE, bool ANYHIT, int STACK_SMEM, bool STATS, typename Fetch, typename Finish>
-RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_min, int *smem_stack, int stride,
-                           Fetch fetch, Finish finish, TraceStats &st) {
+RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_min, int *smem_block, Fetch fetch,
+                           Finish finish, TraceStats &st) {
+    int *const smem_stack = smem_block + threadIdx.x;
+    constexpr int stride = WW_THREADS;
 #ifdef RUMI_HOST_BUILD
     // Host build of the kernels (CPU tests under sanitizers): one emulated thread takes
     // the queue's rays one after another through the per-ray walk; the warp-cooperative
@@ -1274,13 +1185,8 @@ RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_mi
     const int lane = threadIdx.x & 31;
     int spill[RUMI_MAX_BVH_DEPTH - STACK_SMEM > 0 ? RUMI_MAX_BVH_DEPTH - STACK_SMEM : 1];
     if (MODE == 3) {
-#if RUMI_BVH_WIDE
-        traverse_queue_ww4<ANYHIT, STACK_SMEM, STATS>([&](int) { return &s; }, n, counter, refill_min, smem_stack,
-                                                      stride, fetch, finish, st);
-#else
-        traverse_queue_ww<ANYHIT, STACK_SMEM, STATS>([&](int) { return &s; }, n, counter, refill_min, smem_stack,
-                                                     stride, fetch, finish, st);
-#endif
+        traverse_queue_ww<ANYHIT, STACK_SMEM, STATS, false>([&](int) { return &s; }, n, counter, refill_min, smem_block,
+                                                            fetch, finish, st);
         return;
     }
     if (MODE == 4) {

@@ -1,0 +1,103 @@
+// The four-wide tree of the default walk: node and leaf-record formats and their packing
+// (host and device, so that a host test builds the same bytes).
+#pragma once
+#include "common.cuh"
+#include <cmath>
+
+// 96-byte four-wide node (three 32-byte loads): four child boxes as centre and half extent.
+// A word of hxy holds two half extents: as a float it is at least that of y (the lower bits only
+// add to it), shifted up by 16 it is that of x, rounded up to 16 bits.  x and y of a centre are
+// adjacent, so that one packed operation (fma.rn.f32x2) serves both axes with the ray's
+// constants as they lie in registers, and with |1/d| per ray the slab ends are t_c -+ h |1/d|:
+// no minimum or maximum picks near from far, which matters because those run at half the rate of
+// multiply-adds.  The walk is bound by the L1's rate for divergent loads (one 128-byte line per
+// cycle and SM: 80% busy with a 128-byte node in four loads, 66% with this one), then by the
+// half-rate pipe (59%).  Measured per 1024x1024x64 frame of the 1M-triangle workload, closest-hit
+// / any-hit: binary tree, scalar slabs 85.8 / 46.5 ms; binary, this slab form 78.5 / 42.1;
+// four-wide with 32-bit half extents (128 bytes) 71.6 / 38.7; this node 65.7 / 35.2; a 64-byte
+// node with 8-bit planes 73.9 / 40.1 (the byte decoding costs more half-rate operations than the
+// saved load is worth).
+// ref[k] >= 0: node index of child k, larger than the node's own; ref[k] < 0: its leaf, whose
+// records start at recs[~ref[k]].  An empty slot has negative half extents, which no ray with
+// finite origin enters, and refers to record 0, which nothing hits.  wide[0] is the root.
+struct __align__(32) WideNode {
+    float2 cxy[4];
+    float cz[4];
+    unsigned hxy[4];
+    float hz[4];
+    int ref[4];
+};
+static_assert(sizeof(WideNode) == 96, "WideNode is three 32-byte loads");
+
+// 96-byte leaf record: two triangles, every component of the pair adjacent (-v0, e1, e2 per axis)
+// for the packed operations, or one rect or sphere as its three leaf_prims float4.  id[0] carries
+// the flags; an odd triangle fills both places.
+struct __align__(32) LeafRec {
+    float nv[6], e1[6], e2[6];
+    unsigned id[2];
+    unsigned unused[4];
+};
+static_assert(sizeof(LeafRec) == 96, "LeafRec is three 32-byte loads");
+#define REC_LAST 0x80000000u    // the leaf's last record
+#define REC_SINGLE 0x40000000u  // a rect or sphere
+#define REC_ID 0x3fffffffu
+
+RUMI_HD unsigned wide_bits(float f) {
+    union {
+        float f;
+        unsigned u;
+    } v;
+    v.f = f;
+    return v.u;
+}
+
+// Absolute padding of every child box, for a scene whose largest coordinate is amax: 2^-21 of it
+// exceeds the rounding of (c - o) / d and of o / d for origins within a few scene extents (the
+// binary node's own padding is relative to each face).
+RUMI_HD float wide_pad(float amax) { return amax * 4.76837158203125e-7f; }
+
+// Half extent of [lo, hi] about c, padded, rounded up.
+RUMI_HD float wide_half(float lo, float hi, float c, float pad) {
+    const double up = (double)hi - c, dn = (double)c - lo;
+    const double h = (up > dn ? up : dn) + pad;
+    const float f = (float)h;
+    return (double)f < h ? nextafterf(f, INFINITY) : f;
+}
+
+RUMI_HD void wide_set_half(WideNode &o, int k, float hx, float hy, float hz) {
+    const unsigned x = (wide_bits(hx) + 0xffffu) >> 16, y = wide_bits(hy);
+    // the smallest upper half with which the whole word is no smaller than hy
+    o.hxy[k] = x | ((y & 0xffffu) > x ? (y & 0xffff0000u) + 0x10000u : y & 0xffff0000u);
+    o.hz[k] = hz;
+}
+
+RUMI_HD void wide_empty(WideNode &o, int k) {
+    o.cxy[k] = make_float2(0.0f, 0.0f);
+    o.cz[k] = 0.0f;
+    wide_set_half(o, k, -1e30f, -1e30f, -1e30f);
+    o.ref[k] = ~0;
+}
+
+RUMI_HD void wide_child(WideNode &o, int k, const BvhNode &c, float pad, int ref) {
+    o.cxy[k] = make_float2(0.5f * c.lo_x + 0.5f * c.hi_x, 0.5f * c.lo_y + 0.5f * c.hi_y);
+    o.cz[k] = 0.5f * c.lo_z + 0.5f * c.hi_z;
+    wide_set_half(o, k, wide_half(c.lo_x, c.hi_x, o.cxy[k].x, pad), wide_half(c.lo_y, c.hi_y, o.cxy[k].y, pad),
+                  wide_half(c.lo_z, c.hi_z, o.cz[k], pad));
+    o.ref[k] = ref;
+}
+
+// Triangle in place `slot` of a record, from its leaf_prims float4.
+RUMI_HD void rec_triangle(LeafRec &r, int slot, float4 A, float4 B, float4 C) {
+    r.nv[slot] = -A.x; r.nv[2 + slot] = -A.y; r.nv[4 + slot] = -A.z;
+    r.e1[slot] = B.x; r.e1[2 + slot] = B.y; r.e1[4 + slot] = B.z;
+    r.e2[slot] = C.x; r.e2[2 + slot] = C.y; r.e2[4 + slot] = C.z;
+    r.id[slot] = wide_bits(A.w);
+}
+
+RUMI_HD void rec_single(LeafRec &r, float4 A, float4 B, float4 C) {
+    float4 *f = reinterpret_cast<float4 *>(&r);
+    f[0] = A;
+    f[1] = B;
+    f[2] = C;
+    r.id[0] = wide_bits(A.w) | REC_SINGLE;
+}
