@@ -10,6 +10,7 @@
 // counts once, then allocates the two arrays to size and writes the leaf records, a warp per
 // leaf.
 #include "renderer.h"
+#include "traverse.cuh"
 
 namespace rumi {
 
@@ -193,7 +194,13 @@ __global__ void records_kernel(const float4 *__restrict__ lp, const LeafJob *__r
             } else {
                 const int r = pairs + one0 + __popc(mo & lt);
                 LeafRec &rec = recs[jb.at + r];
-                rec_single(rec, A, B, C);
+                if ((__float_as_int(B.w) & 0xff) == PRIM_RECT) {
+                    const RectGeom g = rect_geom(f4xyz(B), f4xyz(C));
+                    rec_rect(rec, A, B, C, g.n, g.length, g.width, __fmul_rn(g.inv_area, g.width),
+                             __fmul_rn(g.inv_area, g.length));
+                } else {
+                    rec_single(rec, A, B, C);
+                }
                 if (r + 1 == total) rec.id[0] |= REC_LAST;
             }
         }

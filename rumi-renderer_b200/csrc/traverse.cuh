@@ -72,10 +72,9 @@ RUMI_D RectGeom rect_geom(float3 l, float3 w) {
     return g;
 }
 
-RUMI_D bool isect_rect(float3 o, float3 d, float tmax, float tbest, float4 A, float4 B, float4 C, bool emissive,
-                       float &t_out) {
-    const float3 p = f4xyz(A), l = f4xyz(B), w = f4xyz(C);
-    const RectGeom g = rect_geom(l, w);
+// g: the rect's geometry; by_width / by_length: inv_area * width / length.
+RUMI_D bool isect_rect_geom(float3 o, float3 d, float tmax, float tbest, float3 p, float3 l, float3 w, const RectGeom &g,
+                            float by_width, float by_length, bool emissive, float &t_out) {
     const float cost = rn_dot(d, g.n);
     if (cost == 0.0f) return false;
     const float t = __fdiv_rn(-rn_dot(rn_sub(o, p), g.n), cost);
@@ -86,12 +85,20 @@ RUMI_D bool isect_rect(float3 o, float3 d, float tmax, float tbest, float4 A, fl
     if (t > tbest && tbest > 0.0f) return false;
     const float3 ip = rn_madd(o, d, t);
     const float3 on = rn_sub(ip, p);
-    const float il = __fmul_rn(rn_dot(on, l), __fmul_rn(g.inv_area, g.width));
+    const float il = __fmul_rn(rn_dot(on, l), by_width);
     if (il < 0.0f || il > g.length) return false;
-    const float iw = __fmul_rn(rn_dot(on, w), __fmul_rn(g.inv_area, g.length));
+    const float iw = __fmul_rn(rn_dot(on, w), by_length);
     if (iw < 0.0f || iw > g.width) return false;
     t_out = t;
     return true;
+}
+
+RUMI_D bool isect_rect(float3 o, float3 d, float tmax, float tbest, float4 A, float4 B, float4 C, bool emissive,
+                       float &t_out) {
+    const float3 l = f4xyz(B), w = f4xyz(C);
+    const RectGeom g = rect_geom(l, w);
+    return isect_rect_geom(o, d, tmax, tbest, f4xyz(A), l, w, g, __fmul_rn(g.inv_area, g.width),
+                           __fmul_rn(g.inv_area, g.length), emissive, t_out);
 }
 
 RUMI_D bool isect_sphere(float3 o, float3 d, float tmax, float tbest, float4 A, float4 B, bool in_object, bool ibl,
@@ -594,8 +601,14 @@ RUMI_D bool rec_isect(const float4 *__restrict__ recs, int i, const RayPairs &rp
         if (STATS) st.prims++;
         const int tag = __float_as_int(B.w);
         float t;
+        RectGeom g;
+        g.n = f4xyz(D);
+        g.length = D.w;
+        g.width = E.x;
+        g.inv_area = 0.0f;  // only through the two factors
         const bool ok = (tag & 0xff) == PRIM_RECT
-                            ? isect_rect(o, d, tmax, h.t, A, B, C, (tag & PRIM_FLAG_EMISSIVE) != 0, t)
+                            ? isect_rect_geom(o, d, tmax, h.t, f4xyz(A), f4xyz(B), f4xyz(C), g, E.y, F.x,
+                                              (tag & PRIM_FLAG_EMISSIVE) != 0, t)
                             : isect_sphere(o, d, tmax, h.t, A, B, in_object && !ANYHIT, (tag & PRIM_FLAG_IBL) != 0, t);
         if (!ok || (t == h.t && id0 < h.id)) return false;
         h.t = t;
@@ -629,6 +642,30 @@ RUMI_D bool rec_isect(const float4 *__restrict__ recs, int i, const RayPairs &rp
     bool hit = accept_triangle(det0, u0, v0, t0, tmax, id0, h);
     hit |= accept_triangle(det1, u1, v1, t1, tmax, id1, h);
     return hit;
+}
+
+// A four-wide node's child boxes against a ray (inv = 1 / d, noi = -o / d): which it enters up to
+// `lim`, and where (FLT_MAX when it misses).
+RUMI_D void wide_slabs(float4 N0, float4 N1, float4 N2, float4 N3, float4 N4, float3 inv, float3 noi, float lim, bool &h0,
+                       bool &h1, bool &h2, bool &h3, float &t0, float &t1, float &t2, float &t3) {
+    const f2 ixy = pk(inv.x, inv.y), nxy = pk(noi.x, noi.y), axy = pk(fabsf(inv.x), fabsf(inv.y)),
+             mxy = pk(-fabsf(inv.x), -fabsf(inv.y));
+    const float az = fabsf(inv.z);
+    auto child = [&](float cx, float cy, float cz, float hxy, float hz, bool &hit) -> float {
+        const f2 c = fma2(pk(cx, cy), ixy, nxy);
+        const f2 e = pk(__uint_as_float(__float_as_uint(hxy) << 16), hxy);
+        const float zc = fmaf(cz, inv.z, noi.z);
+        float nx, ny, fx, fy;
+        unpk(fma2(e, mxy, c), nx, ny);
+        unpk(fma2(e, axy, c), fx, fy);
+        const float tn = max3(nx, ny, fmaf(hz, -az, zc)), tf = min3(fx, fy, fmaf(hz, az, zc));
+        hit = tn <= tf && tf >= 0.0f && tn <= lim;
+        return hit ? tn : FLT_MAX;
+    };
+    t0 = child(N0.x, N0.y, N2.x, N3.x, N4.x, h0);
+    t1 = child(N0.z, N0.w, N2.y, N3.y, N4.y, h1);
+    t2 = child(N1.x, N1.y, N2.z, N3.z, N4.z, h2);
+    t3 = child(N1.z, N1.w, N2.w, N3.w, N4.w, h3);
 }
 
 // Speculative while-while traversal with per-lane refill (Aila & Laine, "Understanding
@@ -753,34 +790,19 @@ RUMI_D void traverse_queue_ww(SceneOf scene_of, int n, int *counter, int refill_
             ldg32(np + 2, N2, N3);
             ldg32(np + 4, N4, N5);
             if (STATS) st.nodes += 6;
-            const f2 ixy = pk(inv.x, inv.y), nxy = pk(noi.x, noi.y), axy = pk(fabsf(inv.x), fabsf(inv.y)),
-                     mxy = pk(-fabsf(inv.x), -fabsf(inv.y));
-            const float az = fabsf(inv.z);
-            // entry distance of a child, FLT_MAX when the ray misses it
-            auto child = [&](float cx, float cy, float cz, float hxy, float hz, bool &hit) -> float {
-                const f2 c = fma2(pk(cx, cy), ixy, nxy);
-                const f2 e = pk(__uint_as_float(__float_as_uint(hxy) << 16), hxy);
-                const float zc = fmaf(cz, inv.z, noi.z);
-                float nx, ny, fx, fy;
-                unpk(fma2(e, mxy, c), nx, ny);
-                unpk(fma2(e, axy, c), fx, fy);
-                const float tn = max3(nx, ny, fmaf(hz, -az, zc)), tf = min3(fx, fy, fmaf(hz, az, zc));
-                hit = tn <= tf && tf >= 0.0f && tn <= lim;
-                return hit ? tn : FLT_MAX;
-            };
             bool h0, h1, h2, h3;
-            const float t0 = child(N0.x, N0.y, N2.x, N3.x, N4.x, h0), t1 = child(N0.z, N0.w, N2.y, N3.y, N4.y, h1),
-                        t2 = child(N1.x, N1.y, N2.z, N3.z, N4.z, h2), t3 = child(N1.z, N1.w, N2.w, N3.w, N4.w, h3);
+            float t0, t1, t2, t3;
+            wide_slabs(N0, N1, N2, N3, N4, inv, noi, lim, h0, h1, h2, h3, t0, t1, t2, t3);
             const int r0 = __float_as_int(N5.x), r1 = __float_as_int(N5.y), r2 = __float_as_int(N5.z),
                       r3 = __float_as_int(N5.w);
             const float best = fminf(min3(t0, t1, t2), t3);
-            const bool s0 = t0 == best, s1 = !s0 && t1 == best, s2 = !s0 && !s1 && t2 == best,
-                       s3 = !s0 && !s1 && !s2;
-            cur = s0 ? r0 : s1 ? r1 : s2 ? r2 : r3;
-            if (!s0 && h0) push(r0);
-            if (!s1 && h1) push(r1);
-            if (!s2 && h2) push(r2);
-            if (!s3 && h3) push(r3);
+            // (a node's references differ, so comparing them tells the chosen child from the others
+            // also where entry distances tie)
+            cur = t0 == best ? r0 : t1 == best ? r1 : t2 == best ? r2 : r3;
+            if (h0 && r0 != cur) push(r0);
+            if (h1 && r1 != cur) push(r1);
+            if (h2 && r2 != cur) push(r2);
+            if (h3 && r3 != cur) push(r3);
             const bool none = !(h0 || h1 || h2 || h3);
             if (none || (cur < 0 && leaf == 0)) {
                 if (!none) leaf = cur;  // postpone the leaf, keep walking

@@ -101,3 +101,16 @@ RUMI_HD void rec_single(LeafRec &r, float4 A, float4 B, float4 C) {
     f[2] = C;
     r.id[0] = wide_bits(A.w) | REC_SINGLE;
 }
+
+// A rect's record also holds what its test derives from the edges alone (the Rect constructor's
+// values, which cost more than the rest of the test): normal, lengths, and the factors
+// inv_area * width and inv_area * length.
+RUMI_HD void rec_rect(LeafRec &r, float4 A, float4 B, float4 C, float3 n, float length, float width, float by_width,
+                      float by_length) {
+    float4 *f = reinterpret_cast<float4 *>(&r);
+    f[3] = make_float4(n.x, n.y, n.z, length);
+    f[4].x = width;
+    f[4].y = by_width;
+    f[5].x = by_length;
+    rec_single(r, A, B, C);
+}

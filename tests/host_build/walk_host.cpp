@@ -63,7 +63,13 @@ struct Tree {
         if (held >= 0) add(held, held);
         for (int p : one) {
             LeafRec r = {};
-            rec_single(r, prims[3 * p], prims[3 * p + 1], prims[3 * p + 2]);
+            const float4 A = prims[3 * p], B = prims[3 * p + 1], C = prims[3 * p + 2];
+            if ((__float_as_int(B.w) & 0xff) == PRIM_RECT) {
+                const RectGeom g = rect_geom(f4xyz(B), f4xyz(C));
+                rec_rect(r, A, B, C, g.n, g.length, g.width, g.inv_area * g.width, g.inv_area * g.length);
+            } else {
+                rec_single(r, A, B, C);
+            }
             recs.push_back(r);
         }
         recs.back().id[0] |= REC_LAST;
