@@ -83,8 +83,9 @@ RUMI_D unsigned flags_of(float w) {
     const unsigned b = __float_as_uint(w);
     return ((b >> 31) ? PFL_IN : 0u) | (((b >> 30) & 1u) ? PFL_LE : 0u);
 }
-// counters
-enum { C_RAY0 = 0, C_RAY1 = 1, C_SHADOW = 2, C_FETCH_EXT = 3, C_FETCH_SH = 4, C_NUM = 8 };
+// counters.  The shadow queue has two sets of them (PtLaunch::sh_set, by the bounce's parity), so
+// that the kernels can clear each other's without a launch for it (PtLaunch::chained).
+enum { C_RAY0 = 0, C_RAY1 = 1, C_SHADOW = 2, C_FETCH_EXT = 3, C_FETCH_SH = 4, C_SHADOW1 = 5, C_FETCH_SH1 = 6, C_NUM = 8 };
 // 64-bit device statistics
 enum { S_RAYS_EXT = 0, S_RAYS_SH = 1, S_NAN = 2, S_NODES = 3, S_PRIMS = 4, S_NUM = 8 };
 
@@ -102,6 +103,12 @@ struct PtLaunch {
     unsigned long long *stats;
     float *film;
     int refill_min;
+    // chained: the bounce's kernels keep the counters and statistics themselves.  Closest hit of
+    // bounce b clears the queue count and the shadow set that shading of b fills (their last
+    // readers, shading of b - 1 and the any-hit launch of b - 2, are done), shading clears the
+    // closest-hit work counter and counts its rays, any hit counts its own.  0: pt_reset and
+    // pt_finish do all that.
+    int chained, sh_set;
     // multi-scene batches (scenes == nullptr: the single scene s)
     const DevScene *scenes;
     const long long *scene_path0;  // n_scenes + 1 prefix: first global path of each scene
@@ -167,6 +174,27 @@ RUMI_D int find_scene(const long long *prefix, int n, long long g) {
             hi = mid;
     }
     return lo;
+}
+
+// The chained kernels' bookkeeping, by one thread of the grid.
+RUMI_D bool first_thread() { return blockIdx.x == 0 && threadIdx.x == 0; }
+RUMI_D int *shadow_count(const PtLaunch &P) { return P.cnt + (P.sh_set ? C_SHADOW1 : C_SHADOW); }
+RUMI_D int *shadow_fetch(const PtLaunch &P) { return P.cnt + (P.sh_set ? C_FETCH_SH1 : C_FETCH_SH); }
+RUMI_D void chain_extend(const PtLaunch &P, int bounce) {
+    if (P.chained && first_thread()) {
+        P.cnt[(bounce & 1) ^ 1] = 0;
+        *shadow_count(P) = 0;
+        *shadow_fetch(P) = 0;
+    }
+}
+RUMI_D void chain_shade(const PtLaunch &P, int bounce) {
+    if (P.chained && first_thread()) {
+        P.stats[S_RAYS_EXT] += (unsigned long long)P.cnt[bounce & 1];
+        P.cnt[C_FETCH_EXT] = 0;
+    }
+}
+RUMI_D void chain_shadow(const PtLaunch &P) {
+    if (P.chained && first_thread()) P.stats[S_RAYS_SH] += (unsigned long long)*shadow_count(P);
 }
 
 RUMI_D int isqrt_floor(int n) {
@@ -236,22 +264,6 @@ __global__ void pt_reset(PtLaunch P, int bounce) {
 
 __global__ void pt_finish(PtLaunch P) { P.stats[S_RAYS_SH] += (unsigned long long)P.cnt[C_SHADOW]; }
 
-// pt_reset in two halves for the overlapped schedule: before a closest-hit launch (its
-// queue into the statistics, its work counter cleared), and before shading, once the
-// previous bounce's shadow rays are traced (their count into the statistics, the queues
-// shading pushes into cleared).
-__global__ void pt_reset_extend(PtLaunch P, int bounce) {
-    P.stats[S_RAYS_EXT] += (unsigned long long)P.cnt[bounce & 1];
-    P.cnt[C_FETCH_EXT] = 0;
-}
-__global__ void pt_reset_shade(PtLaunch P, int bounce) {
-    // (at bounce 0 the count is the previous wave's last bounce, which pt_finish added)
-    if (bounce > 0) P.stats[S_RAYS_SH] += (unsigned long long)P.cnt[C_SHADOW];
-    P.cnt[C_SHADOW] = 0;
-    P.cnt[C_FETCH_SH] = 0;
-    P.cnt[(bounce & 1) ^ 1] = 0;
-}
-
 // Persistent traversal kernels: every block takes rays from the bounce's queue until it
 // is empty (traverse_queue in traverse.cuh; MODE selects the scheme, see there).
 // SMEM: traversal stack entries per thread kept in shared memory (deeper entries spill to
@@ -260,6 +272,7 @@ template <int MODE, bool STATS, int SMEM = STACK_SMEM>
 __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, true)) pt_extend(PtLaunch P, int bounce) {
     __shared__ int stack[SMEM * TRACE_THREADS];
     const int cur = bounce & 1;
+    chain_extend(P, bounce);
     TraceStats st{0, 0};
     auto fetch = [&](int i, float3 &o, float3 &d, float &tmax, bool &in_obj) {
         const float4 o4 = P.ray_o[cur][i];
@@ -284,6 +297,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, true)) p
 template <int MODE, bool ADJ = false, int SMEM = STACK_SMEM>
 __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, false)) pt_shadow(PtLaunch P) {
     __shared__ int stack[SMEM * TRACE_THREADS];
+    chain_shadow(P);
     TraceStats st{0, 0};
     float acc_sigma = 0.0f, acc_g = 0.0f;  // adjoint: score-weighted contributions
     auto fetch = [&](int i, float3 &o, float3 &d, float &tmax, bool &in_obj) {
@@ -312,7 +326,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, false)) 
             }
         }
     };
-    traverse_queue<MODE, true, SMEM, false>(P.s, P.cnt[C_SHADOW], &P.cnt[C_FETCH_SH], P.refill_min,
+    traverse_queue<MODE, true, SMEM, false>(P.s, *shadow_count(P), shadow_fetch(P), P.refill_min,
                                             stack, fetch, finish, st);
     if (ADJ) {
         __syncwarp();
@@ -333,8 +347,12 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(DEFAULT_WALK_M
     pt_trace_multi(PtLaunch P, int bounce) {
     __shared__ int stack[WALK_SMEM * TRACE_THREADS];
     const int cur = bounce & 1;
-    const int n = ANYHIT ? P.cnt[C_SHADOW] : P.cnt[cur];
-    int *counter = ANYHIT ? &P.cnt[C_FETCH_SH] : &P.cnt[C_FETCH_EXT];
+    const int n = ANYHIT ? *shadow_count(P) : P.cnt[cur];
+    int *counter = ANYHIT ? shadow_fetch(P) : &P.cnt[C_FETCH_EXT];
+    if (ANYHIT)
+        chain_shadow(P);
+    else
+        chain_extend(P, bounce);
     TraceStats st{0, 0};
     auto scene_of = [&](int i) -> const DevScene * {
         if (i < 0) return &P.scenes[0];
@@ -423,6 +441,7 @@ template <bool ADJ, bool LEAN = false>
 __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LEAN_MIN_BLOCKS : RUMI_SHADE_MIN_BLOCKS))
     pt_shade(PtLaunch P, int bounce) {
     const int cur = bounce & 1, nxt = cur ^ 1;
+    chain_shade(P, bounce);
     const int n = P.cnt[cur];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < n;
@@ -735,7 +754,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
     __syncthreads();
     const int kn = want_next ? s_bins[dkey] + drank : -1;
 #endif
-    const int ks = warp_push(&P.cnt[C_SHADOW], want_sh);
+    const int ks = warp_push(shadow_count(P), want_sh);
     if (want_next) {
         P.ray_o[nxt][kn] = make_float4(nx_o.x, nx_o.y, nx_o.z, pack_slot(slot, nx_flags));
         P.ray_d[nxt][kn] = make_float4(nx_d.x, nx_d.y, nx_d.z, FLT_MAX);
@@ -786,6 +805,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
 // carries the index of the material a refracted ray entered.
 __global__ void __launch_bounds__(SHADE_THREADS) pt_shade_whitted(PtLaunch P, int bounce) {
     const int cur = bounce & 1, nxt = cur ^ 1;
+    chain_shade(P, bounce);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = P.cnt[cur];
     const bool active = i < n;
@@ -891,7 +911,7 @@ __global__ void __launch_bounds__(SHADE_THREADS) pt_shade_whitted(PtLaunch P, in
         }
     }
     const int kn = warp_push(&P.cnt[nxt], want_next);
-    const int ks = warp_push(&P.cnt[C_SHADOW], want_sh);
+    const int ks = warp_push(shadow_count(P), want_sh);
     if (want_next) {
         P.ray_o[nxt][kn] = make_float4(nx_o.x, nx_o.y, nx_o.z, pack_slot(slot, nx_flags));
         P.ray_d[nxt][kn] = make_float4(nx_d.x, nx_d.y, nx_d.z, FLT_MAX);
@@ -1088,6 +1108,11 @@ size_t pt_workspace_bytes(long long paths) {
 }
 
 #ifndef RUMI_HOST_BUILD
+// Counters and statistics (adjacent in the wave state) to zero.
+static void clear_counters(const PtLaunch &L, cudaStream_t stream) {
+    cudaMemsetAsync(L.cnt, 0, align256(C_NUM * sizeof(int)) + S_NUM * sizeof(unsigned long long), stream);
+}
+
 // The scene's second stream and its fork / join events, made on first use.
 static rumi_status ensure_aux(rumi_scene *sc) {
     if (sc->aux_stream) return RUMI_OK;
@@ -1141,8 +1166,7 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
     L.grid_d = d;
     L.square = d * d == spp;
     L.film = film_dev;
-    cudaMemsetAsync(L.cnt, 0, C_NUM * sizeof(int), stream);
-    cudaMemsetAsync(L.stats, 0, S_NUM * sizeof(unsigned long long), stream);
+    clear_counters(L, stream);
 
     // traversal scheme and persistent grid (autotuner knobs; 0 = defaults)
     const int mode = trace_scheme(p->trace_mode);
@@ -1179,8 +1203,9 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
             // for both, as it refills the shadow queue and adds to the radiance
             // (with timing, a closest-hit launch's events include the time it shares the
             // GPU with the previous bounce's any-hit launch)
+            L.chained = 1;
             for (int b = 0; b < bounces; ++b) {
-                pt_reset_extend<<<1, 1, 0, stream>>>(L, b);
+                L.sh_set = b & 1;
                 int e0 = 0;
                 if (timing) { e0 = (int)evs.size(); mark(); }
                 if (count_stats)
@@ -1189,7 +1214,6 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
                     launch_extend<false>(mode, smem, grid, stream, L, b);
                 if (timing) { mark(); ext_ev.push_back({e0, e0 + 1}); }
                 if (b > 0) cudaStreamWaitEvent(stream, sc->ev_join, 0);
-                pt_reset_shade<<<1, 1, 0, stream>>>(L, b);
                 if (timing) { e0 = (int)evs.size(); mark(); }
                 if (whitted)
                     pt_shade_whitted<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(L, b);
@@ -1207,7 +1231,6 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
                 if (timing) { mark_on(ss); sh_ev.push_back({e0, e0 + 1}); }
                 if (aside) cudaEventRecord(sc->ev_join, sc->aux_stream);
             }
-            pt_finish<<<1, 1, 0, stream>>>(L);
             pt_resolve<<<cdiv(L.n_pix * 32LL, 256), 256, 0, stream>>>(L);
             if (keep_L)
                 cudaMemcpyAsync(keep_L + L.path0, L.L, sizeof(float4) * (size_t)L.n_paths, cudaMemcpyDeviceToDevice,
@@ -1328,6 +1351,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
     A.grid_d = d;
     A.square = d * d == spp;
     A.refill_min = 8;
+    A.chained = 1;
     PtLaunch B = A;
     float4 *Lt = (float4 *)w; w += align256(Wp * sizeof(float4));
     B.Lt = Lt;
@@ -1336,8 +1360,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
     B.dfilm = dfilm_dev;
     B.g_albedo = g_albedo;
     B.g_medium = g_medium;
-    cudaMemsetAsync(A.cnt, 0, C_NUM * sizeof(int), stream);
-    cudaMemsetAsync(A.stats, 0, S_NUM * sizeof(unsigned long long), stream);
+    clear_counters(A, stream);
     cudaMemsetAsync(g_medium, 0, GM_NUM * sizeof(float), stream);
     if (g_albedo) cudaMemsetAsync(g_albedo, 0, sizeof(float) * 3 * (size_t)sc->dev.n_tris, stream);
 
@@ -1370,10 +1393,9 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
         auto pass = [&](PtLaunch &X, bool adj) {
             pt_generate<<<cdiv(X.n_paths, 256), 256, 0, stream>>>(X);
             for (int b = 0; b < p->max_depth; ++b) {
-                pt_reset_extend<<<1, 1, 0, stream>>>(X, b);
+                X.sh_set = b & 1;
                 launch_extend<false>(mode, smem, grid, stream, X, b);
                 if (b > 0 && overlap) cudaStreamWaitEvent(stream, sc->ev_join, 0);
-                pt_reset_shade<<<1, 1, 0, stream>>>(X, b);
                 if (adj)
                     pt_shade<true><<<cdiv(X.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(X, b);
                 else
@@ -1390,7 +1412,6 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
                     launch_shadow<false>(mode, smem, grid_sh, ss, X);
                 if (aside) cudaEventRecord(sc->ev_join, sc->aux_stream);
             }
-            pt_finish<<<1, 1, 0, stream>>>(X);
         };
         // pass 1: radiance of every path (or the radiance rumi_forward kept for this frame)
         if (reuse) {
@@ -1459,8 +1480,8 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
     L.n_scenes = F.n_scenes;
     L.spp = 1;
     L.refill_min = 8;
-    cudaMemsetAsync(L.cnt, 0, C_NUM * sizeof(int), stream);
-    cudaMemsetAsync(L.stats, 0, S_NUM * sizeof(unsigned long long), stream);
+    L.chained = 1;
+    clear_counters(L, stream);
     const int mb = trace_min_blocks(DEFAULT_WALK_MODE, true), mb_sh = trace_min_blocks(DEFAULT_WALK_MODE, false);
     for (const BatchWave &wv : F.waves) {
         L.pix0 = (int)wv.pix0;
@@ -1473,10 +1494,9 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
         // the two-stream schedule of pt_render_in (a graph capture takes the auxiliary
         // stream in through the fork event and every fork is joined before shading)
         for (int b = 0; b < F.max_depth; ++b) {
-            pt_reset_extend<<<1, 1, 0, stream>>>(L, b);
+            L.sh_set = b & 1;
             pt_trace_multi<false><<<grid, TRACE_THREADS, 0, stream>>>(L, b);
             if (b > 0 && aux) cudaStreamWaitEvent(stream, ev_join, 0);
-            pt_reset_shade<<<1, 1, 0, stream>>>(L, b);
             launch_shade(F.lean, stream, L, b);
             const bool aside = aux && b + 1 < F.max_depth;
             if (aside) {
@@ -1486,7 +1506,6 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
             pt_trace_multi<true><<<grid_sh, TRACE_THREADS, 0, aside ? aux : stream>>>(L, b);
             if (aside) cudaEventRecord(ev_join, aux);
         }
-        pt_finish<<<1, 1, 0, stream>>>(L);
         pt_resolve<<<cdiv(L.n_pix * 32LL, 256), 256, 0, stream>>>(L);
     }
     cudaError_t e = cudaGetLastError();
