@@ -474,7 +474,7 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         set_error("bvh_build: internal limit reached");
         return fail(RUMI_ERR_INTERNAL);
     }
-    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, &sc->wide, &sc->recs, s);
+    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, &sc->wide, &sc->n_wide, &sc->recs, &sc->n_recs, s);
     if (rc != 0) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);

@@ -23,8 +23,8 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
 
 // Four-wide tree of the default walk, collapsed from the binary one (bvh_wide.cu).  Returns 0, a
 // cudaError_t value, or -1 when an index left its range.
-int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, WideNode **wide_out,
-             LeafRec **recs_out, cudaStream_t stream);
+int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, WideNode **wide_out, int *n_wide,
+             LeafRec **recs_out, int *n_recs, cudaStream_t stream);
 
 // Compressed eight-wide tree collapsed from the binary one (bvh8.cu); prims8 receives the
 // leaf primitives in its order.  Returns the node count, 0 without primitives, -1 on error.

@@ -213,8 +213,8 @@ __global__ void records_kernel(const float4 *__restrict__ lp, const LeafJob *__r
 
 // Builds the four-wide tree of a finished binary tree; *wide_out and *recs_out are allocated to
 // size.  Returns 0, a cudaError_t value, or -1 when an index left its range.
-int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, WideNode **wide_out,
-             LeafRec **recs_out, cudaStream_t stream) {
+int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, WideNode **wide_out, int *n_wide,
+             LeafRec **recs_out, int *n_recs, cudaStream_t stream) {
     // one four-wide node at most per leaf, one job per leaf: a node with an interior child has four
     // children, so nodes are outnumbered by leaves
     const size_t cap = n_prims > 1 ? (size_t)n_prims : 1;
@@ -271,7 +271,9 @@ int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims,
         return e != cudaSuccess ? (int)e : -1;
     }
     *wide_out = w;
+    *n_wide = h[K_WIDE];
     *recs_out = r;
+    *n_recs = h[K_RECS];
     return 0;
 }
 

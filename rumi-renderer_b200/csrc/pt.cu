@@ -51,8 +51,13 @@ static constexpr int TRACE_THREADS = 128;
 #ifndef RUMI_WW_MIN_BLOCKS
 #define RUMI_WW_MIN_BLOCKS 9
 #endif
+// Testing a small scene's records in step (scheme 5): 64 registers without spills; 6 and 10 blocks
+// are 4% slower and equal on the Cornell frame.
+#ifndef RUMI_FEW_MIN_BLOCKS
+#define RUMI_FEW_MIN_BLOCKS 8
+#endif
 static constexpr int trace_min_blocks(int mode, bool extend) {
-    return mode == 3 ? RUMI_WW_MIN_BLOCKS : (extend ? RUMI_EXTEND_MIN_BLOCKS : RUMI_SHADOW_MIN_BLOCKS);
+    return mode == 5 ? RUMI_FEW_MIN_BLOCKS : mode == 3 ? RUMI_WW_MIN_BLOCKS : (extend ? RUMI_EXTEND_MIN_BLOCKS : RUMI_SHADOW_MIN_BLOCKS);
 }
 // 1: each bounce's any-hit launch runs on an auxiliary stream beside the next bounce's
 // closest-hit launch (pt_render_in); 0: one stream, launches in order.
@@ -60,6 +65,11 @@ static constexpr int trace_min_blocks(int mode, bool extend) {
 #define RUMI_PT_OVERLAP 1
 #endif
 static constexpr int STACK_SMEM = 32;
+// Leaf records (the empty one included) up to which a single-node scene's rays are traced in step
+// (scene_scheme).
+#ifndef RUMI_FEW_RECORDS
+#define RUMI_FEW_RECORDS 10
+#endif
 static constexpr int WALK_SMEM = 16;  // of the default walk (stack_entries)
 static_assert(TRACE_THREADS == WW_THREADS, "the walk's shared-memory columns are one per thread");
 static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? 4 : 3;
@@ -437,7 +447,7 @@ RUMI_D bool nee_setup(const LightSample &ls, float3 p, float3 &wi, float &dist, 
 #ifndef RUMI_SHADE_LEAN_MIN_BLOCKS
 #define RUMI_SHADE_LEAN_MIN_BLOCKS 4
 #endif
-template <bool ADJ, bool LEAN = false>
+template <bool ADJ, bool LEAN = false, bool GROUP = true>
 __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LEAN_MIN_BLOCKS : RUMI_SHADE_MIN_BLOCKS))
     pt_shade(PtLaunch P, int bounce) {
     const int cur = bounce & 1, nxt = cur ^ 1;
@@ -726,33 +736,38 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
     // host build (one emulated thread per block): the block's group is its one ray
     const int kn = want_next ? atomicAdd(&P.cnt[nxt], 1) : -1;
 #else
-    __shared__ int s_bins[32];
-    if (threadIdx.x < 32) s_bins[threadIdx.x] = 0;
-    __syncthreads();
-    int dkey = 0, drank = 0;
-    if (want_next) {
-        const float ax = fabsf(nx_d.x), ay = fabsf(nx_d.y), az = fabsf(nx_d.z);
-        const int dom = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
-        const int oct = (nx_d.x < 0.0f ? 1 : 0) | (nx_d.y < 0.0f ? 2 : 0) | (nx_d.z < 0.0f ? 4 : 0);
-        dkey = oct * 3 + dom;
-        drank = atomicAdd(&s_bins[dkey], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {  // exclusive scan of the bins, then the block's range of the queue
-        const int v = s_bins[threadIdx.x];
-        int incl = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)threadIdx.x >= o) incl += u;
+    int kn = -1;
+    if (GROUP) {
+        __shared__ int s_bins[32];
+        if (threadIdx.x < 32) s_bins[threadIdx.x] = 0;
+        __syncthreads();
+        int dkey = 0, drank = 0;
+        if (want_next) {
+            const float ax = fabsf(nx_d.x), ay = fabsf(nx_d.y), az = fabsf(nx_d.z);
+            const int dom = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
+            const int oct = (nx_d.x < 0.0f ? 1 : 0) | (nx_d.y < 0.0f ? 2 : 0) | (nx_d.z < 0.0f ? 4 : 0);
+            dkey = oct * 3 + dom;
+            drank = atomicAdd(&s_bins[dkey], 1);
         }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int base = 0;
-        if (threadIdx.x == 0 && total > 0) base = atomicAdd(&P.cnt[nxt], total);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        s_bins[threadIdx.x] = base + incl - v;
+        __syncthreads();
+        if (threadIdx.x < 32) {  // exclusive scan of the bins, then the block's range of the queue
+            const int v = s_bins[threadIdx.x];
+            int incl = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)threadIdx.x >= o) incl += u;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            int base = 0;
+            if (threadIdx.x == 0 && total > 0) base = atomicAdd(&P.cnt[nxt], total);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            s_bins[threadIdx.x] = base + incl - v;
+        }
+        __syncthreads();
+        if (want_next) kn = s_bins[dkey] + drank;
+    } else {
+        kn = warp_push(&P.cnt[nxt], want_next);
     }
-    __syncthreads();
-    const int kn = want_next ? s_bins[dkey] + drank : -1;
 #endif
     const int ks = warp_push(shadow_count(P), want_sh);
     if (want_next) {
@@ -974,6 +989,18 @@ static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 static inline int trace_scheme(int trace_mode) {
     return trace_mode >= 1 && trace_mode <= 5 ? trace_mode - 1 : DEFAULT_WALK_MODE;
 }
+// The scheme of a scene's frames: the default walk gives way to testing the records in step
+// (mode 5) where the four-wide tree is a single node of few records, unless the call asks for a
+// scheme or for traversal counts.  Closest-hit / any-hit ms of a 512x512, 16 spp, depth-6 frame,
+// walk against mode 5: 10 triangles and a light (7 records) 0.71 / 0.55 and 0.68 / 0.54; 12
+// triangles, a light and a sphere (9) 0.96 / 0.61 and 0.93 / 0.65; and of the 256x256, 16 spp,
+// depth-8 Cornell frame (9 records) 0.31 / 0.23 and 0.27 / 0.22.
+static inline int scene_scheme(const rumi_scene *sc, const rumi_render_params *p) {
+    const bool few = sc->n_wide == 1 && sc->n_recs <= RUMI_FEW_RECORDS;
+    return few && DEFAULT_WALK_MODE == 3 && p->trace_mode == 0 && !(p->flags & RUMI_FLAG_STATS)
+               ? 5
+               : trace_scheme(p->trace_mode);
+}
 bool uses_bvh8(int trace_mode) { return trace_scheme(trace_mode) == 4; }
 
 using ExtendKernel = void (*)(PtLaunch, int);
@@ -994,6 +1021,7 @@ static ExtendKernel extend_kernel(int mode, int smem) {
         case 0: return pt_extend<0, STATS>;
         case 1: return pt_extend<1, STATS>;
         case 2: return pt_extend<2, STATS>;
+        case 5: return pt_extend<5, STATS, 1>;
         case 3: return smem == 8 ? pt_extend<3, STATS, 8> : smem == 16 ? pt_extend<3, STATS, 16> : pt_extend<3, STATS>;
         default: return smem == 8 ? pt_extend<4, STATS, 8> : smem == 16 ? pt_extend<4, STATS, 16> : pt_extend<4, STATS>;
     }
@@ -1005,6 +1033,7 @@ static ShadowKernel shadow_kernel(int mode, int smem) {
         case 0: return pt_shadow<0, ADJ>;
         case 1: return pt_shadow<1, ADJ>;
         case 2: return pt_shadow<2, ADJ>;
+        case 5: return pt_shadow<5, ADJ, 1>;
         case 3: return smem == 8 ? pt_shadow<3, ADJ, 8> : smem == 16 ? pt_shadow<3, ADJ, 16> : pt_shadow<3, ADJ>;
         default: return smem == 8 ? pt_shadow<4, ADJ, 8> : smem == 16 ? pt_shadow<4, ADJ, 16> : pt_shadow<4, ADJ>;
     }
@@ -1015,12 +1044,13 @@ static ShadowKernel shadow_kernel(int mode, int smem) {
 // forward pass of a scene (render, forward with or without kept radiance, the first pass of
 // backward, a batch of such scenes) takes the same instantiation, so their paths agree bit
 // for bit; the two instantiations differ in the compiler's FMA contraction, not in the
-// algorithm.
-static void launch_shade(bool lean, cudaStream_t st, const PtLaunch &L, int b) {
-    if (lean)
-        pt_shade<false, true><<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
-    else
-        pt_shade<false><<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
+// algorithm.  group: the general kernel groups the block's next rays by direction; without it
+// (frames of scheme 5, which gains nothing from the order) it has no block-wide barriers: 1.37
+// against 1.42 ms of shading in a 333x251, 25 spp, depth-9 frame of a medium around a glass
+// sphere.  The lean kernel is the other way round (0.40 against 0.38 ms, Cornell frame).
+static void launch_shade(bool lean, bool group, cudaStream_t st, const PtLaunch &L, int b) {
+    const auto k = lean ? pt_shade<false, true> : (group ? pt_shade<false> : pt_shade<false, false, false>);
+    k<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
 }
 
 template <bool STATS>
@@ -1169,7 +1199,7 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
     clear_counters(L, stream);
 
     // traversal scheme and persistent grid (autotuner knobs; 0 = defaults)
-    const int mode = trace_scheme(p->trace_mode);
+    const int mode = scene_scheme(sc, p);
     const int smem = stack_entries(p->stack_depth);
     L.refill_min = p->refill_min > 0 ? p->refill_min : 8;
     const bool timing = (p->flags & RUMI_FLAG_TIMING) != 0;
@@ -1218,7 +1248,7 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
                 if (whitted)
                     pt_shade_whitted<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(L, b);
                 else
-                    launch_shade(lean, stream, L, b);
+                    launch_shade(lean, lean || mode != 5, stream, L, b);
                 if (timing) { mark(); shade_ev.push_back({e0, e0 + 1}); }
                 const bool aside = b + 1 < bounces;
                 cudaStream_t ss = aside ? sc->aux_stream : stream;
@@ -1251,7 +1281,7 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
             if (whitted)
                 pt_shade_whitted<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(L, b);
             else
-                launch_shade(lean, stream, L, b);
+                launch_shade(lean, lean || mode != 5, stream, L, b);
             if (timing) { mark(); shade_ev.push_back({e0, e0 + 1}); }
             if (timing) { e0 = (int)evs.size(); mark(); }
             launch_shadow<false>(mode, smem, shadow_grid, stream, L);
@@ -1366,7 +1396,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
 
     // the same traversal scheme as rumi_render, so both passes and the forward frame
     // resolve exact-distance ties alike
-    const int mode = trace_scheme(p->trace_mode);
+    const int mode = scene_scheme(sc, p);
     const int smem = stack_entries(p->stack_depth);
     A.refill_min = B.refill_min = p->refill_min > 0 ? p->refill_min : 8;
     int grid = 0, grid_sh = 0, grid_dummy = 0, grid_sh_adj = 0;
@@ -1399,7 +1429,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
                 if (adj)
                     pt_shade<true><<<cdiv(X.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(X, b);
                 else
-                    launch_shade(shade_lean(sc), stream, X, b);
+                    launch_shade(shade_lean(sc), shade_lean(sc) || mode != 5, stream, X, b);
                 const bool aside = overlap && b + 1 < p->max_depth;
                 cudaStream_t ss = aside ? sc->aux_stream : stream;
                 if (aside) {
@@ -1497,7 +1527,7 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
             L.sh_set = b & 1;
             pt_trace_multi<false><<<grid, TRACE_THREADS, 0, stream>>>(L, b);
             if (b > 0 && aux) cudaStreamWaitEvent(stream, ev_join, 0);
-            launch_shade(F.lean, stream, L, b);
+            launch_shade(F.lean, true, stream, L, b);
             const bool aside = aux && b + 1 < F.max_depth;
             if (aside) {
                 cudaEventRecord(ev_fork, stream);

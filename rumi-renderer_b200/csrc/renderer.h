@@ -26,6 +26,7 @@ struct rumi_scene {
     float4 *leaf_prims = nullptr;
     WideNode *wide = nullptr;
     LeafRec *recs = nullptr;
+    int n_wide = 0, n_recs = 0;  // nodes, and leaf records with the empty one
     float4 *tri_shade = nullptr;
     float4 *tri_albedo = nullptr;
     float4 *rects = nullptr;

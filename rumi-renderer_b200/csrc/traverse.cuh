@@ -668,6 +668,43 @@ RUMI_D void wide_slabs(float4 N0, float4 N1, float4 N2, float4 N3, float4 N4, fl
     t3 = child(N1.z, N1.w, N2.w, N3.w, N4.w, h3);
 }
 
+// One ray per lane against a four-wide tree of a single node (every child a leaf), the warp in
+// step: a leaf that any lane's ray enters is read once for all lanes.  Called by all 32 lanes;
+// `on`: this lane has a ray.  The walk's hits exactly: it tests the records of the same leaves
+// (or, once it has a hit, of fewer), and the closest of them does not depend on the order.
+template <bool ANYHIT>
+RUMI_D HitRec few_isect(const DevScene &s, bool on, float3 o, float3 d, float tmax, bool in_obj) {
+    HitRec h;
+    h.t = 0.0f;
+    h.id = -1;
+    h.u = h.v = 0.0f;
+    h.back = 0;
+    on = on && !(d.x == 0.0f && d.y == 0.0f && d.z == 0.0f);  // bvh.cpp:161-162
+    const float3 inv = safe_inv(d), noi = mk3(-(o.x * inv.x), -(o.y * inv.y), -(o.z * inv.z));
+    float4 N0, N1, N2, N3, N4, N5;
+    ldg32(s.wide, N0, N1);
+    ldg32(s.wide + 2, N2, N3);
+    ldg32(s.wide + 4, N4, N5);
+    bool h0, h1, h2, h3;
+    float t0, t1, t2, t3;
+    wide_slabs(N0, N1, N2, N3, N4, inv, noi, tmax, h0, h1, h2, h3, t0, t1, t2, t3);
+    const RayPairs rp = {make_float4(d.x, d.x, d.y, d.y), make_float4(d.z, d.z, o.x, o.x),
+                         make_float4(o.y, o.y, o.z, o.z)};
+    TraceStats st{0, 0};
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const int ref = __float_as_int(k == 0 ? N5.x : k == 1 ? N5.y : k == 2 ? N5.z : N5.w);
+        bool in = on && (k == 0 ? h0 : k == 1 ? h1 : k == 2 ? h2 : h3);
+        for (int i = ~ref; __any_sync(0xffffffffu, in); ++i) {
+            bool last = (__float_as_uint(__ldg(&s.recs[6 * (size_t)i + 4].z)) & REC_LAST) != 0;
+            const bool end = last;
+            if (in && rec_isect<ANYHIT, false>(s.recs, i, rp, tmax, in_obj, h, last, st) && ANYHIT) in = on = false;
+            if (end) break;
+        }
+    }
+    return h;
+}
+
 // Speculative while-while traversal with per-lane refill (Aila & Laine, "Understanding
 // the efficiency of ray traversal on GPUs", HPG 2009; Aila, Laine & Karras 2012) over the
 // four-wide tree (wide.cuh): each lane walks interior nodes until it holds a postponed leaf, and
@@ -1183,6 +1220,8 @@ RUMI_D void traverse_queue_walk(SceneOf scene_of, int n, int *counter, int refil
 //           leaves, then the warp intersects those leaves together.
 //   MODE 3: speculative while-while over the four-wide tree (traverse_queue_ww).
 //   MODE 4: the same scheme over the compressed eight-wide tree (traverse_queue_ww8).
+//   MODE 5: a warp takes 32 rays and tests the records of a single-node four-wide tree in step
+//           (few_isect).
 // smem_block: the block's STACK_SMEM * WW_THREADS ints.  fetch(i, o, d, tmax, in_obj) loads ray i; finish(i, hit) consumes its result.
 template <int MODE, bool ANYHIT, int STACK_SMEM, bool STATS, typename Fetch, typename Finish>
 RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_min, int *smem_block, Fetch fetch,
@@ -1209,6 +1248,18 @@ RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_mi
     if (MODE == 3) {
         traverse_queue_ww<ANYHIT, STACK_SMEM, STATS, false>([&](int) { return &s; }, n, counter, refill_min, smem_block,
                                                             fetch, finish, st);
+        return;
+    }
+    if (MODE == 5) {
+        for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n; base += gridDim.x * blockDim.x) {
+            const int i = base + lane;
+            float3 o = mk3(0, 0, 0), d = mk3(0, 0, 0);
+            float tmax = 0.0f;
+            bool in_obj = false;
+            if (i < n) fetch(i, o, d, tmax, in_obj);
+            const HitRec h = few_isect<ANYHIT>(s, i < n, o, d, tmax, in_obj);
+            if (i < n) finish(i, h);
+        }
         return;
     }
     if (MODE == 4) {
