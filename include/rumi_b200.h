@@ -353,6 +353,12 @@ rumi_status rumi_film_tonemap(const float *film, int32_t width, int32_t height, 
 rumi_status rumi_film_fireflies(const uint8_t *in, int32_t width, int32_t height, int32_t bytes_per_pixel,
                                 uint8_t *out, int32_t on_device, void *stream);
 
+/* Page-locked host memory for buffers that results are copied to (a film copied to ordinary
+ * memory goes through a staging buffer of the driver, and into pages that the system has
+ * yet to map).  rumi_host_free(NULL) does nothing. */
+rumi_status rumi_host_alloc(size_t bytes, void **out);
+rumi_status rumi_host_free(void *p);
+
 /* Text of the calling thread's last error ("" if none). */
 const char *rumi_last_error_string(void);
 

@@ -192,6 +192,7 @@ void free_scene(rumi_scene *sc) {
     if (sc->ev_fork) cudaEventDestroy(sc->ev_fork);
     if (sc->ev_join) cudaEventDestroy(sc->ev_join);
     if (s) cudaStreamSynchronize(s);  // nothing uses the workspace any more
+    if (sc->stage) cudaFreeHost(sc->stage);
     workspace_release(sc);
     if (s) {
         cudaStreamSynchronize(s);
@@ -579,11 +580,30 @@ rumi_status rumi_render(rumi_scene *sc, const rumi_render_params *p, float *film
     return st;
 }
 
+rumi_status rumi_host_alloc(size_t bytes, void **out) {
+    if (!out) return set_error("out is NULL"), RUMI_ERR_INVALID_ARG;
+    *out = nullptr;
+    const cudaError_t e = cudaHostAlloc(out, bytes > 0 ? bytes : 1, cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+        *out = nullptr;
+        cudaGetLastError();
+        return cuda_status(e, "page-locked allocation");
+    }
+    return RUMI_OK;
+}
+
+rumi_status rumi_host_free(void *p) {
+    if (!p) return RUMI_OK;
+    const cudaError_t e = cudaFreeHost(p);
+    return e == cudaSuccess ? RUMI_OK : cuda_status(e, "cudaFreeHost");
+}
+
 rumi_status rumi_trace_rays(rumi_scene *sc, int64_t n, const float *rays, int32_t anyhit, float *t, int32_t *prim,
                             int32_t on_device, int64_t *node_visits, int64_t *prim_tests, void *stream) {
     if (!sc || n < 0 || (n > 0 && (!rays || !t || !prim))) return set_error("bad argument"), RUMI_ERR_INVALID_ARG;
     cudaStream_t s = stream ? (cudaStream_t)stream : sc->stream;
     if (on_device) return trace_rays(sc, n, rays, anyhit, t, prim, node_visits, prim_tests, s);
+    if (n > 0 && n <= STAGED_RAYS) return trace_rays_staged(sc, n, rays, anyhit, t, prim, node_visits, prim_tests, s);
     float *dr = nullptr, *dt = nullptr;
     int32_t *dp = nullptr;
     rumi_status st = RUMI_OK;

@@ -55,6 +55,8 @@ struct rumi_scene {
     cudaStream_t stream = nullptr;
     int device = 0;
     int num_sms = 148;
+    // page-locked staging of small host ray queries (trace_rays_staged), made on first use
+    void *stage = nullptr;
     // render workspace, grown on demand
     void *ws = nullptr;
     size_t ws_bytes = 0;
@@ -114,6 +116,11 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
                          float4 *keep_L = nullptr);
 rumi_status trace_rays(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, float *t_dev, int32_t *prim_dev,
                        int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream);
+// The same for up to STAGED_RAYS rays in host memory: through the scene's page-locked staging
+// buffer, one copy each way.
+static constexpr int64_t STAGED_RAYS = 8192;
+rumi_status trace_rays_staged(rumi_scene *sc, int64_t n, const float *rays, int anyhit, float *t, int32_t *prim,
+                              int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream);
 rumi_status trace_rays_scheme(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, int trace_mode,
                               float *t_dev, int32_t *prim_dev, cudaStream_t stream);
 rumi_status ensure_workspace(rumi_scene *sc, size_t bytes);

@@ -9,7 +9,7 @@ import ctypes as C
 
 import numpy as np
 
-from . import _capi
+from . import _capi, hostmem
 from .scene import (Scene, FlatScene, PathTracer, BidirectionalPathTracer, RayTracer, PATH_TRACER, BDPT, RAY_TRACER,
                     LIGHT_AREA, LIGHT_SPOT, LIGHT_IBL, TEX_CHECKER, TEX_IMAGE)
 
@@ -162,7 +162,7 @@ class GpuScene:
             _capi.check(self.lib.rumi_render(self.h, C.byref(p), C.c_void_p(film_device_ptr), 1, C.byref(st)),
                         "rumi_render")
             return None, st.as_dict()
-        film = np.zeros((self.height, self.width, 3), np.float32)
+        film = hostmem.empty((self.height, self.width, 3), np.float32)
         _capi.check(self.lib.rumi_render(self.h, C.byref(p), film.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_render")
         return film, st.as_dict()
@@ -192,7 +192,7 @@ class GpuScene:
             _capi.check(self.lib.rumi_forward(self.h, C.byref(p), C.c_void_p(film_device_ptr), 1, C.byref(st)),
                         "rumi_forward")
             return None, st.as_dict()
-        film = np.zeros((self.height, self.width, 3), np.float32)
+        film = hostmem.empty((self.height, self.width, 3), np.float32)
         _capi.check(self.lib.rumi_forward(self.h, C.byref(p), film.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_forward")
         return film, st.as_dict()
@@ -323,7 +323,7 @@ class GpuBatch:
             _capi.check(self.lib.rumi_render_batch(self.h, C.byref(p), C.c_void_p(films_device_ptr), 1, C.byref(st)),
                         "rumi_render_batch")
             return None, st.as_dict()
-        flat = np.zeros(self.n_floats, np.float32)
+        flat = hostmem.empty((self.n_floats,), np.float32)
         _capi.check(self.lib.rumi_render_batch(self.h, C.byref(p), flat.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_render_batch")
         films, o = [], 0

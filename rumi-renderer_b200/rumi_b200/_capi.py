@@ -125,6 +125,10 @@ def load(path: str = LIB_PATH):
     L.rumi_trace_rays.restype = C.c_int
     L.rumi_trace_rays.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,
                                   C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.c_void_p]
+    L.rumi_host_alloc.restype = C.c_int
+    L.rumi_host_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
+    L.rumi_host_free.restype = C.c_int
+    L.rumi_host_free.argtypes = [C.c_void_p]
     L.rumi_batch_create.restype = C.c_int
     L.rumi_batch_create.argtypes = [C.POINTER(C.c_void_p), C.c_int32, C.POINTER(C.c_void_p)]
     L.rumi_batch_destroy.restype = C.c_int

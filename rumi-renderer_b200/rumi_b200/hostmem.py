@@ -1,0 +1,76 @@
+"""Result arrays in page-locked memory.
+
+A film copied to a fresh numpy array costs more in page faults and staging copies than the
+frame's last kernels (3.7 MB: 0.5 ms).  ``empty`` hands out arrays over page-locked blocks that
+go back to a pool when the last view of them is gone; the pool and what it has handed out are
+bounded together, and beyond the bound (or without a device) the array is an ordinary one."""
+from __future__ import annotations
+
+import ctypes as C
+import threading
+import weakref
+
+import numpy as np
+
+from . import _capi
+
+LIMIT = 256 << 20    # bytes of page-locked memory, handed out and pooled
+SMALLEST = 1 << 16   # block sizes are powers of two from here
+
+
+class _Pool:
+    def __init__(self, limit: int = LIMIT):
+        self.limit = limit
+        self.total = 0
+        self.free = {}
+        # a finalizer can run inside any allocation of the thread that holds the lock
+        self.lock = threading.RLock()
+
+    def take(self, size: int):
+        """Address of a block of `size` bytes (a power of two), or None."""
+        with self.lock:
+            blocks = self.free.get(size)
+            if blocks:
+                return blocks.pop()
+            if self.total + size > self.limit:
+                self._drop(self.total + size - self.limit)
+            if self.total + size > self.limit:
+                return None
+            self.total += size
+        p = C.c_void_p()
+        if _capi.load().rumi_host_alloc(size, C.byref(p)) != 0:
+            with self.lock:
+                self.total -= size
+            return None
+        return p.value
+
+    def _drop(self, need: int):
+        """Gives pooled blocks of other sizes back, largest first."""
+        for size in sorted(self.free, reverse=True):
+            while need > 0 and self.free[size]:
+                _capi.load().rumi_host_free(C.c_void_p(self.free[size].pop()))
+                self.total -= size
+                need -= size
+
+    def give(self, address: int, size: int):
+        with self.lock:
+            self.free.setdefault(size, []).append(address)
+
+
+_pool = _Pool()
+
+
+def empty(shape, dtype) -> np.ndarray:
+    """An uninitialised C-contiguous array, page-locked when the pool has room."""
+    dtype = np.dtype(dtype)
+    count = int(np.prod(shape, dtype=np.int64))
+    need = count * dtype.itemsize
+    if need == 0 or need > _pool.limit // 4:
+        return np.empty(shape, dtype)
+    size = max(SMALLEST, 1 << (need - 1).bit_length())
+    address = _pool.take(size)
+    if address is None:
+        return np.empty(shape, dtype)
+    block = (C.c_char * size).from_address(address)
+    weakref.finalize(block, _pool.give, address, size).atexit = False
+    return np.frombuffer(block, dtype, count).reshape(shape)
