@@ -91,7 +91,7 @@ class rumi_bvh_info(C.Structure):
 
 # every symbol include/rumi_b200.h and include/rumi_b200_test.h declare
 EXPORTS = ["rumi_scene_create", "rumi_scene_destroy", "rumi_scene_bvh_info", "rumi_render", "rumi_render_noalloc",
-           "rumi_trace_rays", "rumi_batch_create", "rumi_batch_destroy", "rumi_batch_film_floats",
+           "rumi_host_alloc", "rumi_host_free", "rumi_trace_rays", "rumi_batch_create", "rumi_batch_destroy", "rumi_batch_film_floats",
            "rumi_render_batch", "rumi_forward", "rumi_backward", "rumi_scene_set_albedo", "rumi_scene_set_volume",
            "rumi_film_tonemap", "rumi_film_fireflies",
            "rumi_last_error_string", "rumi_version",
