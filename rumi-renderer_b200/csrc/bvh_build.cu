@@ -6,29 +6,39 @@
 // entirely on the GPU and deterministically (same input -> same tree):
 //
 //  large phase (tasks with > SMALL_MAX primitives), one level per iteration:
-//    make_chunks   one block: chunk list (CHUNK primitives each); reset_bins: empty bins
-//                  for every task
-//    bin           one block per chunk: 3 axes x 32 centroid bins in shared memory,
-//                  merged into the task's bins with global atomics (ordered-int floats)
-//    split         one warp per task, lane = bin: prefix/suffix scans, SAH argmin
-//    count/scan/scatter  stable partition: per-chunk left counts, per-task scan,
-//                  per-chunk block scan + scatter; child bounds by block reduction
-//    emit          child nodes + next-level tasks, or small tasks
-//  small phase: one warp per task with <= SMALL_MAX primitives builds its whole subtree
-//    in shared memory (binned SAH, ballot-based stable partition, explicit stack),
-//    allocating node pairs from a range reserved by its primitive range.
+//    bin           one block per chunk of CHUNK primitives: 3 axes x 32 centroid bins in shared
+//                  memory, merged into the task's bins with global atomics (ordered-int floats)
+//    split         one warp per task, lane = bin: prefix/suffix scans, SAH argmin; empties what
+//                  this level's scatter and the next level's bin accumulate into
+//    count/scan/scatter  stable partition into the other index array: per-chunk left counts,
+//                  per-task scan, per-chunk block scan + scatter; child bounds by block reduction
+//    level         one block: child nodes, the next level's tasks in order and their chunks,
+//                  small tasks
+//  small phase, one warp per task, the subtree built in shared memory (binned SAH, ballot-based
+//    stable partition, explicit stack): first down to tasks of SMALL_MID primitives, then, a warp
+//    for each of those, to the leaves.  (A warp that built a whole 256-primitive subtree was the
+//    longest kernel of a build: 0.8 of 2.6 ms for 262k triangles, most SMs idle at its end.)
 //
-// Node index space: [0] root, [1] unused (pairs start 64-byte aligned), small-phase
-// region [2, 2 + 2N), large-phase region after it.
+// No launch depends on a count that the host would have to read: grids are sized by what a level
+// can hold and kernels stop at the device's counts.  The host looks once after the expected number
+// of levels and once at the end.
+//
+// Node index space: [0] root, [1] unused (pairs start 64-byte aligned), then one pair per split, at
+// the position of its boundary in the primitive order (node 2 + 2 m for the split in front of
+// primitive m, which no other split of the tree shares), then pairs for splits that leave a side
+// empty.
 #include "bvh_build.h"
 #include <cstdio>
+#include <type_traits>
 
 namespace rumi {
 
 static constexpr int NBINS = 32;
-static constexpr int CHUNK = 2048;
+static constexpr int CHUNK = 1024;
 static constexpr int BIN_THREADS = 256;
+static constexpr int PAIRS = 2;  // first node of the pair region
 static constexpr int SMALL_MAX = 256;
+static constexpr int SMALL_MID = 64;
 // Leaf size cap and SAH traversal cost (relative to one primitive test).  Measured on the
 // 1024x1024x64 BVH-bound frame (ms): cap 8 / C_TRAV 1: 239; cap 16 / 1: 239; 16 / 1.5: 250;
 // 16, 24 or 32 / 2: 225.5; 16 / 3: 231; 8 / 2: 250 (larger leaves pay only when the cap
@@ -46,8 +56,29 @@ static constexpr float C_TRAV = RUMI_SAH_CTRAV;
 static constexpr float C_ISECT = 1.0f;
 
 struct BuildTask {
-    int first, count, node, depth;
+    int first, count, node;
+    int depth;  // a small task's depth carries the index array that holds it (IN_TMP)
 };
+static constexpr int IN_TMP = 1 << 20;
+
+// Device counters of a build.
+enum { K_LARGE = 0, K_LARGE1 = 1, K_SMALL = 2, K_CHUNKS = 3, K_ERR = 4, K_MID = 5, K_LEVELS = 6, K_SPARE = 7, K_NUM = 16 };
+
+// Appends a task to one of the small phase's lists (n + 1 entries; a task per primitive at most,
+// and empty sides of degenerate splits).
+__device__ __forceinline__ void append_task(BuildTask *list, int *count, const BuildTask &t, int n, int *counters) {
+    const int k = atomicAdd(count, 1);
+    if (k <= n)
+        list[k] = t;
+    else
+        atomicExch(counters + K_ERR, 5);
+}
+
+// Nodes of a split's two children: the pair of its boundary, or (a side is empty) a spare pair.
+__device__ __forceinline__ int split_pair(int first, int nleft, int count, int n, int *counters) {
+    if (nleft > 0 && nleft < count) return PAIRS + 2 * (first + nleft);
+    return PAIRS + 2 * n + 2 * atomicAdd(counters + K_SPARE, 1);
+}
 
 struct Bounds12 {  // ordered ints: aabb lo/hi, centroid lo/hi
     int v[12];
@@ -91,8 +122,10 @@ __device__ __forceinline__ float3 centroid(float4 lo, float4 hi) {
 // triangle however its edges round) and its 48-byte intersection record.
 __global__ void prim_prepare_kernel(const float *tri_v, int n_tris, const float4 *rects, int n_rects,
                                     const float4 *spheres, const int *prim_flags, int n_spheres,
-                                    float4 *aabb_lo, float4 *aabb_hi, float4 *prims) {
+                                    float4 *aabb_lo, float4 *aabb_hi, float4 *prims, int *idx, int *root_bounds) {
     const int N = n_tris + n_rects + n_spheres;
+    float b[12];  // of this thread's primitives: box low / high, centroid low / high
+    for (int j = 0; j < 12; ++j) b[j] = (j % 6) < 3 ? INFINITY : -INFINITY;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         float3 lo, hi;
         float4 A, B, C;
@@ -129,86 +162,54 @@ __global__ void prim_prepare_kernel(const float *tri_v, int n_tris, const float4
         }
         aabb_lo[i] = make_float4(lo.x, lo.y, lo.z, 0.0f);
         aabb_hi[i] = make_float4(hi.x, hi.y, hi.z, 0.0f);
+        idx[i] = i;
+        const float3 c = centroid(aabb_lo[i], aabb_hi[i]);
+        b[0] = fminf(b[0], lo.x); b[1] = fminf(b[1], lo.y); b[2] = fminf(b[2], lo.z);
+        b[3] = fmaxf(b[3], hi.x); b[4] = fmaxf(b[4], hi.y); b[5] = fmaxf(b[5], hi.z);
+        b[6] = fminf(b[6], c.x); b[7] = fminf(b[7], c.y); b[8] = fminf(b[8], c.z);
+        b[9] = fmaxf(b[9], c.x); b[10] = fmaxf(b[10], c.y); b[11] = fmaxf(b[11], c.z);
         prims[3 * (size_t)i + 0] = A;
         prims[3 * (size_t)i + 1] = B;
         prims[3 * (size_t)i + 2] = C;
     }
-}
-
-__global__ void iota_kernel(int *idx, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) idx[i] = i;
-}
-
-// Root bounds + root task (one block).
-__global__ void root_kernel(const float4 *aabb_lo, const float4 *aabb_hi, int n, BvhNode *nodes,
-                            BuildTask *large, int *n_large, BuildTask *small, int *n_small) {
-    __shared__ float red[6][32];
-    float3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        float4 a = aabb_lo[i], b = aabb_hi[i];
-        lo = mk3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
-        hi = mk3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-    }
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    if (lane == 0) {
-        red[0][w] = lo.x; red[1][w] = lo.y; red[2][w] = lo.z;
-        red[3][w] = hi.x; red[4][w] = hi.y; red[5][w] = hi.z;
+    __shared__ int s_b[12];
+    if (threadIdx.x < 12) s_b[threadIdx.x] = (threadIdx.x % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+    __syncthreads();
+    for (int j = 0; j < 12; ++j) {
+        const bool mx = (j % 6) >= 3;
+        int v = f2o(b[j]);
+        v = mx ? __reduce_max_sync(0xffffffffu, v) : __reduce_min_sync(0xffffffffu, v);
+        if ((threadIdx.x & 31) == 0) {
+            if (mx)
+                atomicMax(s_b + j, v);
+            else
+                atomicMin(s_b + j, v);
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < nw; ++k) {
-            lo.x = fminf(lo.x, red[0][k]); lo.y = fminf(lo.y, red[1][k]); lo.z = fminf(lo.z, red[2][k]);
-            hi.x = fmaxf(hi.x, red[3][k]); hi.y = fmaxf(hi.y, red[4][k]); hi.z = fmaxf(hi.z, red[5][k]);
-        }
-        if (n == 0) {
-            BvhNode &r = nodes[0];
-            r.lo_x = r.lo_y = r.lo_z = INFINITY;
-            r.hi_x = r.hi_y = r.hi_z = -INFINITY;
-            r.first = 0;
-            r.count = 1;  // an empty leaf that is never entered
-            *n_large = 0;
-            *n_small = 0;
-            return;
-        }
-        write_node_bounds(nodes, 0, lo, hi);
-        nodes[1] = nodes[0];
-        nodes[1].count = -1;  // unused slot
-        BuildTask t;
-        t.first = 0; t.count = n; t.node = 0; t.depth = 0;
-        if (n > SMALL_MAX) {
-            large[0] = t;
-            *n_large = 1;
-            *n_small = 0;
-        } else {
-            small[0] = t;
-            *n_small = 1;
-            *n_large = 0;
-        }
+    if (threadIdx.x < 12) {
+        if ((threadIdx.x % 6) < 3)
+            atomicMin(root_bounds + threadIdx.x, s_b[threadIdx.x]);
+        else
+            atomicMax(root_bounds + threadIdx.x, s_b[threadIdx.x]);
     }
 }
 
-// ------------------------------------------------------------- large phase
+__global__ void init_kernel(int *root_bounds, int *counters) {
+    if (threadIdx.x < 12) root_bounds[threadIdx.x] = (threadIdx.x % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+    if (threadIdx.x < K_NUM) counters[threadIdx.x] = 0;
+}
+
 struct ChunkInfo {
     int task;
     int start;   // absolute index into idx
     int len;
 };
 
-// One block: chunk list for this level's tasks, bins reset, per-task centroid bounds
-// (taken from the task's node box is not enough -- centroid bounds come from cb).
-__global__ void make_chunks_kernel(const BuildTask *tasks, const int *n_tasks_p, ChunkInfo *chunks, int *n_chunks,
-                                   int *bins /*[task][3][NBINS][7]*/) {
+// One block: the chunks of `n_tasks` tasks (consecutive per task), and each task's first chunk.
+__device__ void list_chunks(const BuildTask *tasks, int n_tasks, ChunkInfo *chunks, int *task_first_chunk, int *n_chunks) {
     __shared__ int s_scan[1024];
     __shared__ int s_base;
-    const int n_tasks = *n_tasks_p;
     if (threadIdx.x == 0) s_base = 0;
     __syncthreads();
     for (int t0 = 0; t0 < n_tasks; t0 += blockDim.x) {
@@ -225,6 +226,7 @@ __global__ void make_chunks_kernel(const BuildTask *tasks, const int *n_tasks_p,
         const int excl = s_scan[threadIdx.x] - nc + s_base;
         if (t < n_tasks) {
             const BuildTask tk = tasks[t];
+            task_first_chunk[t] = excl;
             for (int c = 0; c < nc; ++c) {
                 ChunkInfo ci;
                 ci.task = t;
@@ -240,18 +242,48 @@ __global__ void make_chunks_kernel(const BuildTask *tasks, const int *n_tasks_p,
     if (threadIdx.x == 0) *n_chunks = s_base;
 }
 
-// Empty bins for every task of the level (count 0, bounds +inf / -inf as ordered ints),
-// grid-stride: a level can hold thousands of tasks.
-__global__ void reset_bins_kernel(const int *n_tasks_p, int *bins /*[task][3][NBINS][7]*/) {
-    const int n = *n_tasks_p * 3 * NBINS;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int *b = bins + 7 * (size_t)i;
+__device__ __forceinline__ void empty_bins(int *bins, int from, int step) {
+    for (int i = from; i < 3 * NBINS; i += step) {
+        int *b = bins + 7 * i;
         b[0] = 0;
         b[1] = b[2] = b[3] = f2o(INFINITY);
         b[4] = b[5] = b[6] = f2o(-INFINITY);
     }
 }
 
+// Root node and root task (one block).
+__global__ void root_kernel(const int *root_bounds, int n, BvhNode *nodes, BuildTask *large, int *cb, BuildTask *small,
+                            int *bins, ChunkInfo *chunks, int *task_first_chunk, int *counters) {
+    if (threadIdx.x == 0) {
+        if (n == 0) {
+            BvhNode &r = nodes[0];
+            r.lo_x = r.lo_y = r.lo_z = INFINITY;
+            r.hi_x = r.hi_y = r.hi_z = -INFINITY;
+            r.first = 0;
+            r.count = 1;  // an empty leaf that is never entered
+        } else {
+            const int *b = root_bounds;
+            write_node_bounds(nodes, 0, mk3(o2f(b[0]), o2f(b[1]), o2f(b[2])), mk3(o2f(b[3]), o2f(b[4]), o2f(b[5])));
+            nodes[1] = nodes[0];
+            nodes[1].count = -1;  // unused slot
+            BuildTask t;
+            t.first = 0; t.count = n; t.node = 0; t.depth = 0;
+            if (n > SMALL_MAX) {
+                large[0] = t;
+                for (int j = 0; j < 6; ++j) cb[j] = b[6 + j];
+                counters[K_LARGE] = 1;
+            } else {
+                small[0] = t;
+                counters[K_SMALL] = 1;
+            }
+        }
+    }
+    empty_bins(bins, threadIdx.x, blockDim.x);
+    __syncthreads();
+    if (n > SMALL_MAX) list_chunks(large, 1, chunks, task_first_chunk, counters + K_CHUNKS);
+}
+
+// ------------------------------------------------------------- large phase
 // centroid bounds of each task, stored as ordered ints in cb[task][6]
 __global__ void bin_kernel(const ChunkInfo *chunks, const int *n_chunks, const int *idx, const float4 *aabb_lo,
                            const float4 *aabb_hi, const int *cb, int *bins) {
@@ -259,11 +291,7 @@ __global__ void bin_kernel(const ChunkInfo *chunks, const int *n_chunks, const i
     const int c = blockIdx.x;
     if (c >= *n_chunks) return;
     const ChunkInfo ci = chunks[c];
-    for (int i = threadIdx.x; i < 3 * NBINS; i += blockDim.x) {
-        s_bins[7 * i + 0] = 0;
-        s_bins[7 * i + 1] = s_bins[7 * i + 2] = s_bins[7 * i + 3] = f2o(INFINITY);
-        s_bins[7 * i + 4] = s_bins[7 * i + 5] = s_bins[7 * i + 6] = f2o(-INFINITY);
-    }
+    empty_bins(s_bins, threadIdx.x, blockDim.x);
     __syncthreads();
     const int *tcb = cb + 6 * ci.task;
     const float cmin[3] = {o2f(tcb[0]), o2f(tcb[1]), o2f(tcb[2])};
@@ -376,10 +404,14 @@ __device__ void warp_sah(const int *bins /* [3][NBINS][7] */, float &best_cost, 
     }
 }
 
-__global__ void split_kernel(const BuildTask *tasks, const int *n_tasks, const int *bins, const BvhNode *nodes,
-                             SplitDecision *dec) {
+// next_bins: the other level's bins, emptied here for the children of every task.
+__global__ void split_kernel(const BuildTask *tasks, const int *n_tasks, const int *bins, int *next_bins, int max_tasks,
+                             int *child_bounds, SplitDecision *dec) {
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= *n_tasks) return;
+    const int lane = threadIdx.x & 31;
+    if (lane < 24) child_bounds[24 * t + lane] = (lane % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+    for (int k = 2 * t; k < 2 * t + 2 && k < max_tasks; ++k) empty_bins(next_bins + (size_t)k * 3 * NBINS * 7, lane, 32);
     const BuildTask tk = tasks[t];
     float cost;
     int axis, bin, nl;
@@ -463,13 +495,6 @@ __global__ void chunk_scan_kernel(const ChunkInfo *chunks, const int *n_chunks, 
         if (any_invalid) break;
     }
     if (lane == 0) dec[t].nleft = running;  // exact left count of the partition
-}
-
-__global__ void task_first_chunk_kernel(const ChunkInfo *chunks, const int *n_chunks, int *task_first_chunk) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= *n_chunks) return;
-    const int t = chunks[c].task;
-    if (c == 0 || chunks[c - 1].task != t) task_first_chunk[t] = c;
 }
 
 __global__ void scatter_kernel(const ChunkInfo *chunks, const int *n_chunks, const BuildTask *tasks,
@@ -563,284 +588,305 @@ __global__ void scatter_kernel(const ChunkInfo *chunks, const int *n_chunks, con
     }
 }
 
-__global__ void copy_back_kernel(const ChunkInfo *chunks, const int *n_chunks, const int *idx_tmp, int *idx) {
-    const int c = blockIdx.x;
-    if (c >= *n_chunks) return;
-    const ChunkInfo ci = chunks[c];
-    for (int k = threadIdx.x; k < ci.len; k += blockDim.x) idx[ci.start + k] = idx_tmp[ci.start + k];
-}
-
-__global__ void reset_child_bounds_kernel(int *child_bounds, const int *n_tasks) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * (*n_tasks) * 12) return;
-    const int j = i % 12;
-    child_bounds[i] = ((j % 6) < 3) ? f2o(INFINITY) : f2o(-INFINITY);
-}
-
-// Children of every large task: node pair, bounds, next tasks.  Large children go to
-// slot 2t+s of a sparse array (compacted in order afterwards, so the next level's task
-// order -- and with it the node layout -- is deterministic); small children are
-// appended with an atomic counter (their processing order does not matter: each small
-// subtree writes only the node range reserved by its primitive range).
-__global__ void emit_kernel(const BuildTask *tasks, const int *n_tasks, const SplitDecision *dec,
-                            const int *child_bounds, BvhNode *nodes, int pair_base, BuildTask *sparse,
-                            int *sparse_cb, BuildTask *small, int *n_small) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *n_tasks) return;
-    const BuildTask tk = tasks[t];
-    const SplitDecision d = dec[t];
-    const int pair = pair_base + 2 * t;
-    nodes[tk.node].first = pair;
-    nodes[tk.node].count = 0;
-    for (int s = 0; s < 2; ++s) {
-        const int *b = child_bounds + 12 * (2 * t + s);
-        const int node = pair + s;
-        write_node_bounds(nodes, node, mk3(o2f(b[0]), o2f(b[1]), o2f(b[2])), mk3(o2f(b[3]), o2f(b[4]), o2f(b[5])));
-        nodes[node].first = 0;
-        nodes[node].count = 0;
-        BuildTask ch;
-        ch.first = s == 0 ? tk.first : tk.first + d.nleft;
-        ch.count = s == 0 ? d.nleft : tk.count - d.nleft;
-        ch.node = node;
-        ch.depth = tk.depth + 1;
-        BuildTask sl = ch;
-        if (ch.count > SMALL_MAX) {
-            for (int j = 0; j < 6; ++j) sparse_cb[6 * (2 * t + s) + j] = b[6 + j];
-        } else {
-            const int k = atomicAdd(n_small, 1);
-            small[k] = ch;
-            sl.count = 0;
-        }
-        sparse[2 * t + s] = sl;
-    }
-}
-
-// One block: ordered compaction of the sparse child slots into the next level's tasks.
-__global__ void compact_next_kernel(const BuildTask *sparse, const int *sparse_cb, const int *n_tasks_p,
-                                    BuildTask *next, int *next_cb, int *n_next) {
-    __shared__ int s_scan[1024];
+// One block: the children of every large task (node pair, bounds), the next level's tasks (large
+// children in order, so that the task order and with it the build is deterministic) with their
+// centroid bounds and chunks, and small tasks, appended in any order (each builds only the nodes
+// and index range of its own primitives).  in_tmp: which index array this level's scatter filled.
+__global__ void level_kernel(const BuildTask *tasks, int *n_tasks_p, const SplitDecision *dec, const int *child_bounds,
+                             int n, int max_nodes, BvhNode *nodes, BuildTask *next, int *next_cb, int *n_next, BuildTask *small,
+                             int in_tmp, ChunkInfo *chunks, int *task_first_chunk, int *counters) {
+    __shared__ int s_warp[32];
     __shared__ int s_base;
-    const int m = 2 * (*n_tasks_p);
-    if (threadIdx.x == 0) s_base = 0;
+    const int n_tasks = *n_tasks_p;
+    if (n_tasks == 0) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        s_base = 0;
+        ++counters[K_LEVELS];
+    }
     __syncthreads();
-    for (int i0 = 0; i0 < m; i0 += blockDim.x) {
+    for (int i0 = 0; i0 < 2 * n_tasks; i0 += blockDim.x) {  // thread = child i = 2 task + side
         const int i = i0 + threadIdx.x;
-        const int f = (i < m && sparse[i].count > 0) ? 1 : 0;
-        s_scan[threadIdx.x] = f;
-        __syncthreads();
-        for (int o = 1; o < blockDim.x; o <<= 1) {
-            int v = threadIdx.x >= o ? s_scan[threadIdx.x - o] : 0;
-            __syncthreads();
-            s_scan[threadIdx.x] += v;
-            __syncthreads();
+        const bool here = i < 2 * n_tasks;
+        BuildTask ch;
+        const int *b = child_bounds + 12 * (size_t)i;
+        bool large = false;
+        int pair = 0;
+        if (here && (i & 1) == 0) {
+            const BuildTask tk = tasks[i >> 1];
+            pair = split_pair(tk.first, dec[i >> 1].nleft, tk.count, n, counters);
+            if (pair + 1 >= max_nodes) {
+                atomicExch(counters + K_ERR, 4);
+                pair = 0;
+            } else {
+                nodes[tk.node].first = pair;
+                nodes[tk.node].count = 0;
+            }
         }
-        const int base = s_base;
-        const int dst = base + s_scan[threadIdx.x] - f;
-        if (f) {
-            next[dst] = sparse[i];
-            for (int j = 0; j < 6; ++j) next_cb[6 * dst + j] = sparse_cb[6 * i + j];
+        pair = __shfl_sync(0xffffffffu, pair, lane & ~1);
+        if (here && pair > 0) {
+            const BuildTask tk = tasks[i >> 1];
+            const int nleft = dec[i >> 1].nleft, side = i & 1;
+            ch.first = side == 0 ? tk.first : tk.first + nleft;
+            ch.count = side == 0 ? nleft : tk.count - nleft;
+            ch.node = pair + side;
+            ch.depth = tk.depth + 1;
+            write_node_bounds(nodes, ch.node, mk3(o2f(b[0]), o2f(b[1]), o2f(b[2])), mk3(o2f(b[3]), o2f(b[4]), o2f(b[5])));
+            nodes[ch.node].first = 0;
+            nodes[ch.node].count = 0;
+            large = ch.count > SMALL_MAX;
+            if (!large) {
+                ch.depth |= in_tmp ? IN_TMP : 0;
+                append_task(small, counters + K_SMALL, ch, n, counters);
+            }
+        }
+        // ordered compaction of the large children
+        const unsigned m = __ballot_sync(0xffffffffu, large);
+        if (lane == 0) s_warp[w] = __popc(m);
+        __syncthreads();
+        int before = 0, total = 0;
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+            if (k < w) before += s_warp[k];
+            total += s_warp[k];
+        }
+        if (large) {
+            const int dst = s_base + before + __popc(m & ((1u << lane) - 1u));
+            next[dst] = ch;
+            for (int j = 0; j < 6; ++j) next_cb[6 * dst + j] = b[6 + j];
         }
         __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) s_base = base + s_scan[threadIdx.x];
+        if (threadIdx.x == 0) s_base += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) *n_next = s_base;
+    const int m = s_base;
+    if (threadIdx.x == 0) {
+        *n_next = m;
+        *n_tasks_p = 0;  // counts the level after next
+    }
+    list_chunks(next, m, chunks, task_first_chunk, counters + K_CHUNKS);
 }
 
 // ------------------------------------------------------------- small phase
 static constexpr int SMALL_WARPS = 4;
 static constexpr int SMALL_STACK = 24;
 
-__global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const BuildTask *small, const int *n_small,
-                                                                        int *idx, const float4 *aabb_lo,
-                                                                        const float4 *aabb_hi, BvhNode *nodes,
-                                                                        int small_region, int *error_flag) {
-    __shared__ int s_idx[SMALL_WARPS][SMALL_MAX];
-    __shared__ int s_tmp[SMALL_WARPS][SMALL_MAX];
+// MAX: primitives of a task.  mid != nullptr: children of up to SMALL_MID primitives become tasks of
+// the second pass instead of being built here.
+template <int MAX>
+__global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const BuildTask *small, const int *n_small, int n,
+                                                                        int *idx, const int *idx_tmp, const float4 *aabb_lo,
+                                                                        const float4 *aabb_hi, BvhNode *nodes, int max_nodes,
+                                                                        BuildTask *mid, int *counters) {
+    __shared__ int s_idx[SMALL_WARPS][MAX];
+    __shared__ int s_tmp[SMALL_WARPS][MAX];
     __shared__ int s_bins[SMALL_WARPS][3 * NBINS * 7];
+    int *error_flag = counters + K_ERR;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * SMALL_WARPS + w;
-    if (t >= *n_small) return;
-    const BuildTask root = small[t];
     int *sidx = s_idx[w];
     int *stmp = s_tmp[w];
     int *sb = s_bins[w];
-    for (int k = lane; k < root.count; k += 32) sidx[k] = idx[root.first + k];
-    __syncwarp();
-    int alloc = small_region + 2 * root.first;  // reserved pairs for this subtree
-    // stack entries: off, count, node, depth
-    int st_off[SMALL_STACK], st_cnt[SMALL_STACK], st_node[SMALL_STACK], st_dep[SMALL_STACK];
-    int sp = 0;
-    int off = 0, cnt = root.count, node = root.node, dep = root.depth;
-    for (;;) {
-        // centroid bounds of this sub-range
-        float3 cmn = mk3(INFINITY, INFINITY, INFINITY), cmx = mk3(-INFINITY, -INFINITY, -INFINITY);
-        for (int k = lane; k < cnt; k += 32) {
-            const int p = sidx[off + k];
-            const float3 c = centroid(aabb_lo[p], aabb_hi[p]);
-            cmn = mk3(fminf(cmn.x, c.x), fminf(cmn.y, c.y), fminf(cmn.z, c.z));
-            cmx = mk3(fmaxf(cmx.x, c.x), fmaxf(cmx.y, c.y), fmaxf(cmx.z, c.z));
+    const int n_tasks = min(*n_small, n + 1);
+    for (int t = blockIdx.x * SMALL_WARPS + w; t < n_tasks; t += gridDim.x * SMALL_WARPS) {
+        __syncwarp();
+        BuildTask root = small[t];
+        const int *src = (root.depth & IN_TMP) ? idx_tmp : idx;
+        root.depth &= ~IN_TMP;
+        for (int k = lane; k < root.count; k += 32) sidx[k] = src[root.first + k];
+        __syncwarp();
+        if (mid && root.count <= SMALL_MID) {
+            for (int k = lane; k < root.count; k += 32) idx[root.first + k] = sidx[k];
+            if (lane == 0) append_task(mid, counters + K_MID, root, n, counters);
+            continue;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            cmn.x = fminf(cmn.x, __shfl_xor_sync(0xffffffffu, cmn.x, o));
-            cmn.y = fminf(cmn.y, __shfl_xor_sync(0xffffffffu, cmn.y, o));
-            cmn.z = fminf(cmn.z, __shfl_xor_sync(0xffffffffu, cmn.z, o));
-            cmx.x = fmaxf(cmx.x, __shfl_xor_sync(0xffffffffu, cmx.x, o));
-            cmx.y = fmaxf(cmx.y, __shfl_xor_sync(0xffffffffu, cmx.y, o));
-            cmx.z = fmaxf(cmx.z, __shfl_xor_sync(0xffffffffu, cmx.z, o));
-        }
-        bool make_leaf = cnt <= 1 || dep >= MAX_DEPTH;
-        float best_cost = INFINITY;
-        int axis = -1, bin = 0, nleft = cnt / 2;
-        const float cminv[3] = {cmn.x, cmn.y, cmn.z}, cmaxv[3] = {cmx.x, cmx.y, cmx.z};
-        float scale[3];
-        for (int a = 0; a < 3; ++a) {
-            const float ext = cmaxv[a] - cminv[a];
-            scale[a] = ext > 0.0f ? (float)NBINS * (1.0f - 1e-6f) / ext : 0.0f;
-        }
-        if (!make_leaf) {
-            for (int i = lane; i < 3 * NBINS; i += 32) {
-                sb[7 * i + 0] = 0;
-                sb[7 * i + 1] = sb[7 * i + 2] = sb[7 * i + 3] = f2o(INFINITY);
-                sb[7 * i + 4] = sb[7 * i + 5] = sb[7 * i + 6] = f2o(-INFINITY);
-            }
-            __syncwarp();
+        // stack entries: off, count, node, depth
+        int st_off[SMALL_STACK], st_cnt[SMALL_STACK], st_node[SMALL_STACK], st_dep[SMALL_STACK];
+        int sp = 0;
+        int off = 0, cnt = root.count, node = root.node, dep = root.depth;
+        for (;;) {
+            // centroid bounds of this sub-range
+            float3 cmn = mk3(INFINITY, INFINITY, INFINITY), cmx = mk3(-INFINITY, -INFINITY, -INFINITY);
             for (int k = lane; k < cnt; k += 32) {
                 const int p = sidx[off + k];
-                const float4 lo = aabb_lo[p], hi = aabb_hi[p];
-                const float3 c = centroid(lo, hi);
-                const float cv[3] = {c.x, c.y, c.z};
-                for (int a = 0; a < 3; ++a) {
-                    int *b = sb + 7 * (a * NBINS + bin_of(cv[a], cminv[a], scale[a]));
-                    atomicAdd(b, 1);
-                    atomicMin(b + 1, f2o(lo.x)); atomicMin(b + 2, f2o(lo.y)); atomicMin(b + 3, f2o(lo.z));
-                    atomicMax(b + 4, f2o(hi.x)); atomicMax(b + 5, f2o(hi.y)); atomicMax(b + 6, f2o(hi.z));
+                const float3 c = centroid(aabb_lo[p], aabb_hi[p]);
+                cmn = mk3(fminf(cmn.x, c.x), fminf(cmn.y, c.y), fminf(cmn.z, c.z));
+                cmx = mk3(fmaxf(cmx.x, c.x), fmaxf(cmx.y, c.y), fmaxf(cmx.z, c.z));
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                cmn.x = fminf(cmn.x, __shfl_xor_sync(0xffffffffu, cmn.x, o));
+                cmn.y = fminf(cmn.y, __shfl_xor_sync(0xffffffffu, cmn.y, o));
+                cmn.z = fminf(cmn.z, __shfl_xor_sync(0xffffffffu, cmn.z, o));
+                cmx.x = fmaxf(cmx.x, __shfl_xor_sync(0xffffffffu, cmx.x, o));
+                cmx.y = fmaxf(cmx.y, __shfl_xor_sync(0xffffffffu, cmx.y, o));
+                cmx.z = fmaxf(cmx.z, __shfl_xor_sync(0xffffffffu, cmx.z, o));
+            }
+            bool make_leaf = cnt <= 1 || dep >= MAX_DEPTH;
+            float best_cost = INFINITY;
+            int axis = -1, bin = 0, nleft = cnt / 2;
+            const float cminv[3] = {cmn.x, cmn.y, cmn.z}, cmaxv[3] = {cmx.x, cmx.y, cmx.z};
+            float scale[3];
+            for (int a = 0; a < 3; ++a) {
+                const float ext = cmaxv[a] - cminv[a];
+                scale[a] = ext > 0.0f ? (float)NBINS * (1.0f - 1e-6f) / ext : 0.0f;
+            }
+            if (!make_leaf) {
+                for (int i = lane; i < 3 * NBINS; i += 32) {
+                    sb[7 * i + 0] = 0;
+                    sb[7 * i + 1] = sb[7 * i + 2] = sb[7 * i + 3] = f2o(INFINITY);
+                    sb[7 * i + 4] = sb[7 * i + 5] = sb[7 * i + 6] = f2o(-INFINITY);
                 }
-            }
-            __syncwarp();
-            int bx, bb, bn;
-            warp_sah(sb, best_cost, bx, bb, bn);
-            const BvhNode &nd = nodes[node];
-            const float parent_area = area_of(mk3(nd.lo_x, nd.lo_y, nd.lo_z), mk3(nd.hi_x, nd.hi_y, nd.hi_z));
-            if (bx >= 0 && dep < MEDIAN_DEPTH) {
-                const float split_cost = C_TRAV + C_ISECT * best_cost / fmaxf(parent_area, 1e-30f);
-                const float leaf_cost = C_ISECT * (float)cnt;
-                if (cnt <= LEAF_MAX && leaf_cost <= split_cost) make_leaf = true;
-                axis = bx;
-                bin = bb;
-                nleft = bn;
-            } else if (cnt <= 2 || (bx < 0 && cnt <= LEAF_MAX)) {
-                make_leaf = true;
-            }
-        }
-        if (make_leaf) {
-            if (lane == 0) {
-                nodes[node].first = root.first + off;
-                nodes[node].count = cnt;
-            }
-        } else {
-            // stable partition of sidx[off, off+cnt) by the decision
-            int lbase = 0, rbase = 0;
-            for (int g = 0; g < cnt; g += 32) {
-                const int k = g + lane;
-                bool L = false;
-                int p = -1;
-                if (k < cnt) {
-                    p = sidx[off + k];
-                    if (axis < 0) {
-                        L = k < nleft;
-                    } else {
-                        const float3 c = centroid(aabb_lo[p], aabb_hi[p]);
-                        const float cv = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-                        L = bin_of(cv, cminv[axis], scale[axis]) <= bin;
+                __syncwarp();
+                for (int k = lane; k < cnt; k += 32) {
+                    const int p = sidx[off + k];
+                    const float4 lo = aabb_lo[p], hi = aabb_hi[p];
+                    const float3 c = centroid(lo, hi);
+                    const float cv[3] = {c.x, c.y, c.z};
+                    for (int a = 0; a < 3; ++a) {
+                        int *b = sb + 7 * (a * NBINS + bin_of(cv[a], cminv[a], scale[a]));
+                        atomicAdd(b, 1);
+                        atomicMin(b + 1, f2o(lo.x)); atomicMin(b + 2, f2o(lo.y)); atomicMin(b + 3, f2o(lo.z));
+                        atomicMax(b + 4, f2o(hi.x)); atomicMax(b + 5, f2o(hi.y)); atomicMax(b + 6, f2o(hi.z));
                     }
                 }
-                const unsigned bl = __ballot_sync(0xffffffffu, k < cnt && L);
-                const unsigned br = __ballot_sync(0xffffffffu, k < cnt && !L);
-                const unsigned lt = (1u << lane) - 1u;
-                if (k < cnt) {
-                    const int dst = L ? off + lbase + __popc(bl & lt) : off + nleft + rbase + __popc(br & lt);
-                    if (dst >= off && dst < off + cnt)
-                        stmp[dst] = p;
-                    else
-                        atomicExch(error_flag, 2);
+                __syncwarp();
+                int bx, bb, bn;
+                warp_sah(sb, best_cost, bx, bb, bn);
+                const BvhNode &nd = nodes[node];
+                const float parent_area = area_of(mk3(nd.lo_x, nd.lo_y, nd.lo_z), mk3(nd.hi_x, nd.hi_y, nd.hi_z));
+                if (bx >= 0 && dep < MEDIAN_DEPTH) {
+                    const float split_cost = C_TRAV + C_ISECT * best_cost / fmaxf(parent_area, 1e-30f);
+                    const float leaf_cost = C_ISECT * (float)cnt;
+                    if (cnt <= LEAF_MAX && leaf_cost <= split_cost) make_leaf = true;
+                    axis = bx;
+                    bin = bb;
+                    nleft = bn;
+                } else if (cnt <= 2 || (bx < 0 && cnt <= LEAF_MAX)) {
+                    make_leaf = true;
                 }
-                lbase += __popc(bl);
-                rbase += __popc(br);
             }
-            __syncwarp();
-            for (int k = lane; k < cnt; k += 32) sidx[off + k] = stmp[off + k];
-            __syncwarp();
-            // child bounds
-            const int pair = alloc;
-            alloc += 2;
-            if (pair + 1 >= small_region + 2 * (root.first + root.count)) {  // cannot happen: <= cnt-1 splits
+            if (make_leaf) {
                 if (lane == 0) {
-                    atomicExch(error_flag, 3);
                     nodes[node].first = root.first + off;
                     nodes[node].count = cnt;
                 }
+            } else {
+                // stable partition of sidx[off, off+cnt) by the decision
+                int lbase = 0, rbase = 0;
+                for (int g = 0; g < cnt; g += 32) {
+                    const int k = g + lane;
+                    bool L = false;
+                    int p = -1;
+                    if (k < cnt) {
+                        p = sidx[off + k];
+                        if (axis < 0) {
+                            L = k < nleft;
+                        } else {
+                            const float3 c = centroid(aabb_lo[p], aabb_hi[p]);
+                            const float cv = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
+                            L = bin_of(cv, cminv[axis], scale[axis]) <= bin;
+                        }
+                    }
+                    const unsigned bl = __ballot_sync(0xffffffffu, k < cnt && L);
+                    const unsigned br = __ballot_sync(0xffffffffu, k < cnt && !L);
+                    const unsigned lt = (1u << lane) - 1u;
+                    if (k < cnt) {
+                        const int dst = L ? off + lbase + __popc(bl & lt) : off + nleft + rbase + __popc(br & lt);
+                        if (dst >= off && dst < off + cnt)
+                            stmp[dst] = p;
+                        else
+                            atomicExch(error_flag, 2);
+                    }
+                    lbase += __popc(bl);
+                    rbase += __popc(br);
+                }
                 __syncwarp();
-                if (sp == 0) break;
-                --sp;
-                off = st_off[sp]; cnt = st_cnt[sp]; node = st_node[sp]; dep = st_dep[sp];
+                for (int k = lane; k < cnt; k += 32) sidx[off + k] = stmp[off + k];
+                __syncwarp();
+                // child bounds
+                int pair = 0;
+                if (lane == 0) pair = split_pair(root.first + off, nleft, cnt, n, counters);
+                pair = __shfl_sync(0xffffffffu, pair, 0);
+                if (pair + 1 >= max_nodes) {  // cannot happen: a pair per boundary
+                    if (lane == 0) {
+                        atomicExch(error_flag, 3);
+                        nodes[node].first = root.first + off;
+                        nodes[node].count = cnt;
+                    }
+                    __syncwarp();
+                    if (sp == 0) break;
+                    --sp;
+                    off = st_off[sp]; cnt = st_cnt[sp]; node = st_node[sp]; dep = st_dep[sp];
+                    continue;
+                }
+                for (int s = 0; s < 2; ++s) {
+                    const int o2 = s == 0 ? off : off + nleft;
+                    const int c2 = s == 0 ? nleft : cnt - nleft;
+                    float3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
+                    for (int k = lane; k < c2; k += 32) {
+                        const int p = sidx[o2 + k];
+                        const float4 a = aabb_lo[p], b = aabb_hi[p];
+                        lo = mk3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
+                        hi = mk3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
+                    }
+                    for (int o = 16; o > 0; o >>= 1) {
+                        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+                        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+                        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+                        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+                        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+                        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+                    }
+                    if (lane == 0) {
+                        write_node_bounds(nodes, pair + s, lo, hi);
+                        nodes[pair + s].first = 0;
+                        nodes[pair + s].count = 0;
+                    }
+                }
+                if (lane == 0) {
+                    nodes[node].first = pair;
+                    nodes[node].count = 0;
+                }
+                // continue with the smaller child, push the larger one
+                const int lc = nleft, rc = cnt - nleft;
+                const bool left_small = lc <= rc;
+                const int so = left_small ? off : off + nleft, sc = left_small ? lc : rc, sn = left_small ? pair : pair + 1;
+                const int bo = left_small ? off + nleft : off, bc = left_small ? rc : lc, bn = left_small ? pair + 1 : pair;
+                if (mid && sc <= SMALL_MID) {  // (the smaller child first, so a deferred larger one implies it)
+                    if (lane == 0) append_task(mid, counters + K_MID, BuildTask{root.first + so, sc, sn, dep + 1}, n, counters);
+                    if (bc <= SMALL_MID) {
+                        if (lane == 0) append_task(mid, counters + K_MID, BuildTask{root.first + bo, bc, bn, dep + 1}, n, counters);
+                        __syncwarp();
+                        if (sp == 0) break;
+                        --sp;
+                        off = st_off[sp]; cnt = st_cnt[sp]; node = st_node[sp]; dep = st_dep[sp];
+                        continue;
+                    }
+                    off = bo; cnt = bc; node = bn; dep = dep + 1;
+                    __syncwarp();
+                    continue;
+                }
+                if (sp < SMALL_STACK) {
+                    st_off[sp] = bo; st_cnt[sp] = bc; st_node[sp] = bn; st_dep[sp] = dep + 1;
+                    ++sp;
+                } else {
+                    // cannot happen (stack depth <= log2(SMALL_MAX)); record and make a leaf
+                    if (lane == 0) {
+                        atomicExch(error_flag, 1);
+                        nodes[bn].first = root.first + bo;
+                        nodes[bn].count = bc;
+                    }
+                }
+                off = so; cnt = sc; node = sn; dep = dep + 1;
+                __syncwarp();
                 continue;
             }
-            for (int s = 0; s < 2; ++s) {
-                const int o2 = s == 0 ? off : off + nleft;
-                const int c2 = s == 0 ? nleft : cnt - nleft;
-                float3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
-                for (int k = lane; k < c2; k += 32) {
-                    const int p = sidx[o2 + k];
-                    const float4 a = aabb_lo[p], b = aabb_hi[p];
-                    lo = mk3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
-                    hi = mk3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-                    lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-                    lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-                    hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-                    hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-                    hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-                }
-                if (lane == 0) {
-                    write_node_bounds(nodes, pair + s, lo, hi);
-                    nodes[pair + s].first = 0;
-                    nodes[pair + s].count = 0;
-                }
-            }
-            if (lane == 0) {
-                nodes[node].first = pair;
-                nodes[node].count = 0;
-            }
-            // continue with the smaller child, push the larger one
-            const int lc = nleft, rc = cnt - nleft;
-            const bool left_small = lc <= rc;
-            const int so = left_small ? off : off + nleft, sc = left_small ? lc : rc, sn = left_small ? pair : pair + 1;
-            const int bo = left_small ? off + nleft : off, bc = left_small ? rc : lc, bn = left_small ? pair + 1 : pair;
-            if (sp < SMALL_STACK) {
-                st_off[sp] = bo; st_cnt[sp] = bc; st_node[sp] = bn; st_dep[sp] = dep + 1;
-                ++sp;
-            } else {
-                // cannot happen (stack depth <= log2(SMALL_MAX)); record and make a leaf
-                if (lane == 0) {
-                    atomicExch(error_flag, 1);
-                    nodes[bn].first = root.first + bo;
-                    nodes[bn].count = bc;
-                }
-            }
-            off = so; cnt = sc; node = sn; dep = dep + 1;
             __syncwarp();
-            continue;
+            if (sp == 0) break;
+            --sp;
+            off = st_off[sp]; cnt = st_cnt[sp]; node = st_node[sp]; dep = st_dep[sp];
         }
         __syncwarp();
-        if (sp == 0) break;
-        --sp;
-        off = st_off[sp]; cnt = st_cnt[sp]; node = st_node[sp]; dep = st_dep[sp];
+        for (int k = lane; k < root.count; k += 32) idx[root.first + k] = sidx[k];
     }
-    __syncwarp();
-    for (int k = lane; k < root.count; k += 32) idx[root.first + k] = sidx[k];
 }
 
 __global__ void gather_leaf_prims_kernel(const int *idx, int n, const float4 *prims_canon, float4 *leaf_prims) {
@@ -852,66 +898,64 @@ __global__ void gather_leaf_prims_kernel(const int *idx, int n, const float4 *pr
     }
 }
 
-// Centroid bounds of the root task (ordered ints) for the first large level.
-__global__ void root_cb_kernel(const float4 *aabb_lo, const float4 *aabb_hi, int n, int *cb) {
-    float3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float3 c = centroid(aabb_lo[i], aabb_hi[i]);
-        lo = mk3(fminf(lo.x, c.x), fminf(lo.y, c.y), fminf(lo.z, c.z));
-        hi = mk3(fmaxf(hi.x, c.x), fmaxf(hi.y, c.y), fmaxf(hi.z, c.z));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(cb + 0, f2o(lo.x)); atomicMin(cb + 1, f2o(lo.y)); atomicMin(cb + 2, f2o(lo.z));
-        atomicMax(cb + 3, f2o(hi.x)); atomicMax(cb + 4, f2o(hi.y)); atomicMax(cb + 5, f2o(hi.z));
-    }
-}
-
-__global__ void init_cb_kernel(int *cb) {
-    if (threadIdx.x < 6) cb[threadIdx.x] = threadIdx.x < 3 ? f2o(INFINITY) : f2o(-INFINITY);
-}
-
 // ---------------------------------------------------------------- host driver
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 int bvh_node_capacity(int n_prims) {
     const long long n = n_prims;
-    // root + pad, small region 2N, large region: <= N / SMALL_MAX tasks per level, 64 levels
-    long long cap = 2 + 2 * n + 2 * (n / SMALL_MAX + 1) * 64 + 64;
+    // root + pad, a pair per boundary, and spare pairs for splits that leave a side empty: at most
+    // one per task and level
+    long long cap = PAIRS + 2 * n + 2 * (n / SMALL_MAX + 1) * 64 + 64;
     return (int)cap;
 }
 
-size_t bvh_scratch_bytes(int n_prims) {
+// The build's arrays in its scratch memory.
+struct BuildArrays {
+    float4 *aabb_lo, *aabb_hi, *prims_canon;
+    int *idx[2];
+    BuildTask *tasks[2], *small, *mid;
+    int *cbs[2], *bins[2], *child_bounds;
+    ChunkInfo *chunks;
+    int *chunk_left, *chunk_loff, *task_first_chunk;
+    SplitDecision *dec;
+    int *root_bounds, *counters;
+};
+
+static size_t carve_build(BuildArrays &B, char *base, int n_prims) {
     const size_t n = (size_t)(n_prims > 0 ? n_prims : 1);
     const size_t max_tasks = n / SMALL_MAX + 2;
     const size_t max_chunks = n / CHUNK + max_tasks + 2;
-    size_t b = 0;
-    auto add = [&](size_t bytes) { b += (bytes + 255) & ~(size_t)255; };
-    add(n * sizeof(float4));                         // aabb_lo
-    add(n * sizeof(float4));                         // aabb_hi
-    add(3 * n * sizeof(float4));                     // prims_canon
-    add(n * sizeof(int));                            // idx
-    add(n * sizeof(int));                            // idx_tmp
-    add(2 * max_tasks * sizeof(BuildTask));          // large tasks (cur, next)
-    add(2 * max_tasks * 6 * sizeof(int));            // centroid bounds (cur, next)
-    add((n + 1) * sizeof(BuildTask));                // small tasks
-    add(max_chunks * sizeof(ChunkInfo));
-    add(max_chunks * sizeof(int) * 2);               // chunk_left, chunk_loff
-    add(max_tasks * sizeof(int));                    // task_first_chunk
-    add(max_tasks * sizeof(SplitDecision));
-    add(max_tasks * 3 * NBINS * 7 * sizeof(int));    // bins
-    add(2 * max_tasks * 12 * sizeof(int));           // child bounds
-    add(2 * max_tasks * sizeof(BuildTask));          // sparse next tasks
-    add(2 * max_tasks * 6 * sizeof(int));            // sparse centroid bounds
-    add(16 * sizeof(int));                           // counters
-    return b;
+    char *p = base;
+    auto take = [&](auto *&dst, size_t count) {
+        dst = reinterpret_cast<std::remove_reference_t<decltype(dst)>>(p);
+        p += (count * sizeof(*dst) + 255) & ~(size_t)255;
+    };
+    take(B.aabb_lo, n);
+    take(B.aabb_hi, n);
+    take(B.prims_canon, 3 * n);
+    take(B.idx[0], n);
+    take(B.idx[1], n);
+    for (int k = 0; k < 2; ++k) {
+        take(B.tasks[k], max_tasks);
+        take(B.cbs[k], max_tasks * 6);
+        take(B.bins[k], max_tasks * 3 * NBINS * 7);
+    }
+    take(B.small, n + 1);
+    take(B.mid, n + 1);
+    take(B.child_bounds, 2 * max_tasks * 12);
+    take(B.chunks, max_chunks);
+    take(B.chunk_left, max_chunks);
+    take(B.chunk_loff, max_chunks);
+    take(B.task_first_chunk, max_tasks);
+    take(B.dec, max_tasks);
+    take(B.root_bounds, 12);
+    take(B.counters, K_NUM);
+    return (size_t)(p - base);
+}
+
+size_t bvh_scratch_bytes(int n_prims) {
+    BuildArrays B;
+    return carve_build(B, nullptr, n_prims);
 }
 
 // Builds the BVH of the canonical primitives into `nodes` (bvh_node_capacity entries)
@@ -922,105 +966,72 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
               cudaStream_t stream, BvhBuildInfo *info) {
     const int N = n_tris + n_rects + n_spheres;
     const size_t n = (size_t)(N > 0 ? N : 1);
-    const size_t max_tasks = n / SMALL_MAX + 2;
-    const size_t max_chunks = n / CHUNK + max_tasks + 2;
-    char *p = (char *)scratch;
-    auto take = [&](size_t bytes) {
-        void *r = p;
-        p += (bytes + 255) & ~(size_t)255;
-        return r;
-    };
-    float4 *aabb_lo = (float4 *)take(n * sizeof(float4));
-    float4 *aabb_hi = (float4 *)take(n * sizeof(float4));
-    float4 *prims_canon = (float4 *)take(3 * n * sizeof(float4));
-    int *idx = (int *)take(n * sizeof(int));
-    int *idx_tmp = (int *)take(n * sizeof(int));
-    BuildTask *tasks[2];
-    tasks[0] = (BuildTask *)take(2 * max_tasks * sizeof(BuildTask));
-    tasks[1] = tasks[0] + max_tasks;
-    int *cbs[2];
-    cbs[0] = (int *)take(2 * max_tasks * 6 * sizeof(int));
-    cbs[1] = cbs[0] + max_tasks * 6;
-    BuildTask *small = (BuildTask *)take((n + 1) * sizeof(BuildTask));
-    ChunkInfo *chunks = (ChunkInfo *)take(max_chunks * sizeof(ChunkInfo));
-    int *chunk_left = (int *)take(max_chunks * sizeof(int) * 2);
-    int *chunk_loff = chunk_left + max_chunks;
-    int *task_first_chunk = (int *)take(max_tasks * sizeof(int));
-    SplitDecision *dec = (SplitDecision *)take(max_tasks * sizeof(SplitDecision));
-    int *bins = (int *)take(max_tasks * 3 * NBINS * 7 * sizeof(int));
-    int *child_bounds = (int *)take(2 * max_tasks * 12 * sizeof(int));
-    BuildTask *sparse = (BuildTask *)take(2 * max_tasks * sizeof(BuildTask));
-    int *sparse_cb = (int *)take(2 * max_tasks * 6 * sizeof(int));
-    int *counters = (int *)take(16 * sizeof(int));
-    // counters: [0] n_large cur [1] n_large next [2] n_small [3] n_chunks [4] error
-    int *n_cur = counters + 0, *n_small = counters + 2, *n_chunks = counters + 3, *err = counters + 4;
-
-    cudaMemsetAsync(counters, 0, 16 * sizeof(int), stream);
-    const int small_region = 2;
-    int pair_base = small_region + 2 * (int)n;
+    BuildArrays B;
+    carve_build(B, (char *)scratch, N);
+    int *kc = B.counters;
+    const int max_nodes = bvh_node_capacity(N);
     const int grid_n = cdiv((long long)n, 256) < 148 * 8 ? cdiv((long long)n, 256) : 148 * 8;
-    prim_prepare_kernel<<<grid_n > 0 ? grid_n : 1, 256, 0, stream>>>(d_tri_v, n_tris, d_rects, n_rects, d_spheres,
-                                                                     d_prim_flags, n_spheres, aabb_lo, aabb_hi,
-                                                                     prims_canon);
-    iota_kernel<<<grid_n > 0 ? grid_n : 1, 256, 0, stream>>>(idx, N);
-    root_kernel<<<1, 1024, 0, stream>>>(aabb_lo, aabb_hi, N, nodes, tasks[0], n_cur, small, n_small);
-    init_cb_kernel<<<1, 32, 0, stream>>>(cbs[0]);
-    root_cb_kernel<<<grid_n > 0 ? grid_n : 1, 256, 0, stream>>>(aabb_lo, aabb_hi, N, cbs[0]);
-
-    int cur = 0;
-    int levels = 0;
-    int h_n_tasks = 0;
-    cudaMemcpyAsync(&h_n_tasks, n_cur, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    cudaStreamSynchronize(stream);
-    while (h_n_tasks > 0) {
-        if (levels > 80 || (size_t)h_n_tasks > max_tasks) {
-            return -1;
-        }
-        int *ncur = counters + 0;  // current count lives in counters[0]
-        int *nnext = counters + 1;
-        const int max_ch = (int)(n / CHUNK) + h_n_tasks + 1;
-        make_chunks_kernel<<<1, 1024, 0, stream>>>(tasks[cur], ncur, chunks, n_chunks, bins);
-        reset_bins_kernel<<<cdiv(h_n_tasks * 3 * NBINS, 256), 256, 0, stream>>>(ncur, bins);
-        bin_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(chunks, n_chunks, idx, aabb_lo, aabb_hi, cbs[cur], bins);
-        split_kernel<<<cdiv(h_n_tasks * 32, 128), 128, 0, stream>>>(tasks[cur], ncur, bins, nodes, dec);
-        count_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(chunks, n_chunks, tasks[cur], dec, idx, aabb_lo, aabb_hi,
-                                                         cbs[cur], chunk_left);
-        task_first_chunk_kernel<<<cdiv(max_ch, 256), 256, 0, stream>>>(chunks, n_chunks, task_first_chunk);
-        chunk_scan_kernel<<<cdiv(h_n_tasks * 32, 128), 128, 0, stream>>>(chunks, n_chunks, ncur, chunk_left,
-                                                                         chunk_loff, task_first_chunk, dec);
-        reset_child_bounds_kernel<<<cdiv(2 * h_n_tasks * 12, 256), 256, 0, stream>>>(child_bounds, ncur);
-        scatter_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(chunks, n_chunks, tasks[cur], dec, idx, idx_tmp, aabb_lo,
-                                                           aabb_hi, cbs[cur], chunk_loff, child_bounds);
-        copy_back_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(chunks, n_chunks, idx_tmp, idx);
-        if (pair_base + 2 * h_n_tasks > bvh_node_capacity(N)) return -1;
-        emit_kernel<<<cdiv(h_n_tasks, 128), 128, 0, stream>>>(tasks[cur], ncur, dec, child_bounds, nodes, pair_base,
-                                                              sparse, sparse_cb, small, n_small);
-        compact_next_kernel<<<1, 1024, 0, stream>>>(sparse, sparse_cb, ncur, tasks[cur ^ 1], cbs[cur ^ 1], nnext);
-        pair_base += 2 * h_n_tasks;
-        // next level: its count moves into counters[0]
-        cudaMemcpyAsync(ncur, nnext, sizeof(int), cudaMemcpyDeviceToDevice, stream);
-        cudaMemcpyAsync(&h_n_tasks, nnext, sizeof(int), cudaMemcpyDeviceToHost, stream);
-        cudaStreamSynchronize(stream);
-        cur ^= 1;
-        ++levels;
+    init_kernel<<<1, 32, 0, stream>>>(B.root_bounds, kc);
+    prim_prepare_kernel<<<grid_n, 256, 0, stream>>>(d_tri_v, n_tris, d_rects, n_rects, d_spheres, d_prim_flags,
+                                                    n_spheres, B.aabb_lo, B.aabb_hi, B.prims_canon, B.idx[0],
+                                                    B.root_bounds);
+    root_kernel<<<1, 1024, 0, stream>>>(B.root_bounds, N, nodes, B.tasks[0], B.cbs[0], B.small, B.bins[0], B.chunks,
+                                        B.task_first_chunk, kc);
+    // a level halves its tasks at best; a task has more than SMALL_MAX primitives, so a level holds
+    // at most N / SMALL_MAX of them.  SAH splits are uneven: four levels more than halving takes,
+    // then as many as it needs, four at a time.
+    int level = 0, until = 0, h[K_NUM] = {};
+    if (N > SMALL_MAX) {
+        until = 4;
+        for (size_t m = n; m > SMALL_MAX; m >>= 1) ++until;
     }
-    int h_small = 0;
-    cudaMemcpyAsync(&h_small, n_small, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    cudaStreamSynchronize(stream);
-    if (h_small > 0)
-        small_build_kernel<<<cdiv(h_small, SMALL_WARPS), 32 * SMALL_WARPS, 0, stream>>>(
-            small, n_small, idx, aabb_lo, aabb_hi, nodes, small_region, err);
-    gather_leaf_prims_kernel<<<grid_n > 0 ? grid_n : 1, 256, 0, stream>>>(idx, N, prims_canon, leaf_prims);
-    int h_err = 0;
-    cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    cudaError_t e = cudaStreamSynchronize(stream);
+    for (;;) {
+        for (; level < until; ++level) {
+            const int cur = level & 1;
+            int *n_cur = kc + K_LARGE + cur, *n_next = kc + K_LARGE + (cur ^ 1);
+            long long most = level < 30 ? 1LL << level : (long long)n;
+            if (most > (long long)(n / SMALL_MAX) + 1) most = (long long)(n / SMALL_MAX) + 1;
+            const int max_ch = (int)((long long)(n / CHUNK) + most + 1), warps = cdiv(most * 32, 128);
+            bin_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(B.chunks, kc + K_CHUNKS, B.idx[cur], B.aabb_lo, B.aabb_hi,
+                                                           B.cbs[cur], B.bins[cur]);
+            split_kernel<<<warps, 128, 0, stream>>>(B.tasks[cur], n_cur, B.bins[cur], B.bins[cur ^ 1],
+                                                    (int)(n / SMALL_MAX + 2), B.child_bounds, B.dec);
+            count_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(B.chunks, kc + K_CHUNKS, B.tasks[cur], B.dec, B.idx[cur],
+                                                             B.aabb_lo, B.aabb_hi, B.cbs[cur], B.chunk_left);
+            chunk_scan_kernel<<<warps, 128, 0, stream>>>(B.chunks, kc + K_CHUNKS, n_cur, B.chunk_left, B.chunk_loff,
+                                                         B.task_first_chunk, B.dec);
+            scatter_kernel<<<max_ch, BIN_THREADS, 0, stream>>>(B.chunks, kc + K_CHUNKS, B.tasks[cur], B.dec, B.idx[cur],
+                                                               B.idx[cur ^ 1], B.aabb_lo, B.aabb_hi, B.cbs[cur],
+                                                               B.chunk_loff, B.child_bounds);
+            level_kernel<<<1, 1024, 0, stream>>>(B.tasks[cur], n_cur, B.dec, B.child_bounds, N, max_nodes, nodes,
+                                                 B.tasks[cur ^ 1], B.cbs[cur ^ 1], n_next, B.small, cur ^ 1, B.chunks,
+                                                 B.task_first_chunk, kc);
+        }
+        if (until == 0) break;
+        cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
+        const cudaError_t e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return (int)e;
+        if (h[K_ERR] || level > 80) return -1;
+        if (h[K_LARGE + (level & 1)] == 0) break;
+        until = level + 4;
+    }
+    const int small_grid = 148 * 8;  // resident blocks; warps take tasks in turn
+    small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(B.small, kc + K_SMALL, N, B.idx[0], B.idx[1],
+                                                                               B.aabb_lo, B.aabb_hi, nodes, max_nodes,
+                                                                               B.mid, kc);
+    small_build_kernel<SMALL_MID><<<2 * small_grid, 32 * SMALL_WARPS, 0, stream>>>(B.mid, kc + K_MID, N, B.idx[0], B.idx[1],
+                                                                                   B.aabb_lo, B.aabb_hi, nodes, max_nodes,
+                                                                                   nullptr, kc);
+    gather_leaf_prims_kernel<<<grid_n, 256, 0, stream>>>(B.idx[0], N, B.prims_canon, leaf_prims);
+    cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
+    const cudaError_t e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return (int)e;
-    if (h_err) return -1;
+    if (h[K_ERR]) return -1;
     if (info) {
-        info->large_levels = levels;
-        info->small_tasks = h_small;
-        info->node_capacity = bvh_node_capacity(N);
-        info->node_high_water = pair_base;
+        info->large_levels = h[K_LEVELS];
+        info->small_tasks = h[K_SMALL];
+        info->node_capacity = max_nodes;
+        info->node_high_water = PAIRS + 2 * (int)n + 2 * h[K_SPARE];
     }
     return 0;
 }
