@@ -39,6 +39,10 @@ static constexpr int BIN_THREADS = 256;
 static constexpr int PAIRS = 2;  // first node of the pair region
 static constexpr int SMALL_MAX = 256;
 static constexpr int SMALL_MID = 64;
+// Bins per axis of the tasks of up to SMALL_MID primitives: with ten, the three axes' bins are the
+// lanes of one warp and are scanned together (warp_sah_mid), a quarter of the work of three scans
+// of 32.
+static constexpr int MID_BINS = 10;
 // Leaf size cap and SAH traversal cost (relative to one primitive test).  Measured on the
 // 1024x1024x64 BVH-bound frame (ms): cap 8 / C_TRAV 1: 239; cap 16 / 1: 239; 16 / 1.5: 250;
 // 16, 24 or 32 / 2: 225.5; 16 / 3: 231; 8 / 2: 250 (larger leaves pay only when the cap
@@ -108,9 +112,9 @@ __device__ __forceinline__ void write_node_bounds(BvhNode *nodes, int n, float3 
     nd.hi_x = hi.x; nd.hi_y = hi.y; nd.hi_z = hi.z;
 }
 
-__device__ __forceinline__ int bin_of(float c, float cmin, float scale) {
+__device__ __forceinline__ int bin_of(float c, float cmin, float scale, int bins = NBINS) {
     int b = (int)((c - cmin) * scale);
-    return b < 0 ? 0 : (b >= NBINS ? NBINS - 1 : b);
+    return b < 0 ? 0 : (b >= bins ? bins - 1 : b);
 }
 
 __device__ __forceinline__ float3 centroid(float4 lo, float4 hi) {
@@ -160,6 +164,10 @@ __global__ void prim_prepare_kernel(const float *tri_v, int n_tris, const float4
                             __int_as_float(PRIM_SPHERE | (prim_flags[n_rects + s] ? PRIM_FLAG_IBL : 0)));
             C = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
+        // a coordinate that is NaN in all vertices bounds nothing (NaN orders above all numbers in
+        // the bins' integers, while the minima and maxima of floats drop it)
+        lo = mk3(lo.x == lo.x ? lo.x : INFINITY, lo.y == lo.y ? lo.y : INFINITY, lo.z == lo.z ? lo.z : INFINITY);
+        hi = mk3(hi.x == hi.x ? hi.x : -INFINITY, hi.y == hi.y ? hi.y : -INFINITY, hi.z == hi.z ? hi.z : -INFINITY);
         aabb_lo[i] = make_float4(lo.x, lo.y, lo.z, 0.0f);
         aabb_hi[i] = make_float4(hi.x, hi.y, hi.z, 0.0f);
         idx[i] = i;
@@ -402,6 +410,54 @@ __device__ void warp_sah(const int *bins /* [3][NBINS][7] */, float &best_cost, 
             best_nleft = nl;
         }
     }
+}
+
+// The same over MID_BINS bins of three axes, lane = 10 axis + bin.  Every lane also receives the
+// bounds of the two sides of the best split.
+__device__ void warp_sah_mid(const int *bins /* [3][MID_BINS][7] */, float &best_cost, int &best_axis, int &best_bin,
+                             int &best_nleft, float3 lo[2], float3 hi[2]) {
+    const int lane = threadIdx.x & 31, axis = lane / MID_BINS, bin = lane - axis * MID_BINS;
+    const bool on = axis < 3;
+    const int *b = bins + 7 * (on ? lane : 0);
+    int pc = on ? b[0] : 0;
+    float p[6], q[6];  // this bin and those before it / after it: low, high
+    for (int j = 0; j < 6; ++j) p[j] = q[j] = on ? o2f(b[1 + j]) : (j < 3 ? INFINITY : -INFINITY);
+    int sc = pc;
+    for (int o = 1; o < MID_BINS; o <<= 1) {
+        const int c1 = __shfl_up_sync(0xffffffffu, pc, o), c2 = __shfl_down_sync(0xffffffffu, sc, o);
+        float u[6], d[6];
+        for (int j = 0; j < 6; ++j) {
+            u[j] = __shfl_up_sync(0xffffffffu, p[j], o);
+            d[j] = __shfl_down_sync(0xffffffffu, q[j], o);
+        }
+        if (bin >= o) {
+            pc += c1;
+            for (int j = 0; j < 6; ++j) p[j] = j < 3 ? fminf(p[j], u[j]) : fmaxf(p[j], u[j]);
+        }
+        if (bin + o < MID_BINS && on) {
+            sc += c2;
+            for (int j = 0; j < 6; ++j) q[j] = j < 3 ? fminf(q[j], d[j]) : fmaxf(q[j], d[j]);
+        }
+    }
+    // the right side of a split after this bin
+    const int rc = __shfl_down_sync(0xffffffffu, sc, 1);
+    for (int j = 0; j < 6; ++j) q[j] = __shfl_down_sync(0xffffffffu, q[j], 1);
+    float cost = INFINITY;
+    if (on && bin < MID_BINS - 1 && pc > 0 && rc > 0)
+        cost = area_of(mk3(p[0], p[1], p[2]), mk3(p[3], p[4], p[5])) * (float)pc +
+               area_of(mk3(q[0], q[1], q[2]), mk3(q[3], q[4], q[5])) * (float)rc;
+    // costs are not negative, so their bits order like them; ties go to the lowest lane
+    const int least = __reduce_min_sync(0xffffffffu, __float_as_int(cost));
+    const unsigned at = __ballot_sync(0xffffffffu, __float_as_int(cost) == least);
+    const int best = __ffs(at) - 1;
+    best_cost = __int_as_float(least);
+    best_axis = best_cost < INFINITY ? best / MID_BINS : -1;
+    best_bin = best - (best / MID_BINS) * MID_BINS;
+    best_nleft = __shfl_sync(0xffffffffu, pc, best);
+    lo[0] = mk3(__shfl_sync(0xffffffffu, p[0], best), __shfl_sync(0xffffffffu, p[1], best), __shfl_sync(0xffffffffu, p[2], best));
+    hi[0] = mk3(__shfl_sync(0xffffffffu, p[3], best), __shfl_sync(0xffffffffu, p[4], best), __shfl_sync(0xffffffffu, p[5], best));
+    lo[1] = mk3(__shfl_sync(0xffffffffu, q[0], best), __shfl_sync(0xffffffffu, q[1], best), __shfl_sync(0xffffffffu, q[2], best));
+    hi[1] = mk3(__shfl_sync(0xffffffffu, q[3], best), __shfl_sync(0xffffffffu, q[4], best), __shfl_sync(0xffffffffu, q[5], best));
 }
 
 // next_bins: the other level's bins, emptied here for the children of every task.
@@ -672,6 +728,14 @@ static constexpr int SMALL_STACK = 24;
 
 // MAX: primitives of a task.  mid != nullptr: children of up to SMALL_MID primitives become tasks of
 // the second pass instead of being built here.
+// Minimum of lo / maximum of hi over the warp, in every lane.
+__device__ __forceinline__ void warp_bounds(float3 &lo, float3 &hi) {
+    lo = mk3(o2f(__reduce_min_sync(0xffffffffu, f2o(lo.x))), o2f(__reduce_min_sync(0xffffffffu, f2o(lo.y))),
+             o2f(__reduce_min_sync(0xffffffffu, f2o(lo.z))));
+    hi = mk3(o2f(__reduce_max_sync(0xffffffffu, f2o(hi.x))), o2f(__reduce_max_sync(0xffffffffu, f2o(hi.y))),
+             o2f(__reduce_max_sync(0xffffffffu, f2o(hi.z))));
+}
+
 template <int MAX>
 __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const BuildTask *small, const int *n_small, int n,
                                                                         int *idx, const int *idx_tmp, const float4 *aabb_lo,
@@ -679,7 +743,9 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                                                                         BuildTask *mid, int *counters) {
     __shared__ int s_idx[SMALL_WARPS][MAX];
     __shared__ int s_tmp[SMALL_WARPS][MAX];
-    __shared__ int s_bins[SMALL_WARPS][3 * NBINS * 7];
+    constexpr bool MID = MAX <= SMALL_MID;
+    constexpr int BINS = MID ? MID_BINS : NBINS;
+    __shared__ int s_bins[SMALL_WARPS][3 * BINS * 7];
     int *error_flag = counters + K_ERR;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *sidx = s_idx[w];
@@ -711,25 +777,19 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                 cmn = mk3(fminf(cmn.x, c.x), fminf(cmn.y, c.y), fminf(cmn.z, c.z));
                 cmx = mk3(fmaxf(cmx.x, c.x), fmaxf(cmx.y, c.y), fmaxf(cmx.z, c.z));
             }
-            for (int o = 16; o > 0; o >>= 1) {
-                cmn.x = fminf(cmn.x, __shfl_xor_sync(0xffffffffu, cmn.x, o));
-                cmn.y = fminf(cmn.y, __shfl_xor_sync(0xffffffffu, cmn.y, o));
-                cmn.z = fminf(cmn.z, __shfl_xor_sync(0xffffffffu, cmn.z, o));
-                cmx.x = fmaxf(cmx.x, __shfl_xor_sync(0xffffffffu, cmx.x, o));
-                cmx.y = fmaxf(cmx.y, __shfl_xor_sync(0xffffffffu, cmx.y, o));
-                cmx.z = fmaxf(cmx.z, __shfl_xor_sync(0xffffffffu, cmx.z, o));
-            }
+            warp_bounds(cmn, cmx);
             bool make_leaf = cnt <= 1 || dep >= MAX_DEPTH;
             float best_cost = INFINITY;
             int axis = -1, bin = 0, nleft = cnt / 2;
             const float cminv[3] = {cmn.x, cmn.y, cmn.z}, cmaxv[3] = {cmx.x, cmx.y, cmx.z};
             float scale[3];
+            float3 side_lo[2], side_hi[2];  // of the best split's sides (MID)
             for (int a = 0; a < 3; ++a) {
                 const float ext = cmaxv[a] - cminv[a];
-                scale[a] = ext > 0.0f ? (float)NBINS * (1.0f - 1e-6f) / ext : 0.0f;
+                scale[a] = ext > 0.0f ? (float)BINS * (1.0f - 1e-6f) / ext : 0.0f;
             }
             if (!make_leaf) {
-                for (int i = lane; i < 3 * NBINS; i += 32) {
+                for (int i = lane; i < 3 * BINS; i += 32) {
                     sb[7 * i + 0] = 0;
                     sb[7 * i + 1] = sb[7 * i + 2] = sb[7 * i + 3] = f2o(INFINITY);
                     sb[7 * i + 4] = sb[7 * i + 5] = sb[7 * i + 6] = f2o(-INFINITY);
@@ -741,7 +801,7 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                     const float3 c = centroid(lo, hi);
                     const float cv[3] = {c.x, c.y, c.z};
                     for (int a = 0; a < 3; ++a) {
-                        int *b = sb + 7 * (a * NBINS + bin_of(cv[a], cminv[a], scale[a]));
+                        int *b = sb + 7 * (a * BINS + bin_of(cv[a], cminv[a], scale[a], BINS));
                         atomicAdd(b, 1);
                         atomicMin(b + 1, f2o(lo.x)); atomicMin(b + 2, f2o(lo.y)); atomicMin(b + 3, f2o(lo.z));
                         atomicMax(b + 4, f2o(hi.x)); atomicMax(b + 5, f2o(hi.y)); atomicMax(b + 6, f2o(hi.z));
@@ -749,7 +809,10 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                 }
                 __syncwarp();
                 int bx, bb, bn;
-                warp_sah(sb, best_cost, bx, bb, bn);
+                if constexpr (MID)
+                    warp_sah_mid(sb, best_cost, bx, bb, bn, side_lo, side_hi);
+                else
+                    warp_sah(sb, best_cost, bx, bb, bn);
                 const BvhNode &nd = nodes[node];
                 const float parent_area = area_of(mk3(nd.lo_x, nd.lo_y, nd.lo_z), mk3(nd.hi_x, nd.hi_y, nd.hi_z));
                 if (bx >= 0 && dep < MEDIAN_DEPTH) {
@@ -782,7 +845,7 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                         } else {
                             const float3 c = centroid(aabb_lo[p], aabb_hi[p]);
                             const float cv = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-                            L = bin_of(cv, cminv[axis], scale[axis]) <= bin;
+                            L = bin_of(cv, cminv[axis], scale[axis], BINS) <= bin;
                         }
                     }
                     const unsigned bl = __ballot_sync(0xffffffffu, k < cnt && L);
@@ -821,19 +884,17 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
                     const int o2 = s == 0 ? off : off + nleft;
                     const int c2 = s == 0 ? nleft : cnt - nleft;
                     float3 lo = mk3(INFINITY, INFINITY, INFINITY), hi = mk3(-INFINITY, -INFINITY, -INFINITY);
-                    for (int k = lane; k < c2; k += 32) {
-                        const int p = sidx[o2 + k];
-                        const float4 a = aabb_lo[p], b = aabb_hi[p];
-                        lo = mk3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
-                        hi = mk3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
-                    }
-                    for (int o = 16; o > 0; o >>= 1) {
-                        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-                        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-                        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-                        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-                        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-                        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+                    if (MID && axis >= 0) {
+                        lo = side_lo[s];
+                        hi = side_hi[s];
+                    } else {
+                        for (int k = lane; k < c2; k += 32) {
+                            const int p = sidx[o2 + k];
+                            const float4 a = aabb_lo[p], b = aabb_hi[p];
+                            lo = mk3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
+                            hi = mk3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
+                        }
+                        warp_bounds(lo, hi);
                     }
                     if (lane == 0) {
                         write_node_bounds(nodes, pair + s, lo, hi);
