@@ -419,7 +419,21 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     float *d_tri_v = nullptr, *d_tri_n = nullptr, *d_alb = nullptr;
     int *d_rect_em = nullptr, *d_tri_m = nullptr;
     void *scratch = nullptr;
+    // what only shading reads (normals, material indices, colours) goes up on a second stream while
+    // the tree is built: 55 of a triangle's 91 bytes
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_side = nullptr;
+    auto drop_side = [&]() {
+        if (side) {
+            cudaStreamSynchronize(side);
+            cudaStreamDestroy(side);
+        }
+        if (ev_side) cudaEventDestroy(ev_side);
+        side = nullptr;
+        ev_side = nullptr;
+    };
     auto fail = [&](rumi_status code) {
+        drop_side();
         dfree(d_tri_v, s);
         dfree(d_tri_n, s);
         dfree(d_tri_m, s);
@@ -429,23 +443,7 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         free_scene(sc);
         return code;
     };
-    const int pack_grid = nT > 0 ? (nT + 255) / 256 < sc->num_sms * 8 ? (nT + 255) / 256 : sc->num_sms * 8 : 1;
     if ((st = upload(&d_tri_v, d->tri_vertices, sizeof(float) * 9 * (size_t)nT, s)) != RUMI_OK) return fail(st);
-    if (nT > 0) {
-        if (d->tri_normals &&
-            (st = upload(&d_tri_n, d->tri_normals, sizeof(float) * 9 * (size_t)nT, s)) != RUMI_OK)
-            return fail(st);
-        if ((st = upload(&d_tri_m, d->tri_material, sizeof(int) * (size_t)nT, s)) != RUMI_OK) return fail(st);
-        e = dalloc((void **)&sc->tri_shade, sizeof(float4) * 3 * (size_t)nT, s);
-        if (e != cudaSuccess) return fail(cuda_status(e, "device allocation"));
-        pack_tri_shade_kernel<<<pack_grid, 256, 0, s>>>(d_tri_v, d_tri_n, d_tri_m, nT, sc->tri_shade);
-        if (d->tri_albedo) {
-            if ((st = upload(&d_alb, d->tri_albedo, sizeof(float) * 3 * (size_t)nT, s)) != RUMI_OK) return fail(st);
-            e = dalloc((void **)&sc->tri_albedo, sizeof(float4) * (size_t)nT, s);
-            if (e != cudaSuccess) return fail(cuda_status(e, "device allocation"));
-            pack_albedo_kernel<<<pack_grid, 256, 0, s>>>(d_alb, nT, sc->tri_albedo);
-        }
-    }
     if ((st = upload(&sc->rects, rects.data(), sizeof(float4) * rects.size(), s)) != RUMI_OK) return fail(st);
     if ((st = upload(&d_rect_em, rect_emissive.data(), sizeof(int) * rect_emissive.size(), s)) != RUMI_OK)
         return fail(st);
@@ -454,6 +452,19 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     if ((st = upload(&sc->materials, mats.data(), sizeof(DevMaterial) * mats.size(), s)) != RUMI_OK) return fail(st);
     if ((st = upload(&sc->lights, lights.data(), sizeof(DevLight) * lights.size(), s)) != RUMI_OK) return fail(st);
     if ((st = upload_textures(sc, d, s)) != RUMI_OK) return fail(st);
+    if (nT > 0) {
+        if (d->tri_normals) e = dalloc((void **)&d_tri_n, sizeof(float) * 9 * (size_t)nT, s);
+        if (e == cudaSuccess) e = dalloc((void **)&d_tri_m, sizeof(int) * (size_t)nT, s);
+        if (e == cudaSuccess) e = dalloc((void **)&sc->tri_shade, sizeof(float4) * 3 * (size_t)nT, s);
+        if (e == cudaSuccess && d->tri_albedo) e = dalloc((void **)&d_alb, sizeof(float) * 3 * (size_t)nT, s);
+        if (e == cudaSuccess && d->tri_albedo) e = dalloc((void **)&sc->tri_albedo, sizeof(float4) * (size_t)nT, s);
+        if (e != cudaSuccess) return fail(cuda_status(e, "device allocation"));
+        e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_side, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(ev_side, s);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, ev_side, 0);
+        if (e != cudaSuccess) return fail(cuda_status(e, "upload stream"));
+    }
     // ---- BVH
     sc->n_nodes = bvh_node_capacity(N);
     e = dalloc((void **)&sc->nodes, sizeof(BvhNode) * (size_t)sc->n_nodes, s);
@@ -462,34 +473,67 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     if (e != cudaSuccess) return fail(cuda_status(e, "device allocation (primitives)"));
     e = dalloc(&scratch, bvh_scratch_bytes(N), s);
     if (e != cudaSuccess) return fail(cuda_status(e, "device allocation (BVH scratch)"));
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
+    // build time: from e0 to e1 without the stretch (w0 to w1) in which the GPU, its first launches
+    // done, may wait for the host's copies
+    cudaEvent_t e0, e1, w0, w1;
+    for (cudaEvent_t *ev : {&e0, &e1, &w0, &w1}) cudaEventCreate(ev);
+    auto drop_events = [&]() {
+        for (cudaEvent_t ev : {e0, e1, w0, w1}) cudaEventDestroy(ev);
+    };
+    rumi_status side_st = RUMI_OK;
+    auto upload_shading = [&]() {
+        if (nT == 0) return;
+        cudaEventRecord(w0, s);
+        // allocations on s, before its kernels; the copies and their packing on the side stream,
+        // behind the event that follows them
+        auto copy = [&](auto **dst, const void *src, size_t bytes) {
+            if (side_st != RUMI_OK) return;
+            const cudaError_t ce = cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, side);
+            if (ce != cudaSuccess) side_st = cuda_status(ce, "cudaMemcpyAsync");
+        };
+        const int pack_grid = (nT + 255) / 256 < sc->num_sms * 8 ? (nT + 255) / 256 : sc->num_sms * 8;
+        if (d->tri_normals) copy(&d_tri_n, d->tri_normals, sizeof(float) * 9 * (size_t)nT);
+        copy(&d_tri_m, d->tri_material, sizeof(int) * (size_t)nT);
+        if (d->tri_albedo) copy(&d_alb, d->tri_albedo, sizeof(float) * 3 * (size_t)nT);
+        if (side_st != RUMI_OK) return;
+        pack_tri_shade_kernel<<<pack_grid, 256, 0, side>>>(d_tri_v, d_tri_n, d_tri_m, nT, sc->tri_shade);
+        if (d->tri_albedo) pack_albedo_kernel<<<pack_grid, 256, 0, side>>>(d_alb, nT, sc->tri_albedo);
+        const cudaError_t ce = cudaEventRecord(ev_side, side);
+        if (ce != cudaSuccess) side_st = cuda_status(ce, "scene upload");
+        cudaEventRecord(w1, s);
+    };
     cudaEventRecord(e0, s);
     int rc = bvh_build(d_tri_v, nT, sc->rects, d_rect_em, nR, sc->spheres, nS, sc->nodes, sc->leaf_prims, scratch, s,
-                       &sc->info);
+                       &sc->info, upload_shading);
+    if (rc == 0 && side_st != RUMI_OK) {
+        drop_events();
+        return fail(side_st);
+    }
     if (rc != 0) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        drop_events();
         if (rc > 0) return fail(cuda_status((cudaError_t)rc, "bvh_build"));
         set_error("bvh_build: internal limit reached");
         return fail(RUMI_ERR_INTERNAL);
     }
     rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, &sc->wide, &sc->n_wide, &sc->recs, &sc->n_recs, s);
     if (rc != 0) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        drop_events();
         if (rc > 0) return fail(cuda_status((cudaError_t)rc, "four-wide BVH"));
         set_error("four-wide BVH collapse failed");
         return fail(RUMI_ERR_INTERNAL);
     }
     cudaEventRecord(e1, s);
     cudaEventSynchronize(e1);
-    float ms = 0.0f;
+    float ms = 0.0f, waited = 0.0f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    if (nT > 0) cudaEventElapsedTime(&waited, w0, w1);
+    ms -= waited;
+    drop_events();
     sc->build_ms = ms;
+    if (side) {
+        e = cudaStreamWaitEvent(s, ev_side, 0);  // the frees below follow the side stream's kernels
+        if (e != cudaSuccess) return fail(cuda_status(e, "scene upload"));
+    }
     dfree(d_tri_v, s);
     dfree(d_tri_n, s);
     dfree(d_tri_m, s);
@@ -520,6 +564,7 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     ds.n_textures = sc->textures ? d->n_textures : 0;
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(cuda_status(e, "scene upload"));
+    drop_side();
     if (uses_bvh8(0)) {  // the default walk is the eight-wide one: its tree is needed at once
         const rumi_status st8 = ensure_bvh8(sc);
         if (st8 != RUMI_OK) return fail(st8);

@@ -20,8 +20,8 @@
 //    longest kernel of a build: 0.8 of 2.6 ms for 262k triangles, most SMs idle at its end.)
 //
 // No launch depends on a count that the host would have to read: grids are sized by what a level
-// can hold and kernels stop at the device's counts.  The host looks once after the expected number
-// of levels and once at the end.
+// can hold and kernels stop at the device's counts.  The host looks once, after the expected
+// number of levels and the small phase.
 //
 // Node index space: [0] root, [1] unused (pairs start 64-byte aligned), then one pair per split, at
 // the position of its boundary in the primitive order (node 2 + 2 m for the split in front of
@@ -726,7 +726,7 @@ __global__ void level_kernel(const BuildTask *tasks, int *n_tasks_p, const Split
 static constexpr int SMALL_WARPS = 4;
 static constexpr int SMALL_STACK = 24;
 
-// MAX: primitives of a task.  mid != nullptr: children of up to SMALL_MID primitives become tasks of
+// MAX: primitives of a task.  The list's tasks from `begin` on.  mid != nullptr: children of up to SMALL_MID primitives become tasks of
 // the second pass instead of being built here.
 // Minimum of lo / maximum of hi over the warp, in every lane.
 __device__ __forceinline__ void warp_bounds(float3 &lo, float3 &hi) {
@@ -737,7 +737,7 @@ __device__ __forceinline__ void warp_bounds(float3 &lo, float3 &hi) {
 }
 
 template <int MAX>
-__global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const BuildTask *small, const int *n_small, int n,
+__global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const BuildTask *small, const int *n_small, int begin, int n,
                                                                         int *idx, const int *idx_tmp, const float4 *aabb_lo,
                                                                         const float4 *aabb_hi, BvhNode *nodes, int max_nodes,
                                                                         BuildTask *mid, int *counters) {
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) small_build_kernel(const Bui
     int *stmp = s_tmp[w];
     int *sb = s_bins[w];
     const int n_tasks = min(*n_small, n + 1);
-    for (int t = blockIdx.x * SMALL_WARPS + w; t < n_tasks; t += gridDim.x * SMALL_WARPS) {
+    for (int t = begin + blockIdx.x * SMALL_WARPS + w; t < n_tasks; t += gridDim.x * SMALL_WARPS) {
         __syncwarp();
         BuildTask root = small[t];
         const int *src = (root.depth & IN_TMP) ? idx_tmp : idx;
@@ -1024,7 +1024,7 @@ size_t bvh_scratch_bytes(int n_prims) {
 // success, else a cudaError_t value (or -1 when the builder's internal bounds were hit).
 int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int *d_prim_flags, int n_rects,
               const float4 *d_spheres, int n_spheres, BvhNode *nodes, float4 *leaf_prims, void *scratch,
-              cudaStream_t stream, BvhBuildInfo *info) {
+              cudaStream_t stream, BvhBuildInfo *info, std::function<void()> meanwhile) {
     const int N = n_tris + n_rects + n_spheres;
     const size_t n = (size_t)(N > 0 ? N : 1);
     BuildArrays B;
@@ -1068,7 +1068,14 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
                                                  B.tasks[cur ^ 1], B.cbs[cur ^ 1], n_next, B.small, cur ^ 1, B.chunks,
                                                  B.task_first_chunk, kc);
         }
-        if (until == 0) break;
+        // the small tasks found so far (all of them, unless the expected levels did not suffice)
+        const int small_grid = 148 * 8;  // resident blocks; warps take tasks in turn
+        small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(
+            B.small, kc + K_SMALL, h[K_SMALL], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, B.mid, kc);
+        small_build_kernel<SMALL_MID><<<2 * small_grid, 32 * SMALL_WARPS, 0, stream>>>(
+            B.mid, kc + K_MID, h[K_MID], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, nullptr, kc);
+        if (meanwhile) meanwhile();
+        meanwhile = nullptr;
         cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
         const cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return (int)e;
@@ -1076,18 +1083,7 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
         if (h[K_LARGE + (level & 1)] == 0) break;
         until = level + 4;
     }
-    const int small_grid = 148 * 8;  // resident blocks; warps take tasks in turn
-    small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(B.small, kc + K_SMALL, N, B.idx[0], B.idx[1],
-                                                                               B.aabb_lo, B.aabb_hi, nodes, max_nodes,
-                                                                               B.mid, kc);
-    small_build_kernel<SMALL_MID><<<2 * small_grid, 32 * SMALL_WARPS, 0, stream>>>(B.mid, kc + K_MID, N, B.idx[0], B.idx[1],
-                                                                                   B.aabb_lo, B.aabb_hi, nodes, max_nodes,
-                                                                                   nullptr, kc);
     gather_leaf_prims_kernel<<<grid_n, 256, 0, stream>>>(B.idx[0], N, B.prims_canon, leaf_prims);
-    cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
-    const cudaError_t e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return (int)e;
-    if (h[K_ERR]) return -1;
     if (info) {
         info->large_levels = h[K_LEVELS];
         info->small_tasks = h[K_SMALL];

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
+#include <functional>
 #include "scene.cuh"
 
 namespace rumi {
@@ -15,11 +16,12 @@ struct BvhBuildInfo {
 
 int bvh_node_capacity(int n_prims);
 size_t bvh_scratch_bytes(int n_prims);
+// meanwhile: host work done once after the first launches, while the GPU builds.
 // d_prim_flags: n_rects + n_spheres ints -- per rect "emissive" (one-sided test off), then
 // per sphere "image-based light" (far root from inside)
 int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int *d_prim_flags, int n_rects,
               const float4 *d_spheres, int n_spheres, BvhNode *nodes, float4 *leaf_prims, void *scratch,
-              cudaStream_t stream, BvhBuildInfo *info);
+              cudaStream_t stream, BvhBuildInfo *info, std::function<void()> meanwhile);
 
 // Four-wide tree of the default walk, collapsed from the binary one (bvh_wide.cu).  Returns 0, a
 // cudaError_t value, or -1 when an index left its range.
