@@ -429,13 +429,18 @@ RUMI_D bool nee_setup(const LightSample &ls, float3 p, float3 &wi, float &dist, 
 //                                          weight sigma_s / sigma_t (per channel)
 //   phase direction (applied at the next vertex) and NEE phase value: d log HG / d g
 //   binary shadow transmittance (applied by the shadow kernel to that NEE term alone).
-// Forward shading is bound by the latency of its scattered per-path loads: three blocks
-// of 256 threads per SM (80 registers, a 120-byte spill to L1) ran the 1024x1024x64
-// BVH-bound frame's shading in 31.0 ms against 37.7 ms at two blocks (118 registers);
-// four blocks (64 registers) gave the same as three.  The adjoint replay keeps its
-// registers.
+// Forward shading is bound by the latency of its scattered per-path loads and by instruction
+// fetch, so more warps pay even for spills: a 333x251, 25 spp, depth-9 frame of a medium around a
+// glass sphere shades in 1.56 / 1.43 / 1.37 ms at two / three / four blocks of 256 threads per SM
+// (118, 80 and 64 registers), 1.40 ms in blocks of 128 at the same 64 registers, 1.49 ms at 48.
+// The adjoint replay keeps its registers (two to four blocks: no difference).
 #ifndef RUMI_SHADE_MIN_BLOCKS
-#define RUMI_SHADE_MIN_BLOCKS 3
+#define RUMI_SHADE_MIN_BLOCKS 4
+#endif
+// The Whitted kernel at four blocks (64 registers): 0.29 ms of a 640x480, 9 spp, depth-10 frame's
+// shading against 0.39 ms without a limit (73 registers).
+#ifndef RUMI_SHADE_WHITTED_MIN_BLOCKS
+#define RUMI_SHADE_WHITTED_MIN_BLOCKS 4
 #endif
 // LEAN: the instantiation for scenes without a medium, textures, image-based lights or
 // subsurface materials (the host picks it only for those): the same code with the branches
@@ -818,7 +823,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
 // No medium event: the RayTracer sends rays through a volume unattenuated; only the
 // shadow ray of next-event estimation sees it (HomogeneousVolume::ShadowRayTr).  beta.w
 // carries the index of the material a refracted ray entered.
-__global__ void __launch_bounds__(SHADE_THREADS) pt_shade_whitted(PtLaunch P, int bounce) {
+__global__ void __launch_bounds__(SHADE_THREADS, RUMI_SHADE_WHITTED_MIN_BLOCKS) pt_shade_whitted(PtLaunch P, int bounce) {
     const int cur = bounce & 1, nxt = cur ^ 1;
     chain_shade(P, bounce);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1045,9 +1050,8 @@ static ShadowKernel shadow_kernel(int mode, int smem) {
 // backward, a batch of such scenes) takes the same instantiation, so their paths agree bit
 // for bit; the two instantiations differ in the compiler's FMA contraction, not in the
 // algorithm.  group: the general kernel groups the block's next rays by direction; without it
-// (frames of scheme 5, which gains nothing from the order) it has no block-wide barriers: 1.37
-// against 1.42 ms of shading in a 333x251, 25 spp, depth-9 frame of a medium around a glass
-// sphere.  The lean kernel is the other way round (0.40 against 0.38 ms, Cornell frame).
+// (frames of scheme 5, which gains nothing from the order) it has no block-wide barriers: 3% less
+// shading time in the frame of a medium around a glass sphere.  The lean kernel is the other way round (0.40 against 0.38 ms, Cornell frame).
 static void launch_shade(bool lean, bool group, cudaStream_t st, const PtLaunch &L, int b) {
     const auto k = lean ? pt_shade<false, true> : (group ? pt_shade<false> : pt_shade<false, false, false>);
     k<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
