@@ -186,6 +186,32 @@ RUMI_D int find_scene(const long long *prefix, int n, long long g) {
     return lo;
 }
 
+// warp_push to two queues by every thread of a block, with one addition to each counter per block:
+// additions to one address are done one after another, about one a nanosecond, so a warp's own
+// additions hold a large bounce up (shading of a 1024x1024, 64 spp, depth-10 frame of a million
+// triangles 22.3 ms with an addition per warp to the shadow queue, 21.4 with one per block; a
+// 333x251, 25 spp frame of a medium 1.36 and 1.32 ms with both queues).
+RUMI_D void block_push2(int *count_a, bool want_a, int &a, int *count_b, bool want_b, int &b) {
+#ifdef RUMI_HOST_BUILD
+    a = warp_push(count_a, want_a);
+    b = warp_push(count_b, want_b);
+#else
+    __shared__ int s_n[2], s_base[2];
+    if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    a = warp_push(&s_n[0], want_a);
+    b = warp_push(&s_n[1], want_b);
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int n = s_n[threadIdx.x];
+        s_base[threadIdx.x] = n > 0 ? atomicAdd(threadIdx.x ? count_b : count_a, n) : 0;
+    }
+    __syncthreads();
+    a += s_base[0];
+    b += s_base[1];
+#endif
+}
+
 // The chained kernels' bookkeeping, by one thread of the grid.
 RUMI_D bool first_thread() { return blockIdx.x == 0 && threadIdx.x == 0; }
 RUMI_D int *shadow_count(const PtLaunch &P) { return P.cnt + (P.sh_set ? C_SHADOW1 : C_SHADOW); }
@@ -737,14 +763,16 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
     // in queue order, so a warp then holds rays from a few neighbouring pixels' hit points
     // that head the same way (closest-hit 2% faster per frame on the 1M-triangle
     // workload).  A path's result does not depend on its queue position.
+    int kn = -1, ks = -1;
 #ifdef RUMI_HOST_BUILD
     // host build (one emulated thread per block): the block's group is its one ray
-    const int kn = want_next ? atomicAdd(&P.cnt[nxt], 1) : -1;
+    kn = want_next ? atomicAdd(&P.cnt[nxt], 1) : -1;
+    ks = want_sh ? atomicAdd(shadow_count(P), 1) : -1;
 #else
-    int kn = -1;
     if (GROUP) {
-        __shared__ int s_bins[32];
+        __shared__ int s_bins[32], s_shadow[2];
         if (threadIdx.x < 32) s_bins[threadIdx.x] = 0;
+        if (threadIdx.x == 32) s_shadow[0] = 0;
         __syncthreads();
         int dkey = 0, drank = 0;
         if (want_next) {
@@ -754,6 +782,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
             dkey = oct * 3 + dom;
             drank = atomicAdd(&s_bins[dkey], 1);
         }
+        ks = warp_push(&s_shadow[0], want_sh);
         __syncthreads();
         if (threadIdx.x < 32) {  // exclusive scan of the bins, then the block's range of the queue
             const int v = s_bins[threadIdx.x];
@@ -767,14 +796,16 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
             if (threadIdx.x == 0 && total > 0) base = atomicAdd(&P.cnt[nxt], total);
             base = __shfl_sync(0xffffffffu, base, 0);
             s_bins[threadIdx.x] = base + incl - v;
+        } else if (threadIdx.x == 32) {  // and of the shadow queue
+            s_shadow[1] = s_shadow[0] > 0 ? atomicAdd(shadow_count(P), s_shadow[0]) : 0;
         }
         __syncthreads();
         if (want_next) kn = s_bins[dkey] + drank;
+        ks += s_shadow[1];
     } else {
-        kn = warp_push(&P.cnt[nxt], want_next);
+        block_push2(&P.cnt[nxt], want_next, kn, shadow_count(P), want_sh, ks);
     }
 #endif
-    const int ks = warp_push(shadow_count(P), want_sh);
     if (want_next) {
         P.ray_o[nxt][kn] = make_float4(nx_o.x, nx_o.y, nx_o.z, pack_slot(slot, nx_flags));
         P.ray_d[nxt][kn] = make_float4(nx_d.x, nx_d.y, nx_d.z, FLT_MAX);
@@ -930,8 +961,8 @@ __global__ void __launch_bounds__(SHADE_THREADS, RUMI_SHADE_WHITTED_MIN_BLOCKS) 
             P.L[slot] = l;
         }
     }
-    const int kn = warp_push(&P.cnt[nxt], want_next);
-    const int ks = warp_push(shadow_count(P), want_sh);
+    int kn, ks;
+    block_push2(&P.cnt[nxt], want_next, kn, shadow_count(P), want_sh, ks);
     if (want_next) {
         P.ray_o[nxt][kn] = make_float4(nx_o.x, nx_o.y, nx_o.z, pack_slot(slot, nx_flags));
         P.ray_d[nxt][kn] = make_float4(nx_d.x, nx_d.y, nx_d.z, FLT_MAX);
@@ -1049,9 +1080,9 @@ static ShadowKernel shadow_kernel(int mode, int smem) {
 // forward pass of a scene (render, forward with or without kept radiance, the first pass of
 // backward, a batch of such scenes) takes the same instantiation, so their paths agree bit
 // for bit; the two instantiations differ in the compiler's FMA contraction, not in the
-// algorithm.  group: the general kernel groups the block's next rays by direction; without it
-// (frames of scheme 5, which gains nothing from the order) it has no block-wide barriers: 3% less
-// shading time in the frame of a medium around a glass sphere.  The lean kernel is the other way round (0.40 against 0.38 ms, Cornell frame).
+// algorithm.  group: the general kernel groups the block's next rays by direction; frames of
+// scheme 5 gain nothing from the order and go without it.  The lean kernel is the other way round
+// (0.40 against 0.38 ms, Cornell frame).
 static void launch_shade(bool lean, bool group, cudaStream_t st, const PtLaunch &L, int b) {
     const auto k = lean ? pt_shade<false, true> : (group ? pt_shade<false> : pt_shade<false, false, false>);
     k<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
