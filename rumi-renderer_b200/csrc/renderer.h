@@ -111,9 +111,11 @@ rumi_status bdpt_render(rumi_scene *sc, const rumi_render_params *p, float *film
 // next bounce's closest-hit launch (false: one stream, in order)
 // keep_L: when set, every wave's per-path radiance is copied there at global path index
 // pixel * spp + sample
+// sort: order every wave's rays between bounces, in the sort_bytes(pix_per_wave * spp) bytes after
+// the wave state
 rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *film_dev, rumi_render_stats *stats,
                          cudaStream_t stream, void *ws, long long pix_per_wave, bool overlap = false,
-                         float4 *keep_L = nullptr);
+                         float4 *keep_L = nullptr, bool sort = false);
 rumi_status trace_rays(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, float *t_dev, int32_t *prim_dev,
                        int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream);
 // The same for up to STAGED_RAYS rays in host memory: through the scene's page-locked staging
