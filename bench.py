@@ -100,6 +100,15 @@ def cpu_model():
 
 
 # --------------------------------------------------------------------- clocks
+ORDERED_PATHS = 1 << 22  # paths of a wave from which its rays are ordered between bounces
+
+
+def wave_launches(depth, ordered=False):
+    """Kernel launches of one wave: generation and resolve, closest hit, shading and any hit of
+    every bounce, and where the rays are ordered two more between bounces."""
+    return 2 + 3 * depth + (2 * (depth - 1) if ordered else 0)
+
+
 class ClockSampler:
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -454,7 +463,7 @@ def our_arm(args):
         rays_ext += st["rays_extend"]
         rays_sh += st["rays_shadow"]
         waves = st["extend_launches"] // w["max_depth"]
-        launches += waves * (3 + 5 * w["max_depth"])
+        launches += waves * wave_launches(w["max_depth"], ordered=st["paths"] // waves >= ORDERED_PATHS)
     ev1.record()
     barrier()
     clocks_info = clocks.stop()
@@ -638,13 +647,13 @@ def batched_arm(args):
     def plain(step):
         for g, s, sd, off in zip(gss, spp, seeds(step), offs):
             g.render(spp=s, seed=sd, film_device_ptr=films_plain.data_ptr() + 4 * off, stream=stream)
-        return len(gss) * (3 + 5 * depth)  # rumi_render: per bounce two resets, extend, shade, shadow
+        return len(gss) * wave_launches(depth)  # at least: the largest scenes' rays are ordered too
 
     def batched(step):
         _, st = batch.render(spp, seeds(step), depth, graph=True, films_device_ptr=films_batch.data_ptr(),
                              stream=stream)
         waves = st["extend_launches"] // depth
-        return waves * (3 + 5 * depth)
+        return waves * wave_launches(depth)
 
     def timed(fn):
         for s in range(args.warmup):
@@ -861,7 +870,7 @@ def adjoint_arm(args):
                                     float(abs(m_start[6] - m_tgt[6]))],
                 medium_error_end=[float(np.abs(m_end - m_tgt)[0:3].sum()), float(np.abs(m_end - m_tgt)[3:6].sum()),
                                   float(abs(m_end[6] - m_tgt[6]))],
-                gpu_launches=args.adam_steps * ((3 + 5 * depth) + 2 * (3 + 4 * depth)), clocks=clocks_info)
+                gpu_launches=args.adam_steps * (wave_launches(depth) + 2 * (1 + 3 * depth)), clocks=clocks_info)
     print(json.dumps(line), flush=True)
     g.close()
     return 0
@@ -953,7 +962,7 @@ def cornell_arm(args):
     launches = 0
     for s in range(steps):
         _, st = gs.render(seed=100 + s, film_device_ptr=film.data_ptr(), stream=stream)
-        launches += (st["extend_launches"] // depth) * (3 + 5 * depth)
+        launches += (st["extend_launches"] // depth) * wave_launches(depth)
     ev1.record()
     torch.cuda.synchronize()
     clocks_info = clocks.stop()

@@ -28,6 +28,7 @@
 // primitive m, which no other split of the tree shares), then pairs for splits that leave a side
 // empty.
 #include "bvh_build.h"
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 
@@ -1069,7 +1070,8 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
                                                  B.task_first_chunk, kc);
         }
         // the small tasks found so far (all of them, unless the expected levels did not suffice)
-        const int small_grid = 148 * 8;  // resident blocks; warps take tasks in turn
+        // resident blocks, fewer for few primitives; warps take tasks in turn
+        const int small_grid = std::min(148 * 8, cdiv((long long)n, 32 * SMALL_WARPS));
         small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(
             B.small, kc + K_SMALL, h[K_SMALL], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, B.mid, kc);
         small_build_kernel<SMALL_MID><<<2 * small_grid, 32 * SMALL_WARPS, 0, stream>>>(
