@@ -60,7 +60,7 @@ rumi_status rumi_test_texture_pattern(rumi_scene *scene, int64_t n, const int32_
 
 /* rumi_trace_rays (host arrays, n rays of 8 floats: o, in_object, d, tmax) through the
  * traversal scheme trace_mode selects (as rumi_render_params.trace_mode: 1-3 the binary
- * tree's walks, 5 the eight-wide tree's; 0 = the default), so every scheme's hits can be
+ * tree's walks, 4 the four-wide, 5 the eight-wide tree's; 0 = the default), so every scheme's hits can be
  * compared on the same rays.  t: n distances (0 = miss); prim: n canonical primitive ids
  * (-1 = miss; any-hit: 1 = occluded, 0 = not). */
 rumi_status rumi_test_trace_scheme(rumi_scene *scene, int64_t n, const float *rays, int32_t anyhit,

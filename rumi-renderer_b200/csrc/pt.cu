@@ -47,7 +47,8 @@ static constexpr int TRACE_THREADS = 128;
 #endif
 // The default walk (scheme 3, the speculative while-while walk over the four-wide tree) at 9
 // blocks: 56 registers (a 42-byte spill in closest-hit, none in any-hit); per 1024x1024x64 frame
-// 65.7 / 35.2 ms of closest-hit / any-hit against 66.7 / 36.4 at 8 and 69.9 / 35.2 at 10.
+// 65.7 / 35.2 ms of closest-hit / any-hit against 66.7 / 36.4 at 8 and 69.9 / 35.2 at 10 (before the
+// rays were ordered).
 #ifndef RUMI_WW_MIN_BLOCKS
 #define RUMI_WW_MIN_BLOCKS 9
 #endif
@@ -1170,7 +1171,8 @@ using ShadowKernel = void (*)(PtLaunch);
 // Shared-memory stack depth from rumi_render_params.stack_depth: 8, 16 or 32 entries per
 // thread (0 = 16).  Only the while-while walks (schemes 3 and 4) come in all three depths.
 // Measured on the 1024x1024x64 BVH-bound frame (four-wide walk, closest-hit / any-hit ms):
-// 8: 65.8 / 35.9, 16: 65.7 / 35.2, 32 with the L1 carveout sized to it: 65.5 / 35.2.
+// 8: 65.8 / 35.9, 16: 65.7 / 35.2, 32 with the L1 carveout sized to it: 65.5 / 35.2 (before
+// the rays were ordered).
 static inline int stack_entries(int stack_depth) { return stack_depth == 8 || stack_depth == 32 ? stack_depth : 16; }
 
 // Kernel selection and launches.  A host build of this file (RUMI_HOST_BUILD: the kernels
