@@ -14,9 +14,9 @@
 // cycle and SM: 80% busy with a 128-byte node in four loads, 66% with this one), then by the
 // half-rate pipe (59%).  Measured per 1024x1024x64 frame of the 1M-triangle workload, closest-hit
 // / any-hit: binary tree, scalar slabs 85.8 / 46.5 ms; binary, this slab form 78.5 / 42.1;
-// four-wide with 32-bit half extents (128 bytes) 71.6 / 38.7; this node 64.1 / 33.9 (52.3 / 29.0
-// with the rays of a large wave in order); a 64-byte // node with 8-bit planes 73.9 / 40.1 (the byte decoding costs more half-rate operations than the
-// saved load is worth).
+// four-wide with 32-bit half extents (128 bytes) 71.6 / 38.7; this node 64.1 / 33.9 (52.3 / 29.0 with
+// the rays of a large wave in order); a 64-byte node with 8-bit planes 73.9 / 40.1 (the byte decoding
+// costs more half-rate operations than the saved load is worth).
 // ref[k] >= 0: node index of child k, larger than the node's own; ref[k] < 0: its leaf, whose
 // records start at recs[~ref[k]].  An empty slot has negative half extents, which no ray with
 // finite origin enters, and refers to record 0, which nothing hits.  wide[0] is the root.
