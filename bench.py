@@ -202,6 +202,7 @@ class RefPool:
             a, b = ctx.Pipe()
             p = ctx.Process(target=_ref_worker, args=(b, w, pin), daemon=True)
             p.start()
+            b.close()  # the worker's end alone stays open: recv raises when the worker dies
             self.conns.append(a)
             self.procs.append(p)
         self.spp = None
@@ -230,6 +231,11 @@ class RefPool:
             c.send(None)
         for p in self.procs:
             p.join(timeout=30)
+
+
+def ref_available():
+    """Whether the reference has been built from its sources (oracle/build_ref.py)."""
+    return os.path.exists(os.path.join(ROOT, "oracle", "_ref", "librumi_ref.so"))
 
 
 def ref_procs(limit=None):
@@ -338,6 +344,10 @@ def gpu_rays_per_s(gs, rays, anyhit, repeats=3):
 def reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    if not ref_available():
+        print(json.dumps(dict(impl="reference", unavailable="the reference library is not built (oracle/build_ref.py "
+                                                             "needs the reference's sources)")), flush=True)
         return 0
     w = workload(args)
     procs = ref_procs()
@@ -996,6 +1006,8 @@ def main():
     args = parse()
     if args.impl == "reference":
         return reference_arm(args)
+    if not ref_available():
+        args.no_cpu_baseline = True
     if args.workload == "batched":
         return batched_arm(args)
     if args.workload == "adjoint":
