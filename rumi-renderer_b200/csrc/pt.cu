@@ -11,7 +11,8 @@
 //   generate  camera rays (Pinhole::CastViewRay, the reference's pixel sampler)
 //   extend    closest hit of every queued ray            (persistent, work-fetching)
 //   shade     medium free flight, emission, BSDF sample, NEE; compacts the next
-//             bounce's rays and this bounce's shadow rays with warp-aggregated atomics
+//             bounce's rays and this bounce's shadow rays with block-aggregated atomics
+//   sort      large waves: an order of the next rays by origin and direction
 //   shadow    any-hit test of the shadow rays; adds their contribution
 //   resolve   per-pixel sum of the samples in sample order (NaN samples dropped and
 //             counted, src/Scene/scene.cpp:229-241)
