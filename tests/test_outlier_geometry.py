@@ -1,0 +1,92 @@
+"""Scenes with a primitive far larger than the rest (a sky sphere, a ground plane) under the
+default walk: the rest costs what it costs alone.  On the CPU the walk built for the host over a
+tree packed by the library's packing, on the GPU the library's own tree."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _soup(n, seed=3):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    return (c + rng.uniform(-0.1, 0.1, (n, 3, 3))).astype(np.float32)
+
+
+def _rays(n, seed=5):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    r = np.zeros((n, 8), np.float32)
+    r[:, 0:3] = rng.uniform(-1.5, 1.5, (n, 3))
+    d = rng.normal(size=(n, 3))
+    r[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    r[:, 7] = 3.4e38
+    return r
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    gxx = shutil.which("g++")
+    inc = next((os.path.join(r, "include") for r in (os.environ.get("CUDA_HOME"), "/usr/local/cuda")
+                if r and os.path.isfile(os.path.join(r, "include", "cuda_runtime.h"))), None)
+    if not gxx or not inc:
+        pytest.skip("g++ or the CUDA headers are missing")
+    so = str(tmp_path_factory.mktemp("outlier") / "liboutlier.so")
+    subprocess.run([gxx, "-O1", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-w", "-I", inc, "-o", so,
+                    os.path.join(HERE, "host_build", "outlier_host.cpp")], check=True)
+    return C.CDLL(so)
+
+
+def _prims(tri, sph):
+    n = len(tri) + len(sph)
+    prims = np.zeros((n, 3, 4), np.float32)
+    ids = prims.view(np.int32)
+    nt = len(tri)
+    prims[:nt, 0, :3], prims[:nt, 1, :3], prims[:nt, 2, :3] = tri[:, 0], tri[:, 1] - tri[:, 0], tri[:, 2] - tri[:, 0]
+    prims[nt:, 0, :3], prims[nt:, 1, 0] = sph[:, :3], sph[:, 3]
+    ids[:, 0, 3] = np.arange(n)
+    ids[nt:, 1, 3] = 2
+    box = np.concatenate([np.concatenate([tri.min(1), tri.max(1)], 1),
+                          np.concatenate([sph[:, :3] - sph[:, 3:], sph[:, :3] + sph[:, 3:]], 1)]).astype(np.float32)
+    return prims, box
+
+
+def _f(a):
+    return a.ctypes.data_as(C.POINTER(C.c_float))
+
+
+# 600 triangles in a sphere that every ray may test: of radius 2, and of a far larger one (the same
+# random tree over the same order)
+@pytest.mark.parametrize("radius", [1e2, 1e4, 1e6, 1e9, 1e15])
+def test_a_far_sphere_leaves_the_other_boxes_tight(host, radius):
+    rays = _rays(2000)
+    counts = []
+    for r in (2.0, radius):
+        prims, box = _prims(_soup(600), np.array([[0, 0, 0, r]], np.float32))
+        counts.append(host.rumi_host_walk_tests(_f(prims), _f(box), len(prims), 11, _f(rays), len(rays)))
+    assert counts[1] < 1.5 * counts[0], counts
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("radius", [1e2, 1e4, 1e6])
+def test_gpu_a_far_sphere_leaves_the_other_boxes_tight(radius):
+    import rumi_b200
+    from rumi_b200 import scenes
+    from rumi_b200.scene import Film, Matte, Model, PathTracer, Scene, Sphere
+    rays = _rays(20000)
+    counts = []
+    for r in (2.0, radius):
+        sc = Scene()
+        sc.add(Model(_soup(20000) * np.float32(0.5)), Matte(1.0, scenes.WHITE))
+        sc.add(Sphere((0, 0, 0), r), Matte(0.5, scenes.WHITE))
+        sc.camera, sc.image, sc.tracer = scenes.cornell_camera(), Film(8, 8, 1), PathTracer(1)
+        gs = rumi_b200.GpuScene(sc)
+        try:
+            counts.append(gs.trace(rays)[3])
+        finally:
+            gs.close()
+    assert counts[1] < 1.5 * counts[0], counts
