@@ -89,13 +89,27 @@ RUMI_HD void wide_empty(WideNode &o, int k) {
     o.ref[k] = ~0;
 }
 
+// Centre and half extent of [lo, hi].  An interval that reaches past 2^47 becomes +-2^126 about 0, which
+// every ray is in: c |1/d| stays finite up to there (|1/d| <= 2^80, safe_rcp), and a centre that does
+// not would put both ends of the slab at the same infinity, where its finite end may be entered.
+RUMI_HD void wide_axis(float lo, float hi, float pad, float &c, float &h) {
+    if (fabsf(lo) > 1.40737488e14f || fabsf(hi) > 1.40737488e14f) {
+        c = 0.0f;
+        h = 8.50705917e37f;
+        return;
+    }
+    c = 0.5f * lo + 0.5f * hi;
+    h = wide_half(lo, hi, c, pad);
+}
+
 // scene_pad: wide_pad of the scene.
 RUMI_HD void wide_child(WideNode &o, int k, const BvhNode &c, float scene_pad, int ref) {
     const float pad = wide_box_pad(c, scene_pad);
-    o.cxy[k] = make_float2(0.5f * c.lo_x + 0.5f * c.hi_x, 0.5f * c.lo_y + 0.5f * c.hi_y);
-    o.cz[k] = 0.5f * c.lo_z + 0.5f * c.hi_z;
-    wide_set_half(o, k, wide_half(c.lo_x, c.hi_x, o.cxy[k].x, pad), wide_half(c.lo_y, c.hi_y, o.cxy[k].y, pad),
-                  wide_half(c.lo_z, c.hi_z, o.cz[k], pad));
+    float hx, hy, hz;
+    wide_axis(c.lo_x, c.hi_x, pad, o.cxy[k].x, hx);
+    wide_axis(c.lo_y, c.hi_y, pad, o.cxy[k].y, hy);
+    wide_axis(c.lo_z, c.hi_z, pad, o.cz[k], hz);
+    wide_set_half(o, k, hx, hy, hz);
     o.ref[k] = ref;
 }
 

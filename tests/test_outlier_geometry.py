@@ -71,6 +71,31 @@ def test_a_far_sphere_leaves_the_other_boxes_tight(host, radius):
     assert counts[1] < 1.5 * counts[0], counts
 
 
+# boxes that reach far or without end to one side: their rays are still found.  (A sphere of radius
+# 10^15 beside the rest, one of infinite radius, which nothing hits, and a triangle with a far vertex.)
+@pytest.mark.parametrize("sphere,vertex", [((5e15, 5e15, 5e15, 5e15), None), ((-5e15, 5e15, 0, 5e15), None),
+                                           ((1, 2, 3, np.inf), None), (None, (1e16, 1e16, 1e16)),
+                                           (None, (1e18, -1e18, 1e18)), (None, (-1e18, 0.3, -1e17))])
+def test_a_box_without_end_hides_nothing(host, sphere, vertex):
+    rays = _rays(3000)
+    rays[:1000, 4:7] = 0.0
+    rays[np.arange(1000), 4 + np.arange(1000) % 3] = np.where(np.arange(1000) % 2, 1.0, -1.0)  # along an axis
+    tri = _soup(600)
+    if vertex:
+        tri[17, 1] = vertex
+    prims, box = _prims(tri, np.array([sphere] if sphere else np.zeros((0, 4)), np.float32))
+    m = len(rays)
+    out = [(np.zeros(m, np.float32), np.zeros(m, np.int32), np.zeros((m, 2), np.float32)) for _ in range(2)]
+    ip = C.POINTER(C.c_int)
+    for seed in range(8):
+        host.rumi_host_walk(_f(prims), _f(box), len(prims), seed, _f(rays), m, 0, _f(out[0][0]),
+                            out[0][1].ctypes.data_as(ip), _f(out[0][2]), _f(out[1][0]), out[1][1].ctypes.data_as(ip),
+                            _f(out[1][2]))
+        assert (out[1][1] >= 0).mean() > 0.05
+        for a, b in zip(*out):
+            assert np.array_equal(a, b)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("radius", [1e2, 1e4, 1e6])
 def test_gpu_a_far_sphere_leaves_the_other_boxes_tight(radius):
@@ -90,3 +115,30 @@ def test_gpu_a_far_sphere_leaves_the_other_boxes_tight(radius):
         finally:
             gs.close()
     assert counts[1] < 1.5 * counts[0], counts
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sphere", [(5e15, 5e15, 5e15, 5e15), (1, 2, 3, np.inf)])
+def test_gpu_a_box_without_end_hides_nothing(sphere):
+    import rumi_b200
+    from rumi_b200 import _capi, scenes
+    from rumi_b200.scene import Film, Matte, Model, PathTracer, Scene, Sphere
+    sc = Scene()
+    sc.add(Model(_soup(3000)), Matte(1.0, scenes.WHITE))
+    sc.add(Sphere(sphere[:3], sphere[3]), Matte(0.5, scenes.WHITE))
+    sc.camera, sc.image, sc.tracer = scenes.cornell_camera(), Film(8, 8, 1), PathTracer(1)
+    rays = _rays(6000)
+    m = len(rays)
+    gs = rumi_b200.GpuScene(sc)
+    try:
+        got = []
+        for mode in (1, 4):  # the binary and the four-wide walk
+            t, prim = np.zeros(m, np.float32), np.zeros(m, np.int32)
+            _capi.check(_capi.load().rumi_test_trace_scheme(
+                gs.h, m, rays.ctypes.data_as(C.c_void_p), 0, mode, t.ctypes.data_as(C.c_void_p),
+                prim.ctypes.data_as(C.c_void_p)), "rumi_test_trace_scheme")
+            got.append((t, prim))
+        assert (got[0][1] >= 0).mean() > 0.2
+        assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    finally:
+        gs.close()
