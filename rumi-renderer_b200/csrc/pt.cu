@@ -265,11 +265,20 @@ enum { GROUP_NONE = 0, GROUP_BLOCK = 1, GROUP_FRAME = 2 };
 // as shading follows the same order, any hit of the bounces 2.84, 3.38, 2.84, 2.54 and 2.84, 3.00,
 // 2.29, 2.02 ms.  8^3 origin cells: 0.8 ms more per frame; 16^3 direction cells with 8^3 origins:
 // 0.2 ms more.
+// The low four bits of the origin cell come last, after the direction: with the whole cell first,
+// rays that start in one cell (a view of a small part of the scene, a scene inside a far larger
+// sphere) have 512 counters in 16 lines, and their additions wait for each other.  A 2048x2048, 4 spp,
+// depth-10 frame of 1034 triangles inside a sphere of 40 times their size takes 34.1 / 25.7 / 24.9 /
+// 24.2 ms with 0 / 3 / 4 / 5 such bits and 22.4 ms without the order; the frame above 104.7 / 104.5 /
+// 104.9 / 105.2 ms.
 #ifndef RUMI_SORT_O
 #define RUMI_SORT_O 4
 #endif
 #ifndef RUMI_SORT_D
 #define RUMI_SORT_D 3
+#endif
+#ifndef RUMI_SORT_LOW
+#define RUMI_SORT_LOW 4
 #endif
 static constexpr int SORT_BINS = 1 << (3 * (RUMI_SORT_O + RUMI_SORT_D));
 // Bits 0-3 of the cell of x in [0, 1] at every third bit; outside it the nearest cell, NaN the first.
@@ -285,7 +294,8 @@ RUMI_D int sort_bin(const DevScene &S, float3 o, float3 d) {
                    (sort_cell((o.z - a.z) / (b.y - a.z), RUMI_SORT_O) << 2);
     const int cd = sort_cell(0.5f * d.x + 0.5f, RUMI_SORT_D) | (sort_cell(0.5f * d.y + 0.5f, RUMI_SORT_D) << 1) |
                    (sort_cell(0.5f * d.z + 0.5f, RUMI_SORT_D) << 2);
-    return (co << (3 * RUMI_SORT_D)) | cd;
+    return ((co >> RUMI_SORT_LOW) << (3 * RUMI_SORT_D + RUMI_SORT_LOW)) | (cd << RUMI_SORT_LOW) |
+           (co & ((1 << RUMI_SORT_LOW) - 1));
 }
 
 // The chained kernels' bookkeeping, by one thread of the grid.
