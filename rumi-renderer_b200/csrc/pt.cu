@@ -79,6 +79,10 @@ static constexpr int STACK_SMEM = 32;
 #ifndef RUMI_SORT_NODES
 #define RUMI_SORT_NODES 64
 #endif
+// Rays of one bounce from which they are taken in order (in_order).
+#ifndef RUMI_SORT_RAYS
+#define RUMI_SORT_RAYS (1 << 21)
+#endif
 static constexpr int WALK_SMEM = 16;  // of the default walk (stack_entries)
 static_assert(TRACE_THREADS == WW_THREADS, "the walk's shared-memory columns are one per thread");
 static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? 4 : 3;
@@ -129,7 +133,7 @@ struct PtLaunch {
     // pt_finish do all that.
     int chained, sh_set;
     // ordered frames (GROUP_FRAME): sort_perm lists the bounce's rays in traversal order where
-    // `sorted` (the camera's rays are in order as they are)
+    // `sorted` (the camera's rays are in order as they are) and they are many (in_order)
     int sorted;
     int *sort_bins, *sort_base, *sort_perm;
     int2 *sort_key;
@@ -297,6 +301,11 @@ RUMI_D int sort_bin(const DevScene &S, float3 o, float3 d) {
     return ((co >> RUMI_SORT_LOW) << (3 * RUMI_SORT_D + RUMI_SORT_LOW)) | (cd << RUMI_SORT_LOW) |
            (co & ((1 << RUMI_SORT_LOW) - 1));
 }
+// Whether the n rays of a bounce are taken in that order: in a frame of which most paths leave the
+// scene the later bounces have too few for it, and the pass over all bins would cost more than their
+// walk (a 2048x2048, 4 spp, depth-10 frame of 1024 triangles in the open: 3.00 ms, 3.37 when every
+// bounce is ordered, 3.02 when none is).
+RUMI_D bool in_order(const PtLaunch &P, int n) { return P.sorted && n >= RUMI_SORT_RAYS; }
 
 // The chained kernels' bookkeeping, by one thread of the grid.
 RUMI_D bool first_thread() { return blockIdx.x == 0 && threadIdx.x == 0; }
@@ -394,10 +403,11 @@ __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, true)) p
     __shared__ int stack[SMEM * TRACE_THREADS];
     const int cur = bounce & 1;
     chain_extend(P, bounce);
+    const bool ordered = in_order(P, P.cnt[cur]);
     TraceStats st{0, 0};
     auto fetch = [&](int i, float3 &o, float3 &d, float &tmax, bool &in_obj) {
         float4 o4, d4;
-        load_ray(P.ray[cur], P.sorted ? P.sort_perm[i] : i, o4, d4);
+        load_ray(P.ray[cur], ordered ? P.sort_perm[i] : i, o4, d4);
         o = f4xyz(o4);
         d = f4xyz(d4);
         tmax = d4.w;
@@ -591,7 +601,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
 
     if (active) {
         float4 o4, d4;
-        const int q = GROUP == GROUP_FRAME && P.sorted ? P.sort_perm[i] : i;  // hits are in the order
+        const int q = GROUP == GROUP_FRAME && in_order(P, n) ? P.sort_perm[i] : i;  // hits are in the order
         load_ray(P.ray[cur], q, o4, d4);
         const float4 hv = P.hit[i];
         slot = slot_of(o4.w);
@@ -931,12 +941,14 @@ __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LE
 #ifndef RUMI_HOST_BUILD
 // Ordering a wave's next rays, after shading has counted them by bin and given each its rank there:
 // the queue range of every bin (bins in order within a block's 4096, blocks as they come), counters
-// back to zero; then each ray's queue position into its place of sort_perm.  The rays themselves stay:
+// back to zero; then each ray's queue position into its place of sort_perm.  Where the rays are too
+// few for the order, their bins' counters are cleared and nothing else is done.  The rays themselves stay:
 // moving their 48 bytes takes 16 ms of the frame above, against 2 here and 2 in the gathers of
 // closest hit and shading.
 static constexpr int SORT_THREADS = 1024;
 static_assert(SORT_BINS % (4 * SORT_THREADS) == 0, "one int4 of bins per thread");
-__global__ void __launch_bounds__(SORT_THREADS) pt_sort_bases(PtLaunch P) {
+__global__ void __launch_bounds__(SORT_THREADS) pt_sort_bases(PtLaunch P, int queue) {
+    if (!in_order(P, P.cnt[queue])) return;
     __shared__ int s_sum[32], s_base;
     const int i = blockIdx.x * SORT_THREADS + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int4 v = reinterpret_cast<int4 *>(P.sort_bins)[i];
@@ -965,11 +977,16 @@ __global__ void __launch_bounds__(SORT_THREADS) pt_sort_bases(PtLaunch P) {
 }
 
 __global__ void pt_sort_order(PtLaunch P, int queue) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) P.cnt[C_SORT] = 0;
-    if (i >= P.cnt[queue]) return;
-    const int2 key = P.sort_key[i];
-    P.sort_perm[P.sort_base[key.x] + key.y] = i;
+    const int n = P.cnt[queue], first = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool ordered = in_order(P, n);
+    if (first == 0) P.cnt[C_SORT] = 0;
+    for (int i = first; i < n; i += gridDim.x * blockDim.x) {
+        const int2 key = P.sort_key[i];
+        if (ordered)
+            P.sort_perm[P.sort_base[key.x] + key.y] = i;
+        else
+            P.sort_bins[key.x] = 0;
+    }
 }
 #endif
 
@@ -1412,8 +1429,9 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
     auto sort_next = [&](int b) {
         L.sorted = sort && b + 1 < bounces;
         if (!L.sorted) return;
-        pt_sort_bases<<<SORT_BINS / (4 * SORT_THREADS), SORT_THREADS, 0, stream>>>(L);
-        pt_sort_order<<<cdiv(L.n_paths, 256), 256, 0, stream>>>(L, (b & 1) ^ 1);
+        const int queue = (b & 1) ^ 1, blocks = cdiv(L.n_paths, 256), resident = sc->num_sms * 32;
+        pt_sort_bases<<<SORT_BINS / (4 * SORT_THREADS), SORT_THREADS, 0, stream>>>(L, queue);
+        pt_sort_order<<<blocks < resident ? blocks : resident, 256, 0, stream>>>(L, queue);
     };
     std::vector<cudaEvent_t> evs;
     auto mark_on = [&](cudaStream_t st_) {
