@@ -7,6 +7,7 @@ bounded together, and beyond the bound (or without a device) the array is an ord
 from __future__ import annotations
 
 import ctypes as C
+import os
 import threading
 import weakref
 
@@ -58,6 +59,14 @@ class _Pool:
 
 
 _pool = _Pool()
+
+
+def _after_fork():
+    """In a forked child: another thread of the parent may have held the lock."""
+    _pool.lock = threading.RLock()
+
+
+os.register_at_fork(after_in_child=_after_fork)
 
 
 def empty(shape, dtype) -> np.ndarray:
