@@ -162,7 +162,7 @@ class GpuScene:
             _capi.check(self.lib.rumi_render(self.h, C.byref(p), C.c_void_p(film_device_ptr), 1, C.byref(st)),
                         "rumi_render")
             return None, st.as_dict()
-        film = hostmem.empty((self.height, self.width, 3), np.float32)
+        film = hostmem.result((self.height, self.width, 3), np.float32)
         _capi.check(self.lib.rumi_render(self.h, C.byref(p), film.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_render")
         return film, st.as_dict()
@@ -192,7 +192,7 @@ class GpuScene:
             _capi.check(self.lib.rumi_forward(self.h, C.byref(p), C.c_void_p(film_device_ptr), 1, C.byref(st)),
                         "rumi_forward")
             return None, st.as_dict()
-        film = hostmem.empty((self.height, self.width, 3), np.float32)
+        film = hostmem.result((self.height, self.width, 3), np.float32)
         _capi.check(self.lib.rumi_forward(self.h, C.byref(p), film.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_forward")
         return film, st.as_dict()
@@ -323,7 +323,7 @@ class GpuBatch:
             _capi.check(self.lib.rumi_render_batch(self.h, C.byref(p), C.c_void_p(films_device_ptr), 1, C.byref(st)),
                         "rumi_render_batch")
             return None, st.as_dict()
-        flat = hostmem.empty((self.n_floats,), np.float32)
+        flat = hostmem.result((self.n_floats,), np.float32)
         _capi.check(self.lib.rumi_render_batch(self.h, C.byref(p), flat.ctypes.data_as(C.c_void_p), 0, C.byref(st)),
                     "rumi_render_batch")
         films, o = [], 0

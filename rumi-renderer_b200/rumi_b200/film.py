@@ -21,7 +21,7 @@ def tonemap(film, n_samples: int, gamma: float = 2.2, bytes_per_pixel: int = 3) 
     """(H, W, 3) B,G,R pixel sums -> (H, W, bytes_per_pixel) uint8 as Film::Save converts them."""
     f = np.ascontiguousarray(film, np.float32)
     H, W = f.shape[0], f.shape[1]
-    out = hostmem.empty((H, W, bytes_per_pixel), np.uint8)
+    out = hostmem.result((H, W, bytes_per_pixel), np.uint8)
     L = _capi.load()
     _capi.check(L.rumi_film_tonemap(f.ctypes.data_as(C.c_void_p), W, H, int(n_samples), float(gamma),
                                     bytes_per_pixel, out.ctypes.data_as(C.c_void_p), 0, None), "rumi_film_tonemap")
@@ -32,7 +32,7 @@ def fireflies(img) -> np.ndarray:
     """FirefliesFiltering on an (H, W, 3 or 4) uint8 image in the film's row order."""
     a = np.ascontiguousarray(img, np.uint8)
     H, W, bpp = a.shape
-    out = hostmem.empty(a.shape, np.uint8)
+    out = hostmem.result(a.shape, np.uint8)
     L = _capi.load()
     _capi.check(L.rumi_film_fireflies(a.ctypes.data_as(C.c_void_p), W, H, bpp, out.ctypes.data_as(C.c_void_p), 0,
                                       None), "rumi_film_fireflies")
