@@ -513,8 +513,10 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         cudaEventRecord(w1, s);
     };
     cudaEventRecord(e0, s);
+    const int *build_kc = nullptr;
+    int build_h[BVH_COUNTERS];
     int rc = bvh_build(d_tri_v, nT, sc->rects, d_rect_em, nR, sc->spheres, nS, sc->nodes, sc->leaf_prims, scratch, s,
-                       &sc->info, upload_shading);
+                       &sc->info, upload_shading, &build_kc);
     if (rc == 0 && side_st != RUMI_OK) {
         drop_events();
         return fail(side_st);
@@ -525,7 +527,12 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         set_error("bvh_build: internal limit reached");
         return fail(RUMI_ERR_INTERNAL);
     }
-    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, &sc->wide, &sc->n_wide, &sc->recs, &sc->n_recs, s);
+    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, build_kc, build_h, &sc->wide, &sc->n_wide, &sc->recs, &sc->n_recs, s);
+    if (rc <= 0 && build_kc && bvh_build_check(build_h, N, &sc->info) != 0) {
+        drop_events();
+        set_error("bvh_build: internal limit reached");
+        return fail(RUMI_ERR_INTERNAL);
+    }
     if (rc != 0) {
         drop_events();
         if (rc > 0) return fail(cuda_status((cudaError_t)rc, "four-wide BVH"));

@@ -68,6 +68,8 @@ static constexpr int IN_TMP = 1 << 20;
 
 // Device counters of a build.
 enum { K_LARGE = 0, K_LARGE1 = 1, K_SMALL = 2, K_CHUNKS = 3, K_ERR = 4, K_MID = 5, K_LEVELS = 6, K_SPARE = 7, K_NUM = 16 };
+static_assert(K_NUM == BVH_COUNTERS, "bvh_wide reads these");
+static_assert(BVH_DEFERRED <= SMALL_MAX, "no levels");
 
 // Appends a task to one of the small phase's lists (n + 1 entries; a task per primitive at most,
 // and empty sides of degenerate splits).
@@ -262,7 +264,7 @@ __device__ __forceinline__ void empty_bins(int *bins, int from, int step) {
 
 // Root node and root task (one block).
 __global__ void root_kernel(const int *root_bounds, int n, BvhNode *nodes, BuildTask *large, int *cb, BuildTask *small,
-                            int *bins, ChunkInfo *chunks, int *task_first_chunk, int *counters) {
+                            BuildTask *mid, int *bins, ChunkInfo *chunks, int *task_first_chunk, int *counters) {
     if (threadIdx.x == 0) {
         if (n == 0) {
             BvhNode &r = nodes[0];
@@ -284,6 +286,10 @@ __global__ void root_kernel(const int *root_bounds, int n, BvhNode *nodes, Build
             } else {
                 small[0] = t;
                 counters[K_SMALL] = 1;
+                if (n <= SMALL_MID) {  // the first pass would only hand it on, and is not launched
+                    mid[0] = t;
+                    counters[K_MID] = 1;
+                }
             }
         }
     }
@@ -1025,7 +1031,8 @@ size_t bvh_scratch_bytes(int n_prims) {
 // success, else a cudaError_t value (or -1 when the builder's internal bounds were hit).
 int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int *d_prim_flags, int n_rects,
               const float4 *d_spheres, int n_spheres, BvhNode *nodes, float4 *leaf_prims, void *scratch,
-              cudaStream_t stream, BvhBuildInfo *info, std::function<void()> meanwhile) {
+              cudaStream_t stream, BvhBuildInfo *info, std::function<void()> meanwhile, const int **pending) {
+    *pending = nullptr;
     const int N = n_tris + n_rects + n_spheres;
     const size_t n = (size_t)(N > 0 ? N : 1);
     BuildArrays B;
@@ -1037,7 +1044,7 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
     prim_prepare_kernel<<<grid_n, 256, 0, stream>>>(d_tri_v, n_tris, d_rects, n_rects, d_spheres, d_prim_flags,
                                                     n_spheres, B.aabb_lo, B.aabb_hi, B.prims_canon, B.idx[0],
                                                     B.root_bounds);
-    root_kernel<<<1, 1024, 0, stream>>>(B.root_bounds, N, nodes, B.tasks[0], B.cbs[0], B.small, B.bins[0], B.chunks,
+    root_kernel<<<1, 1024, 0, stream>>>(B.root_bounds, N, nodes, B.tasks[0], B.cbs[0], B.small, B.mid, B.bins[0], B.chunks,
                                         B.task_first_chunk, kc);
     // a level halves its tasks at best; a task has more than SMALL_MAX primitives, so a level holds
     // at most N / SMALL_MAX of them.  SAH splits are uneven: four levels more than halving takes,
@@ -1072,12 +1079,17 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
         // the small tasks found so far (all of them, unless the expected levels did not suffice)
         // resident blocks, fewer for few primitives; warps take tasks in turn
         const int small_grid = std::min(148 * 8, cdiv((long long)n, 32 * SMALL_WARPS));
-        small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(
-            B.small, kc + K_SMALL, h[K_SMALL], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, B.mid, kc);
+        if (N > SMALL_MID)
+            small_build_kernel<SMALL_MAX><<<small_grid, 32 * SMALL_WARPS, 0, stream>>>(
+                B.small, kc + K_SMALL, h[K_SMALL], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, B.mid, kc);
         small_build_kernel<SMALL_MID><<<2 * small_grid, 32 * SMALL_WARPS, 0, stream>>>(
             B.mid, kc + K_MID, h[K_MID], N, B.idx[0], B.idx[1], B.aabb_lo, B.aabb_hi, nodes, max_nodes, nullptr, kc);
         if (meanwhile) meanwhile();
         meanwhile = nullptr;
+        if (N <= BVH_DEFERRED) {
+            *pending = kc;
+            break;
+        }
         cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
         const cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return (int)e;
@@ -1086,11 +1098,16 @@ int bvh_build(const float *d_tri_v, int n_tris, const float4 *d_rects, const int
         until = level + 4;
     }
     gather_leaf_prims_kernel<<<grid_n, 256, 0, stream>>>(B.idx[0], N, B.prims_canon, leaf_prims);
+    return *pending ? 0 : bvh_build_check(h, N, info);
+}
+
+int bvh_build_check(const int *h, int n_prims, BvhBuildInfo *info) {
+    if (h[K_ERR]) return -1;
     if (info) {
         info->large_levels = h[K_LEVELS];
         info->small_tasks = h[K_SMALL];
-        info->node_capacity = max_nodes;
-        info->node_high_water = PAIRS + 2 * (int)n + 2 * h[K_SPARE];
+        info->node_capacity = bvh_node_capacity(n_prims);
+        info->node_high_water = PAIRS + 2 * (n_prims > 0 ? n_prims : 1) + 2 * h[K_SPARE];
     }
     return 0;
 }

@@ -5,12 +5,16 @@
 // while fewer than four, open the interior candidate of largest surface area (its two children
 // take its place).  One launch per level of the four-wide tree, a thread per frontier node: it
 // fills its node, allocates its interior children as one contiguous block after itself and
-// appends them to the next frontier, and appends its leaves to a list of records to write.  The
-// host does not wait between levels (a launch on an empty frontier costs about 2 us); it reads the
-// counts once, then allocates the two arrays to size and writes the leaf records, a warp per
-// leaf.
+// appends them to the next frontier, and appends its leaves to a list of records to write, a warp per
+// leaf.  The host does not wait between levels (a launch on an empty frontier costs about 2 us); it
+// reads the counts once, then allocates the two arrays to size and writes the leaf records.  A small
+// scene's tree is made by one block in one launch, in arrays for as many nodes and records as there
+// can be: of a scene of 11 primitives build and collapse are a chain of short launches and waits, 0.31 ms
+// of its creation with three launches, two copies and a wait for the levels, 0.25 with the one block
+// (0.26 without this tree).
 #include "renderer.h"
 #include "traverse.cuh"
+#include <algorithm>
 
 namespace rumi {
 
@@ -113,23 +117,23 @@ struct Candidates {
     }
 };
 
-// level: this launch's frontier is in[0 .. k[K_LEVELS + level]), the next one's count goes to
-// k[K_LEVELS + level + 1] (the counts start at zero, the first at one).  A level lasts as long as its
-// serial parts: the additions to the four counters, so a warp makes one of each, and the chain of
-// node loads, so candidates stay in registers with their boxes (a million triangles: build and
-// collapse 3.37 -> 3.16 ms).
-__global__ void collapse_level(const BvhNode *__restrict__ nodes2, int n_nodes2, const float4 *__restrict__ lp,
-                               int n_prims, const Frontier *__restrict__ in, Frontier *__restrict__ out, int level,
-                               WideNode *__restrict__ wide, LeafJob *__restrict__ jobs, int cap, int *__restrict__ kc) {
-    const int n_in = kc[K_LEVELS + level];
-    int *n_out = kc + K_LEVELS + level + 1;
+// Fills the four-wide nodes of the frontier in[0 .. n_in) (in == nullptr: the root alone) and appends
+// their interior children to out; thread `first` of `stride`.  A level lasts as long as its serial
+// parts: the additions to the four counters, so a warp makes one of each, and the chain of node loads,
+// so candidates stay in registers with their boxes (a million triangles: build and collapse
+// 3.37 -> 3.16 ms).  All counts start at zero: the nodes are counted without the root, the records
+// without the empty one.
+__device__ __forceinline__ void collapse_front(const BvhNode *__restrict__ nodes2, int n_nodes2,
+                                               const float4 *__restrict__ lp, int n_prims,
+                                               const Frontier *in, int n_in, Frontier *out, int *n_out, WideNode *wide,
+                                               LeafJob *jobs, int cap, int *kc, int first, int stride) {
     const BvhNode top = nodes2[0];
     const float amax = fmaxf(fmaxf(fmaxf(fabsf(top.lo_x), fabsf(top.hi_x)), fmaxf(fabsf(top.lo_y), fabsf(top.hi_y))),
                              fmaxf(fabsf(top.lo_z), fabsf(top.hi_z)));
     const float pad = wide_pad(amax);
     const int lane = threadIdx.x & 31;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i - lane < n_in; i += gridDim.x * blockDim.x) {
-        const Frontier f = i < n_in ? in[i] : Frontier{0, 0};
+    for (int i = first; i - lane < n_in; i += stride) {
+        const Frontier f = i < n_in && in ? in[i] : Frontier{0, 0};
         int err = f.b2 < 0 || f.b2 >= n_nodes2 || f.b4 < 0 || f.b4 >= cap ? 1 : 0;
         Candidates c;
         c.n = 0;
@@ -161,8 +165,8 @@ __global__ void collapse_level(const BvhNode *__restrict__ nodes2, int n_nodes2,
             }
         }
         if (err) n_int = n_leaf = n_rec = 0;
-        const int base = warp_add(kc + K_WIDE, n_int), pos = warp_add(n_out, n_int);
-        int at = warp_add(kc + K_RECS, n_rec), job = warp_add(kc + K_JOBS, n_leaf);
+        const int base = 1 + warp_add(kc + K_WIDE, n_int), pos = warp_add(n_out, n_int);
+        int at = 1 + warp_add(kc + K_RECS, n_rec), job = warp_add(kc + K_JOBS, n_leaf);
         // (the walk counts on children that come after their parent: it then ends)
         if (!err && n_int > 0 && (base + n_int > cap || base <= f.b4)) err = 3;
         if (!err && n_leaf > 0 && (at + n_rec > n_prims + 1 || job + n_leaf > n_prims)) err = 5;
@@ -188,17 +192,19 @@ __global__ void collapse_level(const BvhNode *__restrict__ nodes2, int n_nodes2,
     }
 }
 
-// A warp per leaf: its triangles two by two in order, then its other primitives.
-__global__ void records_kernel(const float4 *__restrict__ lp, const LeafJob *__restrict__ jobs, int n_jobs,
-                               LeafRec *__restrict__ recs) {
-    const int lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w == 0 && lane == 0) {  // record 0: nothing hits it
-        LeafRec z = {};
-        z.id[0] = REC_LAST;
-        recs[0] = z;
-    }
-    if (w >= n_jobs) return;
-    const LeafJob jb = jobs[w];
+// One level of a large tree: the frontier is in[0 .. kc[K_LEVELS + level]), the next one's count goes
+// to kc[K_LEVELS + level + 1].
+__global__ void collapse_level(const BvhNode *__restrict__ nodes2, int n_nodes2, const float4 *__restrict__ lp,
+                               int n_prims, const Frontier *__restrict__ in, Frontier *__restrict__ out, int level,
+                               WideNode *__restrict__ wide, LeafJob *__restrict__ jobs, int cap, int *__restrict__ kc) {
+    collapse_front(nodes2, n_nodes2, lp, n_prims, level > 0 ? in : nullptr, level > 0 ? kc[K_LEVELS + level] : 1, out,
+                   kc + K_LEVELS + level + 1, wide, jobs, cap, kc, blockIdx.x * blockDim.x + threadIdx.x,
+                   gridDim.x * blockDim.x);
+}
+
+// The records of one leaf, by a warp: its triangles two by two in order, then its other primitives.
+__device__ __forceinline__ void leaf_job(const float4 *__restrict__ lp, const LeafJob &jb, LeafRec *recs) {
+    const int lane = threadIdx.x & 31;
     auto is_tri = [&](int i) { return (__float_as_int(lp[3 * (size_t)(jb.first + i) + 1].w) & 0xff) == PRIM_TRI; };
     int n_tri = 0;
     for (int b = 0; b < jb.count; b += 32)
@@ -237,60 +243,113 @@ __global__ void records_kernel(const float4 *__restrict__ lp, const LeafJob *__r
     }
 }
 
+__device__ __forceinline__ void empty_record(LeafRec *recs) {  // record 0: nothing hits it
+    LeafRec z = {};
+    z.id[0] = REC_LAST;
+    recs[0] = z;
+}
+
+__global__ void records_kernel(const float4 *__restrict__ lp, const LeafJob *__restrict__ jobs, int n_jobs,
+                               LeafRec *__restrict__ recs) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w == 0 && (threadIdx.x & 31) == 0) empty_record(recs);
+    if (w < n_jobs) leaf_job(lp, jobs[w], recs);
+}
+
+// The whole tree of a small scene by one block, counters in shared memory; they and the build's go to
+// kc for the host.
+static constexpr int SMALL_THREADS = 512;
+__global__ void __launch_bounds__(SMALL_THREADS)
+    collapse_small(const BvhNode *__restrict__ nodes2, int n_nodes2, const float4 *__restrict__ lp, int n_prims,
+                   Frontier *fr0, Frontier *fr1, WideNode *wide, LeafJob *jobs, int cap, LeafRec *recs,
+                   const int *build_kc, int *kc) {
+    __shared__ int s_k[K_NUM];
+    for (int k = threadIdx.x; k < K_NUM; k += SMALL_THREADS) s_k[k] = 0;
+    __syncthreads();
+    for (int level = 0; level < 128; ++level) {
+        const int n_in = level > 0 ? s_k[K_LEVELS + level] : 1;
+        if (n_in == 0) break;
+        collapse_front(nodes2, n_nodes2, lp, n_prims, level == 0 ? nullptr : level & 1 ? fr1 : fr0, n_in,
+                       level & 1 ? fr0 : fr1, s_k + K_LEVELS + level + 1, wide, jobs, cap, s_k, threadIdx.x, SMALL_THREADS);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) empty_record(recs);
+    if (!s_k[K_ERR])  // (else the jobs may have gaps)
+        for (int w = threadIdx.x >> 5; w < s_k[K_JOBS]; w += SMALL_THREADS / 32) leaf_job(lp, jobs[w], recs);
+    for (int k = threadIdx.x; k < K_NUM; k += SMALL_THREADS) kc[k] = s_k[k];
+    if (threadIdx.x < BVH_COUNTERS) kc[K_NUM + threadIdx.x] = build_kc ? build_kc[threadIdx.x] : 0;
+}
+
 }  // namespace
 
-// Builds the four-wide tree of a finished binary tree; *wide_out and *recs_out are allocated to
-// size.  Returns 0, a cudaError_t value, or -1 when an index left its range.
-int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, WideNode **wide_out, int *n_wide,
-             LeafRec **recs_out, int *n_recs, cudaStream_t stream) {
+// Builds the four-wide tree of a finished binary tree; *wide_out and *recs_out are allocated.  Of a
+// small scene (BVH_DEFERRED) the build's counters, still on the device, are read with this tree's:
+// build_kc to build_h.  Returns 0, a cudaError_t value, or -1 when an index left its range.
+int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims, const int *build_kc, int *build_h,
+             WideNode **wide_out, int *n_wide, LeafRec **recs_out, int *n_recs, cudaStream_t stream) {
     // one four-wide node at most per leaf, one job per leaf: a node with an interior child has four
     // children, so nodes are outnumbered by leaves
     const size_t cap = n_prims > 1 ? (size_t)n_prims : 1;
+    const bool small = n_prims <= BVH_DEFERRED;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t b_wide = al(cap * sizeof(WideNode)), b_front = al(cap * sizeof(Frontier)), b_jobs = al(cap * sizeof(LeafJob));
+    const size_t b_wide = small ? 0 : al(cap * sizeof(WideNode)), b_front = al(cap * sizeof(Frontier)),
+                 b_jobs = al(cap * sizeof(LeafJob));
+    WideNode *w = nullptr;
+    LeafRec *r = nullptr;
     char *tmp = nullptr;
-    cudaError_t e = dalloc((void **)&tmp, b_wide + 2 * b_front + b_jobs + al(K_NUM * sizeof(int)), stream);
-    if (e != cudaSuccess) return (int)e;
-    WideNode *wide = (WideNode *)tmp;
+    cudaError_t e = dalloc((void **)&tmp, b_wide + 2 * b_front + b_jobs + al((K_NUM + BVH_COUNTERS) * sizeof(int)), stream);
+    if (small && e == cudaSuccess) e = dalloc((void **)&w, sizeof(WideNode) * cap, stream);
+    if (small && e == cudaSuccess) e = dalloc((void **)&r, sizeof(LeafRec) * (cap + 1), stream);
+    if (e != cudaSuccess) {
+        dfree(tmp, stream);
+        dfree(w, stream);
+        return (int)e;
+    }
+    WideNode *wide = small ? w : (WideNode *)tmp;
     Frontier *fr[2] = {(Frontier *)(tmp + b_wide), (Frontier *)(tmp + b_wide + b_front)};
     LeafJob *jobs = (LeafJob *)(tmp + b_wide + 2 * b_front);
     int *kc = (int *)(tmp + b_wide + 2 * b_front + b_jobs);
-    int h[K_NUM] = {};
-    h[K_WIDE] = 1;
-    h[K_RECS] = 1;  // record 0 is the one nothing hits
-    h[K_LEVELS] = 1;
-    const Frontier root{0, 0};
-    cudaMemcpyAsync(kc, h, sizeof(h), cudaMemcpyHostToDevice, stream);
-    cudaMemcpyAsync(fr[0], &root, sizeof(root), cudaMemcpyHostToDevice, stream);
-    // levels are launched a few at a time past the expected depth (four-wide: half of log2), up to
-    // the binary tree's deepest level
-    int level = 0, expect = 2;
-    for (size_t n = cap; n > 16; n >>= 2) ++expect;
-    expect += expect / 2;
-    for (;;) {
-        for (; level < expect && level < 128; ++level) {
-            size_t most = 1;  // of a frontier at this level
-            for (int k = 0; k < level && most < cap; ++k) most *= 4;
-            if (most > cap) most = cap;
-            const int grid = (int)((most + 63) / 64);
-            collapse_level<<<grid < 1184 ? grid : 1184, 64, 0, stream>>>(nodes2, n_nodes2, lp, n_prims, fr[level & 1],
-                                                                         fr[(level & 1) ^ 1], level, wide, jobs,
-                                                                         (int)cap, kc);
-        }
+    int h[K_NUM + BVH_COUNTERS] = {}, level = 0;
+    if (small) {
+        collapse_small<<<1, SMALL_THREADS, 0, stream>>>(nodes2, n_nodes2, lp, n_prims, fr[0], fr[1], wide, jobs, (int)cap,
+                                                        r, build_kc, kc);
         cudaMemcpyAsync(h, kc, sizeof(h), cudaMemcpyDeviceToHost, stream);
         e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess || h[K_ERR] || h[K_LEVELS + level] == 0 || level >= 128) break;
-        expect = level + 4;
+        level = 128;
+        if (build_h) std::copy(h + K_NUM, h + K_NUM + BVH_COUNTERS, build_h);
+    } else {
+        cudaMemsetAsync(kc, 0, K_NUM * sizeof(int), stream);
+        // levels are launched a few at a time past the expected depth (four-wide: half of log2), up to
+        // the binary tree's deepest level
+        int expect = 2;
+        for (size_t n = cap; n > 16; n >>= 2) ++expect;
+        expect += expect / 2;
+        for (;;) {
+            for (; level < expect && level < 128; ++level) {
+                size_t most = 1;  // of a frontier at this level
+                for (int k = 0; k < level && most < cap; ++k) most *= 4;
+                if (most > cap) most = cap;
+                const int grid = (int)((most + 63) / 64);
+                collapse_level<<<grid < 1184 ? grid : 1184, 64, 0, stream>>>(nodes2, n_nodes2, lp, n_prims, fr[level & 1],
+                                                                             fr[(level & 1) ^ 1], level, wide, jobs,
+                                                                             (int)cap, kc);
+            }
+            cudaMemcpyAsync(h, kc, K_NUM * sizeof(int), cudaMemcpyDeviceToHost, stream);
+            e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess || h[K_ERR] || h[K_LEVELS + level] == 0 || level >= 128) break;
+            expect = level + 4;
+        }
     }
-    WideNode *w = nullptr;
-    LeafRec *r = nullptr;
     const bool ok = e == cudaSuccess && !h[K_ERR] && h[K_LEVELS + level] == 0;
-    if (ok) e = dalloc((void **)&w, sizeof(WideNode) * (size_t)h[K_WIDE], stream);
-    if (ok && e == cudaSuccess) e = dalloc((void **)&r, sizeof(LeafRec) * (size_t)h[K_RECS], stream);
-    if (ok && e == cudaSuccess) {
-        cudaMemcpyAsync(w, wide, sizeof(WideNode) * (size_t)h[K_WIDE], cudaMemcpyDeviceToDevice, stream);
-        records_kernel<<<(h[K_JOBS] + 4) / 4, 128, 0, stream>>>(lp, jobs, h[K_JOBS], r);
-        e = cudaGetLastError();
+    const int nodes = h[K_WIDE] + 1, records = h[K_RECS] + 1;
+    if (ok && !small) {
+        e = dalloc((void **)&w, sizeof(WideNode) * (size_t)nodes, stream);
+        if (e == cudaSuccess) e = dalloc((void **)&r, sizeof(LeafRec) * (size_t)records, stream);
+        if (e == cudaSuccess) {
+            cudaMemcpyAsync(w, wide, sizeof(WideNode) * (size_t)nodes, cudaMemcpyDeviceToDevice, stream);
+            records_kernel<<<(h[K_JOBS] + 4) / 4, 128, 0, stream>>>(lp, jobs, h[K_JOBS], r);
+            e = cudaGetLastError();
+        }
     }
     dfree(tmp, stream);
     if (!ok || e != cudaSuccess) {
@@ -299,9 +358,9 @@ int bvh_wide(const BvhNode *nodes2, int n_nodes2, const float4 *lp, int n_prims,
         return e != cudaSuccess ? (int)e : -1;
     }
     *wide_out = w;
-    *n_wide = h[K_WIDE];
+    *n_wide = nodes;
     *recs_out = r;
-    *n_recs = h[K_RECS];
+    *n_recs = records;
     return 0;
 }
 
