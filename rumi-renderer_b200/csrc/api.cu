@@ -358,9 +358,10 @@ const char *rumi_last_error_string(void) { return g_last_error.c_str(); }
 
 const char *rumi_version(void) { return "rumi_b200 0.1 (sm_100a)"; }
 
-// Scene creation with the uploads in line / on a second stream: 36 primitives 0.30 / 0.41 ms, 4,106
-// triangles 0.82 / 1.0, 262,154 (the second stream's) 3.0 / 2.4.
-static constexpr int SIDE_UPLOAD_TRIANGLES = 16384;
+// Scene creation with the uploads in line / on a second stream, ms: 11 primitives 0.31 / 0.38, 4,106
+// triangles 0.85 / 1.00, 16,394 1.06 / 1.08, 32,778 1.17 / 1.21, 65,546 1.39 / 1.36, 131,082 1.85 / 1.67,
+// 262,154 2.82 / 2.28.
+static constexpr int SIDE_UPLOAD_TRIANGLES = 65536;
 
 rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     if (!out) return set_error("out is NULL"), RUMI_ERR_INVALID_ARG;
