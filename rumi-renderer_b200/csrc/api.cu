@@ -9,6 +9,7 @@
 #include <unistd.h>
 #include <mutex>
 #include "renderer.h"
+#include "optional_block.h"
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -83,22 +84,36 @@ static void workspace_release(rumi_scene *sc) {
     sc->ws_bytes = 0;
 }
 
+// The device's spare workspace, if it holds `bytes`.
+static bool workspace_from_cache(rumi_scene *sc, size_t bytes) {
+    if (sc->device < 0 || sc->device >= 64) return false;
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    if (!g_ws_cache[sc->device] || g_ws_cache_bytes[sc->device] < bytes) return false;
+    if (sc->ws) dfree(sc->ws, sc->stream);
+    sc->ws = g_ws_cache[sc->device];
+    sc->ws_bytes = g_ws_cache_bytes[sc->device];
+    g_ws_cache[sc->device] = nullptr;
+    g_ws_cache_bytes[sc->device] = 0;
+    return true;
+}
+
+bool try_workspace(rumi_scene *sc, size_t bytes) {
+    if (sc->ws_bytes >= bytes || workspace_from_cache(sc, bytes)) return true;
+    return grow_optional(
+        sc->ws, sc->ws_bytes, sc->order_refused, bytes,
+        [sc](size_t n) {
+            void *p = nullptr;
+            return dalloc(&p, n, sc->stream) == cudaSuccess ? p : nullptr;
+        },
+        [sc](void *p) { dfree(p, sc->stream); });
+}
+
 rumi_status ensure_workspace(rumi_scene *sc, size_t bytes) {
-    if (sc->ws_bytes >= bytes) return RUMI_OK;
+    if (sc->ws_bytes >= bytes || workspace_from_cache(sc, bytes)) return RUMI_OK;
     if (sc->ws) {
         dfree(sc->ws, sc->stream);
         sc->ws = nullptr;
         sc->ws_bytes = 0;
-    }
-    if (sc->device >= 0 && sc->device < 64) {
-        std::lock_guard<std::mutex> lock(g_ws_mutex);
-        if (g_ws_cache[sc->device] && g_ws_cache_bytes[sc->device] >= bytes) {
-            sc->ws = g_ws_cache[sc->device];
-            sc->ws_bytes = g_ws_cache_bytes[sc->device];
-            g_ws_cache[sc->device] = nullptr;
-            g_ws_cache_bytes[sc->device] = 0;
-            return RUMI_OK;
-        }
     }
     cudaError_t e = dalloc(&sc->ws, bytes, sc->stream);
     if (e != cudaSuccess) {

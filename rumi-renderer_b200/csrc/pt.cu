@@ -1372,7 +1372,7 @@ rumi_status pt_render(rumi_scene *sc, const rumi_render_params *p, float *film_d
     }
     const size_t bytes = pt_workspace_bytes(n_paths_max);
     // without memory for ordering the rays the frame goes without the order
-    const bool sort = sort_wave(sc, p, n_paths_max) && ensure_workspace(sc, bytes + sort_bytes(n_paths_max)) == RUMI_OK;
+    const bool sort = sort_wave(sc, p, n_paths_max) && try_workspace(sc, bytes + sort_bytes(n_paths_max));
     rumi_status st = ensure_workspace(sc, bytes);
     if (st != RUMI_OK) return st;
     if (uses_bvh8(p->trace_mode) && (st = ensure_bvh8(sc)) != RUMI_OK) return st;

@@ -60,6 +60,7 @@ struct rumi_scene {
     // render workspace, grown on demand
     void *ws = nullptr;
     size_t ws_bytes = 0;
+    size_t order_refused = 0;  // workspace with room for ordering the rays that could not be had
 };
 
 // A scene without a medium, textures, image-based lights or subsurface materials: its
@@ -126,6 +127,9 @@ rumi_status trace_rays_staged(rumi_scene *sc, int64_t n, const float *rays, int 
 rumi_status trace_rays_scheme(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, int trace_mode,
                               float *t_dev, int32_t *prim_dev, cudaStream_t stream);
 rumi_status ensure_workspace(rumi_scene *sc, size_t bytes);
+// The same for memory that a frame can do without: false, and the workspace as it was, when it cannot
+// be had (no error is recorded)
+bool try_workspace(rumi_scene *sc, size_t bytes);
 // builds the eight-wide tree on first use (trace_mode 5); a no-op once built
 rumi_status ensure_bvh8(rumi_scene *sc);
 // true when trace_mode selects the eight-wide walk
