@@ -707,7 +707,8 @@ rumi_status rumi_trace_rays(rumi_scene *sc, int64_t n, const float *rays, int32_
     if (!sc || n < 0 || (n > 0 && (!rays || !t || !prim))) return set_error("bad argument"), RUMI_ERR_INVALID_ARG;
     cudaStream_t s = stream ? (cudaStream_t)stream : sc->stream;
     if (on_device) return trace_rays(sc, n, rays, anyhit, t, prim, node_visits, prim_tests, s);
-    if (n > 0 && n <= STAGED_RAYS) return trace_rays_staged(sc, n, rays, anyhit, t, prim, node_visits, prim_tests, s);
+    if (n > 0 && n <= STAGED_RAYS && make_stage(sc))
+        return trace_rays_staged(sc, n, rays, anyhit, t, prim, node_visits, prim_tests, s);
     float *dr = nullptr, *dt = nullptr;
     int32_t *dp = nullptr;
     rumi_status st = RUMI_OK;

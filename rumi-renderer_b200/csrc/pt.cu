@@ -23,6 +23,7 @@
 #include "traverse.cuh"
 #include "shading.cuh"
 #include "camera.cuh"
+#include "optional_block.h"
 #include <map>
 #include <mutex>
 #include <utility>
@@ -1867,24 +1868,30 @@ rumi_status trace_rays(rumi_scene *sc, int64_t n, const float *rays_dev, int any
     return RUMI_OK;
 }
 
+static constexpr size_t STAGE_COUNTERS = 256 * 3;
+static_assert(3 * sizeof(unsigned long long) + sizeof(int) <= STAGE_COUNTERS, "counters of one chunk");
+
+bool make_stage(rumi_scene *sc) {
+    return grow_optional(
+        sc->stage, sc->stage_bytes, sc->stage_refused, (size_t)STAGED_RAYS * 40 + STAGE_COUNTERS,
+        [](size_t n) {
+            void *p = nullptr;
+            if (cudaHostAlloc(&p, n, cudaHostAllocPortable) == cudaSuccess) return p;
+            cudaGetLastError();
+            return (void *)nullptr;
+        },
+        [](void *p) { cudaFreeHost(p); });
+}
+
 // A small query is all latency: three allocations, three pageable copies and three waits around
 // a 10 us kernel.  Here the rays and zeroed counters go up in one page-locked copy and counters, t
 // and prim come back in one, through memory the scene keeps (61 rays: 72 us before).
 rumi_status trace_rays_staged(rumi_scene *sc, int64_t n, const float *rays, int anyhit, float *t, int32_t *prim,
                               int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream) {
-    constexpr size_t COUNTERS = 256 * 3;
-    static_assert(3 * sizeof(unsigned long long) + sizeof(int) <= COUNTERS, "counters of one chunk");
+    constexpr size_t COUNTERS = STAGE_COUNTERS;
     const size_t b_rays = sizeof(float) * 8 * (size_t)n, b_t = sizeof(float) * (size_t)n, total = b_rays + COUNTERS + 2 * b_t;
     rumi_status st = ensure_workspace(sc, total);
     if (st != RUMI_OK) return st;
-    if (!sc->stage) {
-        const cudaError_t e = cudaHostAlloc(&sc->stage, (size_t)STAGED_RAYS * 40 + COUNTERS, cudaHostAllocPortable);
-        if (e != cudaSuccess) {
-            sc->stage = nullptr;
-            cudaGetLastError();
-            return cuda_status(e, "page-locked allocation");
-        }
-    }
     char *dev = (char *)sc->ws, *host = (char *)sc->stage;
     memcpy(host, rays, b_rays);
     memset(host + b_rays, 0, COUNTERS);

@@ -57,6 +57,7 @@ struct rumi_scene {
     int num_sms = 148;
     // page-locked staging of small host ray queries (trace_rays_staged), made on first use
     void *stage = nullptr;
+    size_t stage_bytes = 0, stage_refused = 0;
     // render workspace, grown on demand
     void *ws = nullptr;
     size_t ws_bytes = 0;
@@ -120,8 +121,12 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
 rumi_status trace_rays(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, float *t_dev, int32_t *prim_dev,
                        int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream);
 // The same for up to STAGED_RAYS rays in host memory: through the scene's page-locked staging
-// buffer, one copy each way.
+// buffer (make_stage has to have made it), one copy each way.  Three copies through a scene's own
+// arrays / this way, us: 61 rays 90 / 56, 1000 104 / 70, 8192 145 / 100, 16384 175 / 130, 65536 412 / 381,
+// 262144 1128 / 1200.  The line is where the buffer is still small (0.3 MB per scene).
 static constexpr int64_t STAGED_RAYS = 8192;
+// false: the buffer cannot be had, and the query goes the way of larger ones
+bool make_stage(rumi_scene *sc);
 rumi_status trace_rays_staged(rumi_scene *sc, int64_t n, const float *rays, int anyhit, float *t, int32_t *prim,
                               int64_t *node_visits, int64_t *prim_tests, cudaStream_t stream);
 rumi_status trace_rays_scheme(rumi_scene *sc, int64_t n, const float *rays_dev, int anyhit, int trace_mode,

@@ -34,3 +34,10 @@ def test_a_refusal_leaves_the_block_and_is_remembered(block):
     assert block.block_grow(900) == 1 and block.block_bytes() == 900 and block.block_released() == 1
     assert block.block_grow(1100) == 0 and block.block_asked() == 4  # less than what was refused: asked for once
     assert block.block_grow(1100) == 0 and block.block_asked() == 4
+
+
+def test_memory_that_cannot_be_had_at_all(block):
+    """A query's staging: refused once, then the query goes the other way without asking again."""
+    block.block_reset(0)
+    assert [block.block_grow(328448) for _ in range(4)] == [0] * 4
+    assert block.block_asked() == 1 and block.block_bytes() == 0
