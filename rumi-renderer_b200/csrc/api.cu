@@ -97,13 +97,26 @@ static bool workspace_from_cache(rumi_scene *sc, size_t bytes) {
     return true;
 }
 
+// A workspace is allocated in the order of the scene's stream and used on the caller's, which knows
+// nothing of what the pool made that stream wait for (memory that another stream has yet to free):
+// it may be used once the scene's stream has passed the allocation.
+static cudaError_t workspace_alloc(rumi_scene *sc, void **p, size_t bytes) {
+    cudaError_t e = dalloc(p, bytes, sc->stream);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(sc->stream)) != cudaSuccess) {
+        dfree(*p, sc->stream);
+        *p = nullptr;
+    }
+    return e;
+}
+
 bool try_workspace(rumi_scene *sc, size_t bytes) {
     if (sc->ws_bytes >= bytes || workspace_from_cache(sc, bytes)) return true;
     return grow_optional(
         sc->ws, sc->ws_bytes, sc->order_refused, bytes,
         [sc](size_t n) {
             void *p = nullptr;
-            return dalloc(&p, n, sc->stream) == cudaSuccess ? p : nullptr;
+            return workspace_alloc(sc, &p, n) == cudaSuccess ? p : nullptr;
         },
         [sc](void *p) { dfree(p, sc->stream); });
 }
@@ -115,7 +128,7 @@ rumi_status ensure_workspace(rumi_scene *sc, size_t bytes) {
         sc->ws = nullptr;
         sc->ws_bytes = 0;
     }
-    cudaError_t e = dalloc(&sc->ws, bytes, sc->stream);
+    cudaError_t e = workspace_alloc(sc, &sc->ws, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return cuda_status(e, "workspace allocation");
