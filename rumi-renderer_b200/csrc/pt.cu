@@ -47,20 +47,22 @@ static constexpr int TRACE_THREADS = 128;
 #ifndef RUMI_SHADOW_MIN_BLOCKS
 #define RUMI_SHADOW_MIN_BLOCKS RUMI_TRACE_MIN_BLOCKS
 #endif
-// The default walk (scheme 3, the speculative while-while walk over the four-wide tree) at 9
+// The default walk (SCHEME_WIDE, the speculative while-while walk over the four-wide tree) at 9
 // blocks: 56 registers (a 42-byte spill in closest-hit, none in any-hit); per 1024x1024x64 frame
 // 65.7 / 35.2 ms of closest-hit / any-hit against 66.7 / 36.4 at 8 and 69.9 / 35.2 at 10 (before the
 // rays were ordered).
 #ifndef RUMI_WW_MIN_BLOCKS
 #define RUMI_WW_MIN_BLOCKS 9
 #endif
-// Testing a small scene's records in step (scheme 5): 64 registers without spills; 6 and 10 blocks
+// Testing a small scene's records in step (SCHEME_FEW): 64 registers without spills; 6 and 10 blocks
 // are 4% slower and equal on the Cornell frame.
 #ifndef RUMI_FEW_MIN_BLOCKS
 #define RUMI_FEW_MIN_BLOCKS 8
 #endif
 static constexpr int trace_min_blocks(int mode, bool extend) {
-    return mode == 5 ? RUMI_FEW_MIN_BLOCKS : mode == 3 ? RUMI_WW_MIN_BLOCKS : (extend ? RUMI_EXTEND_MIN_BLOCKS : RUMI_SHADOW_MIN_BLOCKS);
+    return mode == SCHEME_FEW    ? RUMI_FEW_MIN_BLOCKS
+           : mode == SCHEME_WIDE ? RUMI_WW_MIN_BLOCKS
+                                 : (extend ? RUMI_EXTEND_MIN_BLOCKS : RUMI_SHADOW_MIN_BLOCKS);
 }
 // 1: each bounce's any-hit launch runs on an auxiliary stream beside the next bounce's
 // closest-hit launch (pt_render_in); 0: one stream, launches in order.
@@ -86,7 +88,7 @@ static constexpr int STACK_SMEM = 32;
 #endif
 static constexpr int WALK_SMEM = 16;  // of the default walk (stack_entries)
 static_assert(TRACE_THREADS == WW_THREADS, "the walk's shared-memory columns are one per thread");
-static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? 4 : 3;
+static constexpr int DEFAULT_WALK_MODE = RUMI_WALK8 ? SCHEME_EIGHT : SCHEME_WIDE;
 // Threads per block of the shading kernels; a block groups its next rays by direction, so
 // the block size is also the grouping's width (128: shading 0.5 ms faster per frame,
 // closest-hit 0.5 ms slower).
@@ -260,7 +262,7 @@ RUMI_D void block_push2(int *count_a, bool want_a, int &a, int *count_b, bool wa
 
 // How shading leaves a block's next rays in the queue: as they come, grouped by direction within the
 // block, or as they come with a bin and a rank in it for ordering the whole wave (pt_sort_order).
-enum { GROUP_NONE = 0, GROUP_BLOCK = 1, GROUP_FRAME = 2 };
+enum Group { GROUP_NONE, GROUP_BLOCK, GROUP_FRAME };
 
 // The order of a large wave's rays: bins of origin cell (16^3 over the scene's bounds) times
 // direction cell (8^3 over [-1, 1]^3), both along a Morton curve.  Rays of one bin walk the same
@@ -574,7 +576,7 @@ RUMI_D bool nee_setup(const LightSample &ls, float3 p, float3 &wi, float &dist, 
 #ifndef RUMI_SHADE_LEAN_MIN_BLOCKS
 #define RUMI_SHADE_LEAN_MIN_BLOCKS 4
 #endif
-template <bool ADJ, bool LEAN = false, int GROUP = GROUP_BLOCK>
+template <bool ADJ, bool LEAN = false, Group GROUP = GROUP_BLOCK>
 __global__ void __launch_bounds__(SHADE_THREADS, ADJ ? 1 : (LEAN ? RUMI_SHADE_LEAN_MIN_BLOCKS : RUMI_SHADE_MIN_BLOCKS))
     pt_shade(PtLaunch P, int bounce) {
     const int cur = bounce & 1, nxt = cur ^ 1;
@@ -1176,29 +1178,29 @@ static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Traversal scheme index (traverse_queue MODE) from rumi_render_params.trace_mode:
 // 1..5 select modes 0..4, 0 selects the default, the speculative while-while walk over the
-// four-wide tree (mode 3), the fastest on the BVH-bound workload.
+// four-wide tree, the fastest on the BVH-bound workload.
 static inline int trace_scheme(int trace_mode) {
     return trace_mode >= 1 && trace_mode <= 5 ? trace_mode - 1 : DEFAULT_WALK_MODE;
 }
 // The scheme of a scene's frames: the default walk gives way to testing the records in step
-// (mode 5) where the four-wide tree is a single node of few records, unless the call asks for a
+// (SCHEME_FEW) where the four-wide tree is a single node of few records, unless the call asks for a
 // scheme or for traversal counts.  Closest-hit / any-hit ms of a 512x512, 16 spp, depth-6 frame,
-// walk against mode 5: 10 triangles and a light (7 records) 0.71 / 0.55 and 0.68 / 0.54; 12
+// walk against that: 10 triangles and a light (7 records) 0.71 / 0.55 and 0.68 / 0.54; 12
 // triangles, a light and a sphere (9) 0.96 / 0.61 and 0.93 / 0.65; and of the 256x256, 16 spp,
 // depth-8 Cornell frame (9 records) 0.31 / 0.23 and 0.27 / 0.22.
 static inline int scene_scheme(const rumi_scene *sc, const rumi_render_params *p) {
     const bool few = sc->n_wide == 1 && sc->n_recs <= RUMI_FEW_RECORDS;
-    return few && DEFAULT_WALK_MODE == 3 && p->trace_mode == 0 && !(p->flags & RUMI_FLAG_STATS)
-               ? 5
+    return few && DEFAULT_WALK_MODE == SCHEME_WIDE && p->trace_mode == 0 && !(p->flags & RUMI_FLAG_STATS)
+               ? SCHEME_FEW
                : trace_scheme(p->trace_mode);
 }
-bool uses_bvh8(int trace_mode) { return trace_scheme(trace_mode) == 4; }
+bool uses_bvh8(int trace_mode) { return trace_scheme(trace_mode) == SCHEME_EIGHT; }
 
 using ExtendKernel = void (*)(PtLaunch, int);
 using ShadowKernel = void (*)(PtLaunch);
 
 // Shared-memory stack depth from rumi_render_params.stack_depth: 8, 16 or 32 entries per
-// thread (0 = 16).  Only the while-while walks (schemes 3 and 4) come in all three depths.
+// thread (0 = 16).  Only the while-while walks (SCHEME_WIDE, SCHEME_EIGHT) come in all three depths.
 // Measured on the 1024x1024x64 BVH-bound frame (four-wide walk, closest-hit / any-hit ms):
 // 8: 65.8 / 35.9, 16: 65.7 / 35.2, 32 with the L1 carveout sized to it: 65.5 / 35.2 (before
 // the rays were ordered).
@@ -1210,39 +1212,57 @@ static inline int stack_entries(int stack_depth) { return stack_depth == 8 || st
 template <bool STATS>
 static ExtendKernel extend_kernel(int mode, int smem) {
     switch (mode) {
-        case 0: return pt_extend<0, STATS>;
-        case 1: return pt_extend<1, STATS>;
-        case 2: return pt_extend<2, STATS>;
-        case 5: return pt_extend<5, STATS, 1>;
-        case 3: return smem == 8 ? pt_extend<3, STATS, 8> : smem == 16 ? pt_extend<3, STATS, 16> : pt_extend<3, STATS>;
-        default: return smem == 8 ? pt_extend<4, STATS, 8> : smem == 16 ? pt_extend<4, STATS, 16> : pt_extend<4, STATS>;
+        case SCHEME_BATCH: return pt_extend<SCHEME_BATCH, STATS>;
+        case SCHEME_REFILL: return pt_extend<SCHEME_REFILL, STATS>;
+        case SCHEME_LEAVES: return pt_extend<SCHEME_LEAVES, STATS>;
+        case SCHEME_FEW: return pt_extend<SCHEME_FEW, STATS, 1>;
+        case SCHEME_WIDE:
+            return smem == 8    ? pt_extend<SCHEME_WIDE, STATS, 8>
+                   : smem == 16 ? pt_extend<SCHEME_WIDE, STATS, 16>
+                                : pt_extend<SCHEME_WIDE, STATS>;
+        default:
+            return smem == 8    ? pt_extend<SCHEME_EIGHT, STATS, 8>
+                   : smem == 16 ? pt_extend<SCHEME_EIGHT, STATS, 16>
+                                : pt_extend<SCHEME_EIGHT, STATS>;
     }
 }
 
 template <bool ADJ>
 static ShadowKernel shadow_kernel(int mode, int smem) {
     switch (mode) {
-        case 0: return pt_shadow<0, ADJ>;
-        case 1: return pt_shadow<1, ADJ>;
-        case 2: return pt_shadow<2, ADJ>;
-        case 5: return pt_shadow<5, ADJ, 1>;
-        case 3: return smem == 8 ? pt_shadow<3, ADJ, 8> : smem == 16 ? pt_shadow<3, ADJ, 16> : pt_shadow<3, ADJ>;
-        default: return smem == 8 ? pt_shadow<4, ADJ, 8> : smem == 16 ? pt_shadow<4, ADJ, 16> : pt_shadow<4, ADJ>;
+        case SCHEME_BATCH: return pt_shadow<SCHEME_BATCH, ADJ>;
+        case SCHEME_REFILL: return pt_shadow<SCHEME_REFILL, ADJ>;
+        case SCHEME_LEAVES: return pt_shadow<SCHEME_LEAVES, ADJ>;
+        case SCHEME_FEW: return pt_shadow<SCHEME_FEW, ADJ, 1>;
+        case SCHEME_WIDE:
+            return smem == 8    ? pt_shadow<SCHEME_WIDE, ADJ, 8>
+                   : smem == 16 ? pt_shadow<SCHEME_WIDE, ADJ, 16>
+                                : pt_shadow<SCHEME_WIDE, ADJ>;
+        default:
+            return smem == 8    ? pt_shadow<SCHEME_EIGHT, ADJ, 8>
+                   : smem == 16 ? pt_shadow<SCHEME_EIGHT, ADJ, 16>
+                                : pt_shadow<SCHEME_EIGHT, ADJ>;
     }
 }
 
+// How a bounce's shading leaves the next rays.  order: the wave's rays are ordered.  The general kernel
+// gains nothing from grouping where the records are tested in step and goes without it; the lean one is
+// the other way round (0.40 against 0.38 ms, Cornell frame).
+static Group shade_group(bool lean, int mode, bool order) {
+    return order ? GROUP_FRAME : lean || mode != SCHEME_FEW ? GROUP_BLOCK : GROUP_NONE;
+}
+
 // Forward shading of one bounce.  lean: the instantiation without the medium, texture,
-// image-based-light and subsurface branches, for scenes that have none of them.  Every
-// forward pass of a scene (render, forward with or without kept radiance, the first pass of
-// backward, a batch of such scenes) takes the same instantiation, so their paths agree bit
-// for bit; the two instantiations differ in the compiler's FMA contraction, not in the
-// algorithm.  group: GROUP_*.  The general kernel groups the block's next rays by direction; frames
-// of scheme 5 gain nothing from the order and go without it.  The lean kernel is the other way round
-// (0.40 against 0.38 ms, Cornell frame).
-static void launch_shade(bool lean, int group, cudaStream_t st, const PtLaunch &L, int b) {
-    const auto k = lean ? (group == GROUP_FRAME ? pt_shade<false, true, GROUP_FRAME> : pt_shade<false, true>)
+// image-based-light and subsurface branches, for scenes that have none of them; it and the general
+// one differ in the compiler's FMA contraction, not in the algorithm, so every forward pass of a scene
+// (render, forward with or without kept radiance, the first pass of backward, a batch that is lean as
+// the scene is) takes the same of the two.  Their instantiations by group share the text of a path's
+// arithmetic but are compiled one by one: that frames of one scene are the same bits with either is
+// tested (over textures, image-based light, subsurface and media), not guaranteed by construction.
+static void launch_shade(bool lean, Group group, cudaStream_t st, const PtLaunch &L, int b) {
+    const auto k = lean ? (group == GROUP_FRAME ? pt_shade<false, true, GROUP_FRAME> : pt_shade<false, true, GROUP_BLOCK>)
                         : (group == GROUP_FRAME   ? pt_shade<false, false, GROUP_FRAME>
-                           : group == GROUP_BLOCK ? pt_shade<false>
+                           : group == GROUP_BLOCK ? pt_shade<false, false, GROUP_BLOCK>
                                                   : pt_shade<false, false, GROUP_NONE>);
     k<<<cdiv(L.n_paths, SHADE_THREADS), SHADE_THREADS, 0, st>>>(L, b);
 }
@@ -1355,7 +1375,7 @@ static size_t sort_bytes(long long paths) {
 // 3.05 / 2.96, 5.22 / 5.31, 9.66 / 10.2, 18.1 / 19.5 ms.  Of 266 triangles (under the line of
 // nodes) 4.47 / 4.44 at 4 million and 15.8 / 16.4 at 17; of 26 triangles 13.2 / 12.9 at 17.
 static bool sort_wave(const rumi_scene *sc, const rumi_render_params *p, long long paths) {
-    return p->integrator == RUMI_PATH_TRACER && scene_scheme(sc, p) == 3 && paths >= RUMI_SORT_PATHS &&
+    return p->integrator == RUMI_PATH_TRACER && scene_scheme(sc, p) == SCHEME_WIDE && paths >= RUMI_SORT_PATHS &&
            sc->n_wide >= RUMI_SORT_NODES;
 }
 
@@ -1417,7 +1437,7 @@ rumi_status pt_render_in(rumi_scene *sc, const rumi_render_params *p, float *fil
     int grid = 0, shadow_grid = 0;
     trace_grids(mode, smem, sc->num_sms, p->blocks_per_sm, false, count_stats, (long long)Wp, grid, shadow_grid);
     const bool lean = shade_lean(sc);
-    const int group = sort ? GROUP_FRAME : (lean || mode != 5 ? GROUP_BLOCK : GROUP_NONE);
+    const Group group = shade_group(lean, mode, sort);
     if (sort) {
         char *w = (char *)ws + pt_workspace_bytes((long long)Wp);
         L.sort_bins = (int *)w; w += SORT_BINS * sizeof(int);
@@ -1626,6 +1646,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
     // the same traversal scheme as rumi_render, so both passes and the forward frame
     // resolve exact-distance ties alike
     const int mode = scene_scheme(sc, p);
+    const bool lean = shade_lean(sc);
     const int smem = stack_entries(p->stack_depth);
     A.refill_min = B.refill_min = p->refill_min > 0 ? p->refill_min : 8;
     int grid = 0, grid_sh = 0, grid_dummy = 0, grid_sh_adj = 0;
@@ -1658,7 +1679,7 @@ rumi_status pt_backward(rumi_scene *sc, const rumi_render_params *p, const float
                 if (adj)
                     pt_shade<true><<<cdiv(X.n_paths, SHADE_THREADS), SHADE_THREADS, 0, stream>>>(X, b);
                 else
-                    launch_shade(shade_lean(sc), shade_lean(sc) || mode != 5, stream, X, b);
+                    launch_shade(lean, shade_group(lean, mode, false), stream, X, b);
                 const bool aside = overlap && b + 1 < p->max_depth;
                 cudaStream_t ss = aside ? sc->aux_stream : stream;
                 if (aside) {
@@ -1756,7 +1777,7 @@ rumi_status pt_enqueue_batch(const BatchFrame &F, void *ws, float *films, cudaSt
             L.sh_set = b & 1;
             pt_trace_multi<false><<<grid, TRACE_THREADS, 0, stream>>>(L, b);
             if (b > 0 && aux) cudaStreamWaitEvent(stream, ev_join, 0);
-            launch_shade(F.lean, true, stream, L, b);
+            launch_shade(F.lean, shade_group(F.lean, DEFAULT_WALK_MODE, false), stream, L, b);
             const bool aside = aux && b + 1 < F.max_depth;
             if (aside) {
                 cudaEventRecord(ev_fork, stream);
@@ -1795,7 +1816,7 @@ struct TraceLaunch {
 template <int MODE, bool ANYHIT, bool STATS>
 __global__ void __launch_bounds__(TRACE_THREADS, trace_min_blocks(MODE, !ANYHIT))
     trace_batch_kernel(TraceLaunch T, long long first, int n, int *fetch_counter) {
-    constexpr int SMEM = MODE == 3 ? WALK_SMEM : STACK_SMEM;
+    constexpr int SMEM = MODE == SCHEME_WIDE ? WALK_SMEM : STACK_SMEM;
     __shared__ int stack[SMEM * TRACE_THREADS];
     TraceStats st{0, 0};
     auto fetch = [&](int i, float3 &o, float3 &d, float &tmax, bool &in_obj) {
@@ -1954,11 +1975,11 @@ rumi_status trace_rays_scheme(rumi_scene *sc, int64_t n, const float *rays_dev, 
                 launch_trace_batch<false, false, M>(T, sc->num_sms, stream);
         };
         switch (m) {
-            case 0: go(std::integral_constant<int, 0>()); break;
-            case 1: go(std::integral_constant<int, 1>()); break;
-            case 2: go(std::integral_constant<int, 2>()); break;
-            case 3: go(std::integral_constant<int, 3>()); break;
-            default: go(std::integral_constant<int, 4>()); break;
+            case SCHEME_BATCH: go(std::integral_constant<int, SCHEME_BATCH>()); break;
+            case SCHEME_REFILL: go(std::integral_constant<int, SCHEME_REFILL>()); break;
+            case SCHEME_LEAVES: go(std::integral_constant<int, SCHEME_LEAVES>()); break;
+            case SCHEME_WIDE: go(std::integral_constant<int, SCHEME_WIDE>()); break;
+            default: go(std::integral_constant<int, SCHEME_EIGHT>()); break;
         }
     }
     cudaError_t e = cudaGetLastError();

@@ -1213,16 +1213,22 @@ RUMI_D void traverse_queue_walk(SceneOf scene_of, int n, int *counter, int refil
 #endif
 }
 
-// Persistent queue traversal shared by every ray kernel.
-//   MODE 0: a warp takes 32 rays and traces each to completion.
-//   MODE 1: per-lane refill; every iteration advances each ray by one node pair.
-//   MODE 2: per-lane refill; interior node pairs until every busy lane holds postponed
-//           leaves, then the warp intersects those leaves together.
-//   MODE 3: speculative while-while over the four-wide tree (traverse_queue_ww).
-//   MODE 4: the same scheme over the compressed eight-wide tree (traverse_queue_ww8).
-//   MODE 5: a warp takes 32 rays and tests the records of a single-node four-wide tree in step
-//           (few_isect).
-// smem_block: the block's STACK_SMEM * WW_THREADS ints.  fetch(i, o, d, tmax, in_obj) loads ray i; finish(i, hit) consumes its result.
+// Schemes of the persistent queue traversal (the MODE of a kernel).  rumi_render_params.trace_mode 1 to 5
+// asks for the first five in this order; SCHEME_FEW is the renderer's own choice (scene_scheme).
+enum TraceScheme {
+    SCHEME_BATCH = 0,   // a warp takes 32 rays and traces each to completion (binary tree)
+    SCHEME_REFILL = 1,  // per-lane refill; every iteration advances each ray by one node pair
+    SCHEME_LEAVES = 2,  // per-lane refill; interior node pairs until every busy lane holds postponed
+                        // leaves, then the warp intersects those leaves together
+    SCHEME_WIDE = 3,    // speculative while-while over the four-wide tree (traverse_queue_ww)
+    SCHEME_EIGHT = 4,   // the same over the compressed eight-wide tree (traverse_queue_ww8)
+    SCHEME_FEW = 5,     // a warp takes 32 rays and tests the records of a single-node four-wide tree
+                        // in step (few_isect)
+};
+
+// Persistent queue traversal shared by every ray kernel.  smem_block: the block's
+// STACK_SMEM * WW_THREADS ints.  fetch(i, o, d, tmax, in_obj) loads ray i; finish(i, hit) consumes its
+// result.
 template <int MODE, bool ANYHIT, int STACK_SMEM, bool STATS, typename Fetch, typename Finish>
 RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_min, int *smem_block, Fetch fetch,
                            Finish finish, TraceStats &st) {
@@ -1245,12 +1251,12 @@ RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_mi
 #endif
     const int lane = threadIdx.x & 31;
     int spill[RUMI_MAX_BVH_DEPTH - STACK_SMEM > 0 ? RUMI_MAX_BVH_DEPTH - STACK_SMEM : 1];
-    if (MODE == 3) {
+    if (MODE == SCHEME_WIDE) {
         traverse_queue_ww<ANYHIT, STACK_SMEM, STATS, false>([&](int) { return &s; }, n, counter, refill_min, smem_block,
                                                             fetch, finish, st);
         return;
     }
-    if (MODE == 5) {
+    if (MODE == SCHEME_FEW) {
         for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n; base += gridDim.x * blockDim.x) {
             const int i = base + lane;
             float3 o = mk3(0, 0, 0), d = mk3(0, 0, 0);
@@ -1262,12 +1268,12 @@ RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_mi
         }
         return;
     }
-    if (MODE == 4) {
+    if (MODE == SCHEME_EIGHT) {
         traverse_queue_ww8<ANYHIT, STACK_SMEM, STATS>([&](int) { return &s; }, n, counter, refill_min, smem_stack,
                                                       stride, fetch, finish, st);
         return;
     }
-    if (MODE == 0) {
+    if (MODE == SCHEME_BATCH) {
         for (;;) {
             int base = 0;
             if (lane == 0) base = atomicAdd(counter, 32);
@@ -1313,7 +1319,7 @@ RUMI_D void traverse_queue(const DevScene &s, int n, int *counter, int refill_mi
             }
         }
         if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        if (MODE == 1) {
+        if (MODE == SCHEME_REFILL) {
             if (ray >= 0 && T.cur != -2) trav_step<ANYHIT, STACK_SMEM, STATS>(s, T, smem_stack, stride, spill, st);
         } else {
             for (int it = 0; it < 4 * RUMI_MAX_BVH_DEPTH; ++it) {
