@@ -100,7 +100,14 @@ def cpu_model():
 
 
 # --------------------------------------------------------------------- clocks
-ORDERED_PATHS = 1 << 22  # paths of a wave from which its rays are ordered between bounces
+ORDERED_PATHS = 1 << 22     # paths of a wave from which its rays are ordered between bounces ...
+ORDERED_TRIANGLES = 1000    # ... over a tree of 64 four-wide nodes: these scenes have 266 triangles or
+                            # fewer (not ordered) or 1,034 and more
+
+
+def ordered(paths, triangles, trace_mode=0):
+    """Whether the default walk's waves of that many paths are ordered (pt.cu, sort_wave)."""
+    return paths >= ORDERED_PATHS and triangles >= ORDERED_TRIANGLES and trace_mode in (0, 4)
 
 
 def wave_launches(depth, ordered=False):
@@ -442,6 +449,7 @@ def our_arm(args):
     w = workload(args)
     sc = build_scene(w)
     gs = rumi_b200.GpuScene(sc)
+    n_tris = gs.flat.tri_vertices.shape[0]
     bvh = gs.bvh_info()
     paths_per_frame = w["width"] * w["height"] * w["spp"]
     film = torch.empty((w["height"], w["width"], 3), dtype=torch.float32, device="cuda")
@@ -473,7 +481,7 @@ def our_arm(args):
         rays_ext += st["rays_extend"]
         rays_sh += st["rays_shadow"]
         waves = st["extend_launches"] // w["max_depth"]
-        launches += waves * wave_launches(w["max_depth"], ordered=st["paths"] // waves >= ORDERED_PATHS)
+        launches += waves * wave_launches(w["max_depth"], ordered(st["paths"] // waves, n_tris, args.trace_mode))
     ev1.record()
     barrier()
     clocks_info = clocks.stop()
@@ -498,10 +506,19 @@ def our_arm(args):
     achieved = bytes_per_ray * rays_per_launch / (avg_launch_ms / 1000.0) / 1e9
     pk, pk_kind = peaks()
     traffic = extend_traffic()
-    roofline = dict(bound="hbm", achieved=achieved, peak=pk["hbm_gbs"], unit="GB/s", frac=achieved / pk["hbm_gbs"],
-                    # DRAM bytes per closest-hit ray from the committed ncu capture, times this
-                    # run's rays per launch (the capture's launches may hold another wave size)
-                    traffic=traffic["dram_bytes_per_ray"] * rays_per_launch if traffic else None,
+    # the tree and primitives are served mostly from L1 and L2 (see the ncu summary), so the
+    # algorithmic bytes are set against an L2-resident copy measured here, and the DRAM bytes that
+    # the committed ncu capture counted per ray against the measured HBM rate
+    l2 = l2_read_gbs()
+    dram = traffic["dram_bytes_per_ray"] * rays_per_launch if traffic else None
+    dram_gbs = dram / (avg_launch_ms / 1000.0) / 1e9 if dram else None
+    roofline = dict(bound="l2", achieved=achieved, peak=l2, unit="GB/s", frac=achieved / l2,
+                    how="one launch re-reading a 64 MiB buffer 50 times (rumi_test_read_bandwidth), best of 5, "
+                        "CUDA events",
+                    hbm=dict(achieved=dram_gbs, peak=pk["hbm_gbs"], unit="GB/s",
+                             frac=dram_gbs / pk["hbm_gbs"] if dram else None),
+                    # (the capture's launches may hold another wave size)
+                    traffic=dram,
                     kernel="pt_extend (closest-hit)", peak_kind=pk_kind,
                     algorithmic_bytes_per_ray=bytes_per_ray, nodes_per_ray=nodes_per_ray, prims_per_ray=prims_per_ray,
                     rays_per_launch=rays_per_launch, avg_launch_ms=avg_launch_ms,
@@ -509,13 +526,6 @@ def our_arm(args):
                     measured="CUDA events around every closest-hit launch of --steps frames rendered with "
                              "RUMI_FLAG_SERIAL (each kernel alone on the GPU), after the timed frames",
                     per_frame_ms_serial={k: round(v, 2) for k, v in kern.items()})
-    # the tree and primitives are served mostly from L2 (see the ncu summary), so the same
-    # algorithmic bytes are also set against an L2-resident copy measured here
-    l2 = l2_read_gbs()
-    roofline["l2"] = dict(peak=l2, unit="GB/s", frac=achieved / l2,
-                          how="one launch re-reading a 64 MiB buffer 50 times (rumi_test_read_bandwidth), "
-                              "best of 5, CUDA events")
-
     # ---- end to end through the C-ABI: pinned host scene -> device, BVH build, render, film -> host
     e2e = None
     if not args.no_e2e:
@@ -880,7 +890,8 @@ def adjoint_arm(args):
                                     float(abs(m_start[6] - m_tgt[6]))],
                 medium_error_end=[float(np.abs(m_end - m_tgt)[0:3].sum()), float(np.abs(m_end - m_tgt)[3:6].sum()),
                                   float(abs(m_end[6] - m_tgt[6]))],
-                gpu_launches=args.adam_steps * (wave_launches(depth) + 2 * (1 + 3 * depth)), clocks=clocks_info)
+                gpu_launches=args.adam_steps * (wave_launches(depth, ordered(size * size * grad_spp, n_mesh)) +
+                                                2 * (1 + 3 * depth)), clocks=clocks_info)
     print(json.dumps(line), flush=True)
     g.close()
     return 0
