@@ -10,9 +10,9 @@
 // adjacent, so that one packed operation (fma.rn.f32x2) serves both axes with the ray's
 // constants as they lie in registers, and with |1/d| per ray the slab ends are t_c -+ h |1/d|:
 // no minimum or maximum picks near from far, which matters because those run at half the rate of
-// multiply-adds.  The walk is bound by the L1's rate for divergent loads (one 128-byte line per
-// cycle and SM: 80% busy with a 128-byte node in four loads, 66% with this one), then by the
-// half-rate pipe (59%).  Measured per 1024x1024x64 frame of the 1M-triangle workload, closest-hit
+// multiply-adds.  The walk is bound by issue (65% active) with half of the lanes waiting, then by the
+// L1's rate for divergent loads (one 128-byte line per cycle and SM: 73%; with a 128-byte node in four
+// loads it was 80% and the first bound) and by the half-rate pipe (59%).  Measured per 1024x1024x64 frame of the 1M-triangle workload, closest-hit
 // / any-hit: binary tree, scalar slabs 85.8 / 46.5 ms; binary, this slab form 78.5 / 42.1;
 // four-wide with 32-bit half extents (128 bytes) 71.6 / 38.7; this node 64.1 / 33.9 (52.3 / 29.0 with
 // the rays of a large wave in order); a 64-byte node with 8-bit planes 73.9 / 40.1 (the byte decoding
