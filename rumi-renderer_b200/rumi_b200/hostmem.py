@@ -55,7 +55,7 @@ class _Pool:
     def _drop(self, need: int):
         """Gives pooled blocks of other sizes back, largest first."""
         for size in sorted(self.free, reverse=True):
-            while need > 0 and self.free[size]:
+            while need > 0 and self.free.get(size):
                 _capi.load().rumi_host_free(C.c_void_p(self.free[size].pop()))
                 self.total -= size
                 need -= size
@@ -63,6 +63,14 @@ class _Pool:
     def give(self, address: int, size: int):
         with self.lock:
             self.free.setdefault(size, []).append(address)
+            if self.total > self.limit:
+                self._drop(self.total - self.limit)
+
+    def set_limit(self, limit: int):
+        with self.lock:
+            self.limit = limit
+            self.gone.clear()
+            self._drop(self.total - limit)
 
     def wanted(self, size: int) -> bool:
         """Whether the next result of this size takes a block."""
@@ -88,6 +96,20 @@ def _after_fork():
 
 
 os.register_at_fork(after_in_child=_after_fork)
+
+
+def set_limit(limit: int):
+    """Bounds the page-locked memory to `limit` bytes from now on (0: none, every array is an ordinary
+    one).  Pooled blocks beyond the bound are given back at once, those in use when their last view is
+    gone."""
+    _pool.set_limit(int(limit))
+
+
+def release():
+    """Gives the pooled blocks back to the system; arrays in use keep theirs."""
+    limit = _pool.limit
+    _pool.set_limit(0)
+    _pool.set_limit(limit)
 
 
 def _block_size(need: int) -> int:

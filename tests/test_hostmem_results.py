@@ -49,6 +49,26 @@ def test_a_view_keeps_an_ordinary_result(lib):  # noqa: F811
     assert sum(hostmem._pool.gone.values()) == 1
 
 
+def test_blocks_are_given_back(lib):  # noqa: F811
+    a, b = hostmem.empty((16384,), np.float32), hostmem.empty((16384,), np.float32)
+    b[:] = 2.0
+    del a
+    gc.collect()
+    assert len(lib.live) == 2
+    hostmem.release()
+    assert len(lib.live) == 1 and (b == 2.0).all()
+    c = hostmem.empty((16384,), np.float32)  # the pool still works
+    assert c.ctypes.data in lib.live
+    hostmem.set_limit(0)
+    assert len(lib.live) == 2 and hostmem.empty((16384,), np.float32).ctypes.data not in lib.live
+    del b, c
+    gc.collect()
+    assert len(lib.live) == 0 and hostmem._pool.total == 0
+    for _ in range(6):
+        hostmem.result((16384,), np.float32)
+    assert len(lib.live) == 0
+
+
 @pytest.mark.gpu
 def test_kept_films_lock_no_pages(monkeypatch):
     import rumi_b200
