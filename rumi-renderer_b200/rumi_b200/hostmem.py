@@ -13,6 +13,7 @@ film takes 0.51 and 0.99; 640x480 films take 0.44 to 1.9 ms, and 1.4 with blocks
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
 import threading
 import weakref
@@ -116,14 +117,7 @@ def _block_size(need: int) -> int:
     return max(SMALLEST, 1 << (need - 1).bit_length())
 
 
-def empty(shape, dtype) -> np.ndarray:
-    """An uninitialised C-contiguous array, page-locked when the pool has room."""
-    dtype = np.dtype(dtype)
-    count = int(np.prod(shape, dtype=np.int64))
-    need = count * dtype.itemsize
-    if need == 0 or need > _pool.limit // 4:
-        return np.empty(shape, dtype)
-    size = _block_size(need)
+def _in_block(shape, dtype, count: int, size: int) -> np.ndarray:
     address = _pool.take(size)
     if address is None:
         return np.empty(shape, dtype)
@@ -132,12 +126,26 @@ def empty(shape, dtype) -> np.ndarray:
     return np.frombuffer(block, dtype, count).reshape(shape)
 
 
+def empty(shape, dtype) -> np.ndarray:
+    """An uninitialised C-contiguous array, page-locked when the pool has room."""
+    dtype = np.dtype(dtype)
+    count = math.prod(shape)
+    need = count * dtype.itemsize
+    if need == 0 or need > _pool.limit // 4:
+        return np.empty(shape, dtype)
+    return _in_block(shape, dtype, count, _block_size(need))
+
+
 def result(shape, dtype) -> np.ndarray:
     """``empty`` where the program has let go of results of this size, else an ordinary array."""
     dtype = np.dtype(dtype)
-    need = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
-    if need == 0 or need > _pool.limit // 4 or _pool.wanted(_block_size(need)):
-        return empty(shape, dtype)
+    count = math.prod(shape)
+    need = count * dtype.itemsize
+    if need == 0 or need > _pool.limit // 4:
+        return np.empty(shape, dtype)
+    size = _block_size(need)
+    if _pool.wanted(size):
+        return _in_block(shape, dtype, count, size)
     base = np.empty(need, np.uint8)
-    weakref.finalize(base, _pool.let_go, _block_size(need)).atexit = False
+    weakref.finalize(base, _pool.let_go, size).atexit = False
     return base.view(dtype).reshape(shape)
