@@ -146,6 +146,6 @@ def result(shape, dtype) -> np.ndarray:
     size = _block_size(need)
     if _pool.wanted(size):
         return _in_block(shape, dtype, count, size)
-    base = np.empty(need, np.uint8)
-    weakref.finalize(base, _pool.let_go, size).atexit = False
-    return base.view(dtype).reshape(shape)
+    array = np.empty(shape, dtype)  # its views refer to it
+    weakref.finalize(array, _pool.let_go, size).atexit = False
+    return array
