@@ -390,6 +390,8 @@ const char *rumi_version(void) { return "rumi_b200 0.1 (sm_100a)"; }
 // triangles 0.85 / 1.00, 16,394 1.06 / 1.08, 32,778 1.17 / 1.21, 65,546 1.39 / 1.36, 131,082 1.85 / 1.67,
 // 262,154 2.82 / 2.28.
 static constexpr int SIDE_UPLOAD_TRIANGLES = 65536;
+// Triangles from which their inputs are released before the four-wide tree is made: 25 GB in the build.
+static constexpr int EARLY_FREE_TRIANGLES = 1 << 26;
 
 rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
     if (!out) return set_error("out is NULL"), RUMI_ERR_INVALID_ARG;
@@ -556,7 +558,28 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         set_error("bvh_build: internal limit reached");
         return fail(RUMI_ERR_INTERNAL);
     }
-    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, build_kc, build_h, &sc->wide, &sc->n_wide, &sc->recs, &sc->n_recs, s);
+    // What the collapse allocates (about 186 bytes a primitive) takes the place of the build's scratch
+    // memory (143) and, where memory may be short, of the inputs (88), at the price of waiting for the
+    // shading data first: at most 423 bytes a triangle in all (631 when everything was kept to the end).
+    auto drop_inputs = [&]() {
+        // (the frees follow the side stream's kernels)
+        const cudaError_t we = side ? cudaStreamWaitEvent(s, ev_side, 0) : cudaSuccess;
+        if (we != cudaSuccess) return we;
+        for (void *p : {(void *)d_tri_v, (void *)d_tri_n, (void *)d_tri_m, (void *)d_alb, (void *)d_rect_em}) dfree(p, s);
+        d_tri_v = d_tri_n = d_alb = nullptr;
+        d_rect_em = d_tri_m = nullptr;
+        return cudaSuccess;
+    };
+    if (!build_kc) {
+        dfree(scratch, s);
+        scratch = nullptr;
+    }
+    if (nT >= EARLY_FREE_TRIANGLES && (e = drop_inputs()) != cudaSuccess) {
+        drop_events();
+        return fail(cuda_status(e, "scene upload"));
+    }
+    rc = bvh_wide(sc->nodes, sc->n_nodes, sc->leaf_prims, N, build_kc, build_h, &sc->wide, &sc->n_wide, &sc->recs,
+                  &sc->n_recs, s);
     if (rc <= 0 && build_kc && bvh_build_check(build_h, N, &sc->info) != 0) {
         drop_events();
         set_error("bvh_build: internal limit reached");
@@ -569,21 +592,11 @@ rumi_status rumi_scene_create(const rumi_scene_desc *d, rumi_scene **out) {
         return fail(RUMI_ERR_INTERNAL);
     }
     cudaEventRecord(e1, s);
-    if (side) {
-        e = cudaStreamWaitEvent(s, ev_side, 0);  // the frees below follow the side stream's kernels
-        if (e != cudaSuccess) {
-            drop_events();
-            return fail(cuda_status(e, "scene upload"));
-        }
+    if ((e = drop_inputs()) != cudaSuccess) {
+        drop_events();
+        return fail(cuda_status(e, "scene upload"));
     }
-    dfree(d_tri_v, s);
-    dfree(d_tri_n, s);
-    dfree(d_tri_m, s);
-    dfree(d_alb, s);
-    dfree(d_rect_em, s);
     dfree(scratch, s);
-    d_tri_v = d_tri_n = d_alb = nullptr;
-    d_rect_em = d_tri_m = nullptr;
     scratch = nullptr;
     ds.nodes = sc->nodes;
     ds.nodes8 = sc->nodes8;

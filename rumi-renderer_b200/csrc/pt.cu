@@ -71,7 +71,7 @@ static constexpr int trace_min_blocks(int mode, bool extend) {
 #endif
 static constexpr int STACK_SMEM = 32;
 // Leaf records (the empty one included) up to which a single-node scene's rays are traced in step
-// (scene_scheme).
+// (scene_scheme; eleven would still gain).
 #ifndef RUMI_FEW_RECORDS
 #define RUMI_FEW_RECORDS 10
 #endif
@@ -1187,7 +1187,10 @@ static inline int trace_scheme(int trace_mode) {
 // scheme or for traversal counts.  Closest-hit / any-hit ms of a 512x512, 16 spp, depth-6 frame,
 // walk against that: 10 triangles and a light (7 records) 0.71 / 0.55 and 0.68 / 0.54; 12
 // triangles, a light and a sphere (9) 0.96 / 0.61 and 0.93 / 0.65; and of the 256x256, 16 spp,
-// depth-8 Cornell frame (9 records) 0.31 / 0.23 and 0.27 / 0.22.
+// depth-8 Cornell frame (9 records) 0.31 / 0.23 and 0.27 / 0.22.  Whole frames: one-node scenes of 7 and 8
+// records 0.60 / 0.63 walked and 0.51 / 0.54 in step, the box with 2, 4, 6 and 8 more triangles (8 to 11
+// records) 0.84 / 0.85 / 0.90 / 0.91 and 0.78 / 0.80 / 0.82 / 0.87; no scene with more records came out as
+// one node.
 static inline int scene_scheme(const rumi_scene *sc, const rumi_render_params *p) {
     const bool few = sc->n_wide == 1 && sc->n_recs <= RUMI_FEW_RECORDS;
     return few && DEFAULT_WALK_MODE == SCHEME_WIDE && p->trace_mode == 0 && !(p->flags & RUMI_FLAG_STATS)
