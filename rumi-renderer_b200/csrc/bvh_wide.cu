@@ -9,9 +9,9 @@
 // leaf.  The host does not wait between levels (a launch on an empty frontier costs about 2 us); it
 // reads the counts once, then allocates the two arrays to size and writes the leaf records.  A small
 // scene's tree is made by one block in one launch, in arrays for as many nodes and records as there
-// can be: of a scene of 11 primitives build and collapse are a chain of short launches and waits, 0.31 ms
-// of its creation with three launches, two copies and a wait for the levels, 0.25 with the one block
-// (0.26 without this tree).
+// can be: build and collapse are a chain of short launches and waits there, and a scene of 11 primitives
+// is created in 0.25 ms, 0.31 with three launches, two copies and a wait for the levels (0.26 without
+// this tree).
 #include "renderer.h"
 #include "traverse.cuh"
 #include <algorithm>
